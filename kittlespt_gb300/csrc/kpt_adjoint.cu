@@ -807,13 +807,13 @@ struct AdjShadowQueue {
     const ShadowRec* rec;
     unsigned char* vis;
     int nsun, cap;
+    __device__ __forceinline__ float tmin() const { return 0.0f; }
     __device__ __forceinline__ int slot(int i) const { return i < nsun ? i : cap - 1 - (i - nsun); }
-    __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmin, float& tmax) const {
+    __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmax) const {
         const int j = slot(i);
         const float4 a = rec[j].o_tmax, b = rec[j].d_item;
         o = make_float3(a.x, a.y, a.z);
         d = make_float3(b.x, b.y, b.z);
-        tmin = 0.0f;
         tmax = a.w;
     }
     __device__ __forceinline__ bool closest(int, const Hit&, float3&, float3&) const { return false; }

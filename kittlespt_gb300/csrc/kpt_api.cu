@@ -109,6 +109,7 @@ struct kpt_context {
     DBuf<TexRec> d_textures;
     DBuf<uint8_t> d_pixels;
     SceneView view{};
+    std::vector<int> mesh_roots;   // per mesh: InstRec::root of its instances
     std::vector<int> mesh_node_base, mesh_tri_base;   // per mesh: first node / triangle in the device arrays
     std::vector<LightRec> h_lights;
     std::vector<InstRec> h_inst;
@@ -222,6 +223,9 @@ static constexpr size_t ADJ_WAVE_BYTES = (size_t)12 << 30;
 // pixel-major waves and shading blocks of 256 (20.51 ms; 6: 20.55-20.60, 8:
 // 20.53, 5: 20.65, 4: 20.83)
 static constexpr int FETCH_BATCH = 7;
+// the same for bounce chains, whatever the tuning: 1M rays and 4 bounces in 2M
+// random triangles take 1.24 ms with 7, 1.38 with 1, 1.26 with 4 and 12
+static constexpr int CHAIN_FETCH_BATCH = 7;
 // threads per block of the shading kernel unless tuned (256: 22.48 ms on the
 // 1080p16 frame against 22.51 with 128 and 64)
 static constexpr int SHADE_BLOCK = SHADE_MAX_BLOCK;
@@ -596,7 +600,7 @@ static InstRec make_inst(const kpt_context* c, const HostInstance& hi) {
     r.material = hi.material;
     r.light_first = -1;
     r.light_all = 0;
-    (void)c;
+    r.root = c->mesh_roots[hi.mesh];
     return r;
 }
 
@@ -647,6 +651,7 @@ kpt_status kpt_commit_scene(kpt_context* c) {
     std::vector<MeshRec> mrec;
     c->mesh_node_base.clear();
     c->mesh_tri_base.clear();
+    c->mesh_roots.clear();
     for (auto& m : c->meshes) {
         MeshRec r{};
         int nb = (int)nodes.size(), tb = (int)(tris.size() / 3);
@@ -659,6 +664,7 @@ kpt_status kpt_commit_scene(kpt_context* c) {
         }
         r.node_root = m.root >= 0 ? nb + m.root : -1;
         r.leaf_first = tb + m.leaf_first;
+        c->mesh_roots.push_back(m.root >= 0 ? nb + m.root : ~(tb + m.leaf_first));
         r.leaf_count = m.leaf_count;
         r.ntris = m.ntris();
         r.tri_base = tb;
@@ -672,6 +678,13 @@ kpt_status kpt_commit_scene(kpt_context* c) {
             tris.push_back(make_float4(p[0], p[1], p[2], lid));
             tris.push_back(make_float4(p[3] - p[0], p[4] - p[1], p[5] - p[2], 0.0f));
             tris.push_back(make_float4(p[6] - p[0], p[7] - p[1], p[8] - p[2], 0.0f));
+        }
+        // the last triangle of each leaf is marked (the queue traversal's leaves end there)
+        auto last_of = [&](int first, int count) { tris[3 * (size_t)(tb + first + count - 1) + 1].w = 1.0f; };
+        if (m.root < 0 && m.leaf_count > 0) last_of(m.leaf_first, m.leaf_count);
+        for (const BvhNode& n : m.nodes) {
+            if (n.d.y) last_of(n.d.x, n.d.y);
+            if (n.d.w) last_of(n.d.z, n.d.w);
         }
         int rank = 0;
         for (int t = 0; t < m.ntris(); ++t) {
@@ -736,6 +749,7 @@ kpt_status kpt_commit_scene(kpt_context* c) {
     KPT_CUDA(c->d_nodes.upload(nodes.data(), nodes.size(), c->stream));
     c->n_nodes = (int)nodes.size();
     c->n_tris = (int)(tris.size() / 3);
+    KPT_CUDA(c->d_tris.ensure(tris.size() + TRI_PAD));
     KPT_CUDA(c->d_tris.upload(tris.data(), tris.size(), c->stream));
     {
         std::vector<int> tri_leaf(tris.size() / 3);
@@ -1556,11 +1570,14 @@ kpt_status kpt_render_samples_device(kpt_context* c, int sample0, int nsamples, 
     return KPT_OK;
 }
 
+// Blocks of a ray batch of n: the resident ones, or fewer when n rays give
+// each warp less than one (the kernels spread a short queue over their warps).
 static int trace_grid(kpt_context* c, const void* kern, int n) {
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TRACE_BLOCK, 0);
     int g = std::max(1, per_sm) * c->sm_count;
-    return std::min(g, (n + TRACE_BLOCK - 1) / TRACE_BLOCK);
+    constexpr int warps = TRACE_BLOCK / 32;
+    return std::min(g, (n - 1) / warps + 1);
 }
 
 static kpt_status scene_ready(kpt_context* c) {
@@ -1608,10 +1625,8 @@ kpt_status kpt_trace_bounces_device(kpt_context* c, int n, const float* o, const
         return fail(KPT_ERR_INVALID, "kpt_trace_bounces_device: bad arguments");
     if (n == 0) return KPT_OK;
     KPT_CUDA(cudaMemsetAsync(c->fetch.p, 0, sizeof(int), c->stream));
-    // a lane of a chain traces its next bounce without a fetch: batching the
-    // fetches measured slower here (675 vs 650 Mrays/s on 2M random triangles)
     SceneView v = c->view;
-    v.fetch_batch = 1;
+    v.fetch_batch = CHAIN_FETCH_BATCH;
     k_trace_chains<<<trace_grid(c, (const void*)k_trace_chains, n), TRACE_BLOCK, 0, c->stream>>>(
         v, n, (const float3*)o, (const float3*)d, nb, inst, tri, t, c->fetch.p, c->counters.p);
     c->launches += 1;
@@ -2166,7 +2181,7 @@ kpt_status merge_scenes(kpt_batch* b, int n, kpt_context* const* jobs) {
         return fail(KPT_ERR_INVALID, "kpt_submit_batch: the jobs' scenes together are too large to merge");
     b->m_key.clear();
     KPT_CUDA(b->m_nodes.ensure(nn));
-    KPT_CUDA(b->m_tris.ensure(3 * nt));
+    KPT_CUDA(b->m_tris.ensure(3 * nt + TRI_PAD));
     KPT_CUDA(b->m_meshes.ensure(nm));
     KPT_CUDA(b->m_inst.ensure(ni));
     KPT_CUDA(b->m_tlas.ensure(nl));
@@ -2188,7 +2203,7 @@ kpt_status merge_scenes(kpt_batch* b, int n, kpt_context* const* jobs) {
             k_merge_meshes<<<blocks(meshes), 256, 0, b->stream>>>(c->d_meshes.p, meshes, b->m_meshes.p + mesh_base,
                                                                    node_base, tri_base);
         if (inst > 0)
-            k_merge_inst<<<blocks(inst), 256, 0, b->stream>>>(c->d_inst.p, inst, b->m_inst.p + inst_base, mesh_base);
+            k_merge_inst<<<blocks(inst), 256, 0, b->stream>>>(c->d_inst.p, inst, b->m_inst.p + inst_base, mesh_base, node_base, tri_base);
         if (tlas > 0)
             k_merge_nodes<<<blocks(tlas), 256, 0, b->stream>>>(c->d_tlas.p, tlas, b->m_tlas.p + tlas_base, tlas_base,
                                                                 inst_base);
@@ -2687,7 +2702,7 @@ extern "C" kpt_status kpt_trace_bounces_noalloc(kpt_context* c, int n, const flo
     // of the staging array) must start at zero
     KPT_CUDA(cudaMemsetAsync(c->fetch.p, 0, sizeof(int), c->stream));
     SceneView v = c->view;
-    v.fetch_batch = 1;
+    v.fetch_batch = CHAIN_FETCH_BATCH;
     k_trace_chains<<<trace_grid(c, (const void*)k_trace_chains, n), TRACE_BLOCK, 0, c->stream>>>(
         v, n, (const float3*)d_o, (const float3*)d_d, nb, d_inst, d_tri, d_t, c->fetch.p, c->counters.p);
     c->launches += 1;

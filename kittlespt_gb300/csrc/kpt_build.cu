@@ -1166,7 +1166,7 @@ __global__ void k_refit_tris(const float* pos, const int* order, int n, int tri_
     const float* p = pos + 9 * (size_t)t;
     float4* o = tris + 3 * ((size_t)tri_base + k);
     o[0] = make_float4(p[0], p[1], p[2], __int_as_float(t));
-    o[1] = make_float4(__fsub_rn(p[3], p[0]), __fsub_rn(p[4], p[1]), __fsub_rn(p[5], p[2]), 0.0f);
+    o[1] = make_float4(__fsub_rn(p[3], p[0]), __fsub_rn(p[4], p[1]), __fsub_rn(p[5], p[2]), o[1].w);
     o[2] = make_float4(__fsub_rn(p[6], p[0]), __fsub_rn(p[7], p[1]), __fsub_rn(p[8], p[2]), 0.0f);
 }
 

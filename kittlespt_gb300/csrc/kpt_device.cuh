@@ -6,7 +6,10 @@
 //                              64-byte record (four 16-byte loads) instead of
 //                              two 32-byte child records;
 //   tris       : float4[3*T]  per triangle in BVH leaf order:
-//                              (v0.xyz, local id), (v1-v0, 0), (v2-v0, 0);
+//                              (v0.xyz, local id), (v1-v0, 1 for the last
+//                              triangle of a leaf, else 0), (v2-v0, 0);
+//                              then TRI_PAD unused entries, so that a group of
+//                              lanes may read past the last leaf's end;
 //   shade      : TriShade[T]  per triangle in mesh order: uvs, local
 //                              geometric normal, material, emissive rank;
 //   meshes     : MeshRec[ ]   BLAS root, offsets;
@@ -63,7 +66,8 @@ struct __align__(16) InstRec {
     int light_first;          // first light of this instance, -1: none
     int light_all;            // 1: every triangle is a light (emissive override)
     int prim_base;            // first triangle of this instance in the expanded numbering
-    int pad0, pad1, pad2;
+    int root;                 // its mesh's BLAS: root node, or ~(first triangle) of a root leaf
+    int pad1, pad2;
 };
 
 struct __align__(16) LightRec {  // one emissive triangle of one instance
@@ -78,6 +82,7 @@ struct __align__(16) LightRec {  // one emissive triangle of one instance
     int pad;
 };
 
+constexpr int TRI_PAD = 3 * 8;   // float4 entries after the triangles
 constexpr int BLAS_STACK = 48;   // traversal stack entries per ray for a BLAS (the reference has 16)
 constexpr int TLAS_STACK = 32;   // traversal stack entries per ray for the TLAS (the reference has 16)
 constexpr int STACK_WORDS = BLAS_STACK + TLAS_STACK;

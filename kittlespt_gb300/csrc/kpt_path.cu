@@ -566,11 +566,11 @@ __global__ void __launch_bounds__(256) k_sort_scatter(FrameParams F, int level) 
 struct ExtendQueue {
     const PathRec* in;
     PrimaryRec* out;
-    __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmin, float& tmax) const {
+    __device__ __forceinline__ float tmin() const { return 0.0f; }
+    __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmax) const {
         const float4 a = in[i].o_pb, b = in[i].d_seed;
         o = make_float3(a.x, a.y, a.z);
         d = make_float3(b.x, b.y, b.z);
-        tmin = 0.0f;
         tmax = __int_as_float(0x7f800000);
     }
     __device__ __forceinline__ bool closest(int i, const Hit& h, float3&, float3&) const {
@@ -602,13 +602,13 @@ struct ShadowQueue {
     const ShadowRec* rec;
     float4* radiance;
     int nsun, cap;
+    __device__ __forceinline__ float tmin() const { return 0.0f; }
     __device__ __forceinline__ int slot(int i) const { return i < nsun ? i : cap - 1 - (i - nsun); }
-    __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmin, float& tmax) const {
+    __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmax) const {
         const int j = slot(i);
         const float4 a = rec[j].o_tmax, b = rec[j].d_item;
         o = make_float3(a.x, a.y, a.z);
         d = make_float3(b.x, b.y, b.z);
-        tmin = 0.0f;
         tmax = a.w;
     }
     __device__ __forceinline__ bool closest(int, const Hit&, float3&, float3&) const { return false; }
@@ -873,13 +873,13 @@ struct BatchExtendQueue {
     BatchQueues Q;
     int level;   // the level the paths enter
     int cur;     // job of the entry being set up (ray() then root())
-    __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmin, float& tmax) {
+    __device__ __forceinline__ float tmin() const { return 0.0f; }
+    __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmax) {
         cur = batch_job_of(Q.ext_prefix, Q.njobs, i);
         const PathRec& p = Q.jobs[cur].paths[level & 1][i - __ldg(Q.ext_prefix + cur)];
         const float4 a = p.o_pb, b = p.d_seed;
         o = make_float3(a.x, a.y, a.z);
         d = make_float3(b.x, b.y, b.z);
-        tmin = 0.0f;
         tmax = __int_as_float(0x7f800000);
     }
     __device__ __forceinline__ void root(int, float4& lo, float4& hi, int& root, int& ninst) const {
@@ -910,7 +910,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, TRACE_MIN_BLOCKS) k_extend_batch(
     int stack[STACK_WORDS];
     TraceStats st = {0, 0, 0, 0};
     BatchExtendQueue q{Q, level, 0};
-    trace_queue<false, BatchExtendQueue, 1, true>(s, __ldg(Q.ext_prefix + Q.njobs), Q.fetch, q, st, stack);
+    trace_queue<false, BatchExtendQueue, true>(s, __ldg(Q.ext_prefix + Q.njobs), Q.fetch, q, st, stack);
     flush_stats(st, counters);
 }
 
@@ -919,19 +919,19 @@ struct BatchShadowQueue {
     int level;
     int cur;
     // the entry's record: sun rays from the front of the job's buffer, light rays from the back
+    __device__ __forceinline__ float tmin() const { return 0.0f; }
     __device__ __forceinline__ const ShadowRec& rec(int j, int i) const {
         const BatchJob& J = Q.jobs[j];
         const int k = i - __ldg(Q.shd_prefix + j);
         const int nsun = J.level_counts[LEVEL_WORDS * level + 1];
         return J.shadow[k < nsun ? k : J.cap - 1 - (k - nsun)];
     }
-    __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmin, float& tmax) {
+    __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmax) {
         cur = batch_job_of(Q.shd_prefix, Q.njobs, i);
         const ShadowRec& r = rec(cur, i);
         const float4 a = r.o_tmax, b = r.d_item;
         o = make_float3(a.x, a.y, a.z);
         d = make_float3(b.x, b.y, b.z);
-        tmin = 0.0f;
         tmax = a.w;
     }
     __device__ __forceinline__ void root(int, float4& lo, float4& hi, int& root, int& ninst) const {
@@ -959,7 +959,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, TRACE_MIN_BLOCKS) k_shadow_batch(
     int stack[STACK_WORDS];
     TraceStats st = {0, 0, 0, 0};
     BatchShadowQueue q{Q, level, 0};
-    trace_queue<true, BatchShadowQueue, 1, true>(s, __ldg(Q.shd_prefix + Q.njobs), Q.fetch + 1, q, st, stack);
+    trace_queue<true, BatchShadowQueue, true>(s, __ldg(Q.shd_prefix + Q.njobs), Q.fetch + 1, q, st, stack);
     flush_stats(st, counters ? counters + 8 : nullptr);
 }
 
@@ -982,11 +982,12 @@ __global__ void k_merge_meshes(const MeshRec* src, int n, MeshRec* dst, int node
     dst[i] = m;
 }
 
-__global__ void k_merge_inst(const InstRec* src, int n, InstRec* dst, int mesh_add) {
+__global__ void k_merge_inst(const InstRec* src, int n, InstRec* dst, int mesh_add, int node_add, int tri_add) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     InstRec r = src[i];
     r.mesh += mesh_add;
+    r.root = r.root >= 0 ? r.root + node_add : ~(~r.root + tri_add);
     dst[i] = r;
 }
 
@@ -1046,16 +1047,16 @@ __global__ void k_sky(SkyParams P, int n, const float3* dirs, float3* out) {
 // Closest hit / occlusion for a batch of rays.
 struct RayBatch {
     const float3 *o, *d;
-    float tmin, tmax;
+    float t_min, tmax;
     const float* tmax_each;
     int *inst, *tri;
     float* t;
     float2* uv;
     uint8_t* occ;
-    __device__ __forceinline__ void ray(int i, float3& ro, float3& rd, float& t0, float& t1) const {
+    __device__ __forceinline__ float tmin() const { return t_min; }
+    __device__ __forceinline__ void ray(int i, float3& ro, float3& rd, float& t1) const {
         ro = o[i];
         rd = d[i];
-        t0 = tmin;
         t1 = tmax_each ? tmax_each[i] : tmax;
     }
     __device__ __forceinline__ bool closest(int i, const Hit& h, float3&, float3&) const {
@@ -1129,11 +1130,11 @@ struct BounceQueue {
     const SceneView* s;
     int b;   // bounce of the chain this lane is tracing
     float3 ro, rd;
-    __device__ __forceinline__ void ray(int i, float3& oo, float3& dd, float& tmin, float& tmax) {
+    __device__ __forceinline__ float tmin() const { return 0.0f; }
+    __device__ __forceinline__ void ray(int i, float3& oo, float3& dd, float& tmax) {
         b = 0;
         ro = oo = o[i];
         rd = dd = d[i];
-        tmin = 0.0f;
         tmax = __int_as_float(0x7f800000);
     }
     __device__ __forceinline__ bool closest(int i, const Hit& h, float3& no, float3& nd) {
@@ -1174,7 +1175,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK, TRACE_MIN_BLOCKS) k_trace_chains(
     int stack[STACK_WORDS];
     TraceStats st = {0, 0, 0, 0};
     BounceQueue q{o, d, n, nbounces, inst, tri, t, &s, 0, make_float3(0.0f, 0.0f, 0.0f), make_float3(0.0f, 0.0f, 0.0f)};
-    trace_queue<false, BounceQueue, 2>(s, n, next, q, st, stack);
+    trace_queue<false, BounceQueue>(s, n, next, q, st, stack);
     flush_stats(st, counters);
 }
 

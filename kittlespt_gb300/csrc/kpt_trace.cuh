@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 
 #include "kpt_device.cuh"
+#include "kpt_internal.h"
 
 namespace kpt {
 
@@ -319,201 +320,352 @@ __device__ __forceinline__ bool trace_any(const SceneView& s, const XRay& r, flo
 }
 
 // ---------------------------------------------------------------------------
-// Queue traversal: a persistent warp walks a queue of rays.  Each lane runs
-// its own ray and, when the ray is done, fetches the next queue entry (one
-// atomic per group of lanes fetching together), so no lane waits for the
-// longest ray of its warp.  One loop iteration is one step of a lane's ray --
-// a node (TLAS and BLAS share the node format), one triangle, entering or
-// leaving an instance -- so lanes at different depths of the two levels keep
-// issuing together.  The visiting order and culling are those of
-// trace_closest / trace_any above (the BLAS keeps its local closest hit and
-// culls against it, and is merged into the ray's closest hit when left), so
-// every result is identical to theirs.
+// Queue traversal: persistent warps walk a queue of rays.  Each lane owns one
+// ray and, when it is done, fetches the next queue entry, so no lane waits
+// for the longest ray of its warp.  The warp alternates between three kinds of
+// work, each run for many lanes at a time:
+//   * interior nodes: every lane whose next entry is a node steps through
+//     nodes until it reaches something else; the loop ends for the warp when
+//     fewer than half of its live lanes are still in it;
+//   * leaves: the warp tests the pending leaves together, four lanes to a
+//     leaf (eight while at most four leaves are pending), one triangle each,
+//     the rays read from shared memory; the group's closest hit goes back to
+//     the lane that owns the ray;
+//   * instances: lanes entering or leaving one change the ray's space.
+// What bounds it: instruction issue (73% of cycles at 21 of 32 lanes active
+// per instruction) and the L1 data pipe (66%: 64-byte nodes and 48-byte
+// triangles at unrelated addresses).  One step of any kind per loop iteration
+// with leaves tested by their own lane, as before, ran 11.7 lanes per
+// instruction: the extension rays of the 1920x1080x16 frame (depth 8) took
+// 11.15 ms and its shadow rays 5.86 ms, now 6.33 and 2.95; 1M bounce chains
+// in 2M triangles 2.29 ms, now 1.39.  Measured on the way (the same frame's
+// extension rays): nodes and leaves in loops of their own 8.99, each left
+// early 7.94, node records in two 32-byte loads 7.61, the stack's first 16
+// entries in shared memory 7.44 (conflict-free; a divergent local pop spreads
+// over lines), leaves shared by the warp 6.74, results reduced only in rounds
+// with a hit 6.33.  Not kept: the entry distance beside each stack entry, to
+// drop far nodes without loading them (9.15: twice the stack traffic);
+// four-wide nodes for the any-hit rays (the same time).
 //
-// Src supplies the queue:  void ray(int i, float3& o, float3& d, float& tmin, float& tmax);
+// The visiting order and culling are those of trace_closest / trace_any above
+// (the BLAS keeps its local closest hit and culls against it, and is merged
+// into the ray's closest hit when left; among equal distances of a leaf the
+// first triangle wins), so every result is identical to theirs.
+//
+// Src supplies the queue:  float tmin();       (one value for the whole queue)
+//                          void ray(int i, float3& o, float3& d, float& tmax);
 //                          bool closest(int i, const Hit& h, float3& o, float3& d);   (ANY == false)
 //                          void any(int i, bool occluded);      (ANY == true)
 // closest() may return true with the next ray of entry i (a bounce chain):
-// the lane traces it at once, with the same tmin and tmax.  TRI triangles of
-// a leaf are tested per loop iteration (in order; 1 is fastest on the
-// instanced full frame, 2 on one BLAS of 2M random triangles).  ROOTS: the
-// queue spans several scenes merged into `s` (a batch), each entry's TLAS
-// root supplied by
+// the lane traces it next, with the same tmax.  ROOTS: the queue spans
+// several scenes merged into `s` (a batch), each entry's TLAS root supplied by
 //                          void root(int i, float4& lo, float4& hi, int& root, int& ninst);
-// (root: a node index of s.tlas, or -(instance) - 1 for a single-instance scene).
-template <bool ANY, class Src, int TRI = 1, bool ROOTS = false>
+// (root: a node index of s.tlas, or ~instance for a single-instance scene).
+// The block has TRACE_BLOCK threads; the stack never overflows (a scene
+// deeper than BLAS_STACK - 1 or TLAS_STACK - 1 is refused when committed, and
+// a node pushes one entry).
+
+constexpr int STACK_SHARED = 16;   // stack entries per ray in shared memory (8: 7.49 ms, 24 and 32: as 16)
+
+// Two 16-byte quarters of a 64-byte node in one load.
+__device__ __forceinline__ void load_half_node(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
+// The bound b' with (t < b') == (t <= b) for every t (denormals are zero here).
+__device__ __forceinline__ float next_up(float b) {
+    if (!(fabsf(b) < __int_as_float(0x7f800000))) return b;   // infinities and NaN
+    if (fabsf(b) < 1.17549435e-38f) return 1.17549435e-38f;
+    return __int_as_float(__float_as_int(b) + (b > 0.0f ? 1 : -1));
+}
+
+// The hit of local triangle record `slot` (leaf order) of instance `inst` by
+// the world ray o, d, at the distance t found by the traversal: its
+// barycentrics by the same operations as tri_test.
+__device__ __forceinline__ Hit hit_at(const SceneView& s, int inst, int slot, float t, float3 o, float3 d) {
+    const InstRec& ir = s.inst[inst];
+    const float4 inv[3] = {__ldg(&ir.inv[0]), __ldg(&ir.inv[1]), __ldg(&ir.inv[2])};
+    const float3 ro = make_float3(xrow(inv[0], o, 1.0f), xrow(inv[1], o, 1.0f), xrow(inv[2], o, 1.0f));
+    const float3 rd = make_float3(xrow(inv[0], d, 0.0f), xrow(inv[1], d, 0.0f), xrow(inv[2], d, 0.0f));
+    const float4* tri = s.tris + 3 * (size_t)slot;
+    const float4 a = __ldg(tri), b = __ldg(tri + 1), c = __ldg(tri + 2);
+    const float3 e1 = make_float3(b.x, b.y, b.z), e2 = make_float3(c.x, c.y, c.z);
+    const float3 pv = xcross(rd, e2);
+    const float rdet = __frcp_rn(xdot(e1, pv));
+    const float3 tv = xsub3(ro, make_float3(a.x, a.y, a.z));
+    Hit h;
+    h.t = t;
+    h.inst = inst;
+    h.tri = __float_as_int(a.w);
+    h.u = xm(rdet, xdot(tv, pv));
+    h.v = xm(rdet, xdot(rd, xcross(tv, e1)));
+    return h;
+}
+
+template <bool ANY, class Src, bool ROOTS = false>
 __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next, Src& src, TraceStats& st,
                                             int* stack) {
+    constexpr unsigned FULL = 0xffffffffu;
+    // what a lane does next (cur, and the entries of its stack): an interior
+    // node (>= 0), a leaf (~its first triangle, or ~instance in the TLAS), or
+    // leave the instance, store the result, nothing more (the queue is empty)
+    constexpr int LEAVE = (int)0x80000000, DONE = (int)0x80000001, DEAD = (int)0x80000002;
     const float INF = __int_as_float(0x7f800000);
-    XRay w, r;               // world ray; current ray (object space inside an instance)
-    float tmin = 0.0f, tmax0 = INF;
-    Hit best, loc;           // closest hit of the ray; of the instance being traversed
-    int ray = -1;            // queue entry, -1: fetch the next one
-    int inst = -1;           // instance being traversed, -1: in the TLAS
-    int base = 0;            // stack height when the instance was entered
+    __shared__ float world[9][TRACE_BLOCK];    // world ray: origin, reciprocal direction, direction
+    __shared__ float object[6][TRACE_BLOCK];   // ray in its instance: origin, direction
+    __shared__ int top[STACK_SHARED][TRACE_BLOCK];
+    __shared__ int owners[TRACE_BLOCK];
+    if (n <= 0) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp0 = tid & ~31;
+    const float tmin = src.tmin();
+    // a queue of fewer rays than the grid has lanes is spread over all its
+    // warps: short queues are bound by the latency of their longest rays,
+    // which other rays of the warp prolong (1021 rays 88 -> 29 us, the 65k
+    // paths of a 256x256 frame 0.85 -> 0.42 ms with this and the above)
+    const int warps = gridDim.x * (TRACE_BLOCK / 32);
+    int cur = lane < (n + warps - 1) / warps ? DONE : DEAD;
+    int ray = -1;                       // queue entry
+    int inst = -1;                      // instance being traversed, -1: in the TLAS
     int sp = 0;
-    // the top of the stack lives in a register: a node step keeps its near
-    // child here instead of pushing and popping it through local memory
-    constexpr int NONE = (int)0x80000000;
-    int top = NONE;
-    int first = 0, count = 0;   // triangles of the leaf being tested
-    best.t = loc.t = INF;
-    best.inst = best.tri = loc.inst = loc.tri = -1;
-    best.u = best.v = loc.u = loc.v = 0.0f;
-    // a new ray: the TLAS root box (TLAS::intersect, tlas.cu:60-75), then its root
-    auto start = [&](float3 o, float3 d) {
-        w = make_xray(o, d);
-        r = w;
-        best.t = INF;
-        best.inst = best.tri = -1;
-        best.u = best.v = 0.0f;
-        inst = -1;
-        sp = 0;
-        top = NONE;
-        count = 0;
-        float te;
-        st.box_tests++;
-        if constexpr (ROOTS) {
-            float4 lo, hi;
-            int root, ninst;
-            src.root(ray, lo, hi, root, ninst);
-            if (ninst > 0 && slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, w, tmin, tmax0, &te)) top = root;
-        } else {
-            if (s.ninst > 0 &&
-                slab(s.tlas_lo.x, s.tlas_lo.y, s.tlas_lo.z, s.tlas_hi.x, s.tlas_hi.y, s.tlas_hi.z, w, tmin, tmax0, &te))
-                top = s.tlas_root_leaf ? -1 : 0;   // TLAS entries: node index, or -(instance) - 1
-        }
+    float tmax = INF;
+    float bound0 = INF, bound = INF;    // boxes entered at or beyond are culled: of the ray, now
+    float best_t = INF;                 // closest hit of the ray: instance, triangle record
+    int best_inst = -1, best_slot = -1;
+    int slot = -1;                      // closest hit in the instance (its distance is `bound`), -1: none
+    bool occluded = false;              // ANY: a triangle blocked the ray
+    const BvhNode* nodes = s.tlas;
+    float3 o = make_float3(0.0f, 0.0f, 0.0f), inv = o, d = o;   // the ray in the space being traversed
+    auto push = [&](int e) {
+        if (sp < STACK_SHARED) top[sp][tid] = e;
+        else stack[sp] = e;
+        ++sp;
     };
-    bool occluded = false;   // ANY: a triangle blocked the ray
+    auto pop = [&]() {
+        --sp;
+        int e;
+        if (sp < STACK_SHARED) e = top[sp][tid];
+        else e = stack[sp];
+        return e;
+    };
+    auto is_leaf = [&]() { return cur < 0 && cur > DEAD && inst >= 0; };
     for (;;) {
-        // a lane whose ray is done waits until fetch_batch lanes of the warp
-        // are (or all are): the result write and the next fetch and set-up
-        // then run for those lanes together instead of one lane at a time
-        const bool fin = ray < 0 || (count == 0 && inst < 0 && top == NONE && sp == 0);
-        const unsigned act = __activemask();
-        const unsigned idle = __ballot_sync(act, fin);
-        if (fin) {
-            if (idle != act && __popc(idle) < s.fetch_batch) continue;
-            if (ray >= 0) {
-                float3 o, d;
+        // ---- rays that are done wait until fetch_batch lanes of the warp
+        // are (or nobody else works), then store their results and fetch and
+        // set up their next rays together
+        const unsigned idle = __ballot_sync(FULL, cur == DONE), dead = __ballot_sync(FULL, cur == DEAD);
+        if (idle && ((idle | dead) == FULL || __popc(idle) >= s.fetch_batch)) {
+            bool more = false;
+            float3 wo, wd;
+            if (cur == DONE && ray >= 0) {
                 if (ANY) {
                     src.any(ray, occluded);
-                    ray = -1;
-                } else if (src.closest(ray, best, o, d)) {
-                    start(o, d);   // the next ray of a bounce chain
-                    continue;
                 } else {
-                    ray = -1;
+                    Hit h;
+                    h.t = best_t;
+                    h.inst = h.tri = -1;
+                    h.u = h.v = 0.0f;
+                    if (best_inst >= 0)
+                        h = hit_at(s, best_inst, best_slot, best_t,
+                                   make_float3(world[0][tid], world[1][tid], world[2][tid]),
+                                   make_float3(world[6][tid], world[7][tid], world[8][tid]));
+                    more = src.closest(ray, h, wo, wd);
                 }
             }
-            cg::coalesced_group g = cg::coalesced_threads();
-            int b = 0;
-            if (g.thread_rank() == 0) b = atomicAdd(next, (int)g.size());
-            ray = g.shfl(b, 0) + (int)g.thread_rank();
-            if (ray >= n) break;
-            float3 o, d;
-            src.ray(ray, o, d, tmin, tmax0);
-            start(o, d);
-            occluded = false;
-        } else if (count > 0) {
-            // TRI triangles of the leaf, in order (BLAS2::intersect /
-            // intersectP leaf loop)
-#pragma unroll
-            for (int k = 0; k < TRI; ++k) {
-                if (count == 0) break;
-                float u, v;
-                int lid;
-                const float tmx = ANY ? tmax0 : fminf(tmax0, loc.t);
-                float t = tri_test(s.tris + 3 * (size_t)first, r, tmin, tmx, &u, &v, &lid);
-                st.tri_tests++;
-                ++first;
-                --count;
-                if (ANY) {
-                    if (t < INF) {   // blocked: the ray is done
-                        occluded = true;
-                        count = 0;
-                        inst = -1;
-                        top = NONE;
-                        sp = 0;
+            const unsigned want = __ballot_sync(FULL, cur == DONE && !more);
+            int base = 0;
+            if (lane == 0 && want) base = atomicAdd(next, __popc(want));
+            base = __shfl_sync(FULL, base, 0);
+            if (cur == DONE) {
+                if (!more) {
+                    ray = base + __popc(want & ((1u << lane) - 1u));
+                    if (ray < n) {
+                        src.ray(ray, wo, wd, tmax);
+                        bound0 = next_up(tmax);
+                        more = true;
+                    } else {
+                        cur = DEAD;
                     }
-                } else if (t < loc.t) {
-                    loc.t = t;
-                    loc.tri = lid;
-                    loc.u = u;
-                    loc.v = v;
+                }
+                if (more) {
+                    // a new ray: the TLAS root box (TLAS::intersect, tlas.cu:60-75), then its root
+                    const XRay w = make_xray(wo, wd);
+                    o = w.o;
+                    inv = w.inv;
+                    d = w.d;
+                    world[0][tid] = o.x; world[1][tid] = o.y; world[2][tid] = o.z;
+                    world[3][tid] = inv.x; world[4][tid] = inv.y; world[5][tid] = inv.z;
+                    world[6][tid] = d.x; world[7][tid] = d.y; world[8][tid] = d.z;
+                    best_t = INF;
+                    best_inst = -1;
+                    bound = bound0;
+                    inst = -1;
+                    occluded = false;
+                    nodes = s.tlas;
+                    sp = 0;
+                    push(DONE);
+                    float4 lo, hi;
+                    int root, ninst;
+                    if constexpr (ROOTS) {
+                        src.root(ray, lo, hi, root, ninst);
+                    } else {
+                        lo = s.tlas_lo;
+                        hi = s.tlas_hi;
+                        root = s.tlas_root_leaf ? ~0 : 0;
+                        ninst = s.ninst;
+                    }
+                    float te;
+                    st.box_tests++;
+                    if (ninst > 0 && slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, w, tmin, tmax, &te)) cur = root;
                 }
             }
-        } else if (inst >= 0 && top == NONE && sp == base) {
-            // leaving the instance: merge its closest hit (tlas.cu:116-121)
-            if (!ANY && loc.t < best.t) {
-                best = loc;
-                best.inst = inst;
+            continue;
+        }
+        if (dead == FULL) break;
+        const int live = 32 - __popc(idle | dead);
+        // ---- interior nodes of the TLAS or of an instance's BLAS, until fewer
+        // than half of the live lanes step (3/8: 6.38 ms, 5/8: as 1/2, none: 7.4)
+        while (cur >= 0) {
+            float4 a, b, c, refs;
+            const float4* q = reinterpret_cast<const float4*>(nodes + cur);
+            load_half_node(q, a, b);
+            load_half_node(q + 2, c, refs);
+            // slab() of both child boxes (the ray's bound in one comparison)
+            const float l1x = xm(xs(a.x, o.x), inv.x), l1y = xm(xs(a.y, o.y), inv.y), l1z = xm(xs(a.z, o.z), inv.z);
+            const float h1x = xm(xs(a.w, o.x), inv.x), h1y = xm(xs(b.x, o.y), inv.y), h1z = xm(xs(b.y, o.z), inv.z);
+            const float l2x = xm(xs(b.z, o.x), inv.x), l2y = xm(xs(b.w, o.y), inv.y), l2z = xm(xs(c.x, o.z), inv.z);
+            const float h2x = xm(xs(c.y, o.x), inv.x), h2y = xm(xs(c.z, o.y), inv.y), h2z = xm(xs(c.w, o.z), inv.z);
+            const float t1 = fmaxf(fmaxf(fminf(l1x, h1x), fminf(l1y, h1y)), fminf(l1z, h1z));
+            const float x1 = fminf(fminf(fmaxf(l1x, h1x), fmaxf(l1y, h1y)), fmaxf(l1z, h1z));
+            const float t2 = fmaxf(fmaxf(fminf(l2x, h2x), fminf(l2y, h2y)), fminf(l2z, h2z));
+            const float x2 = fminf(fminf(fmaxf(l2x, h2x), fmaxf(l2y, h2y)), fmaxf(l2z, h2z));
+            const bool p1 = t1 <= x1 && x1 >= tmin && t1 < bound;
+            const bool p2 = t2 <= x2 && x2 >= tmin && t2 < bound;
+            st.box_tests += 2;
+            const int r1 = __float_as_int(refs.x), r2 = __float_as_int(refs.z);
+            const int c1 = __float_as_int(refs.y) ? ~r1 : r1, c2 = __float_as_int(refs.w) ? ~r2 : r2;
+            // the near child is next, the far one on the stack
+            const bool first = p1 && !(p2 && t1 > t2);
+            if (p1 && p2) push(first ? c2 : c1);
+            if (p1 || p2) cur = first ? c1 : c2;
+            else cur = pop();
+            if (2 * __popc(__activemask()) < live) break;
+        }
+        __syncwarp(FULL);
+        // ---- leaves, until fewer than an eighth of the live lanes have one
+        unsigned leaves = __ballot_sync(FULL, is_leaf());
+        while (leaves) {
+            const int nleaf = __popc(leaves);
+            const int shift = nleaf <= 4 ? 3 : 2, width = 1 << shift;
+            const unsigned gmask = (1u << width) - 1u;
+            const int rank = __popc(leaves & ((1u << lane) - 1u));
+            const bool mine = is_leaf() && rank < (32 >> shift);   // this lane's leaf is in the round
+            if (mine) owners[warp0 + rank] = lane;
+            __syncwarp(FULL);
+            const int g = lane >> shift, j = lane & (width - 1);   // group of lanes, its triangle
+            const bool act = g < nleaf;
+            const int owner = act ? owners[warp0 + g] : 0;
+            const int k = ~__shfl_sync(FULL, cur, owner) + j;
+            // BLAS2::intersect tests against min(tmax, closest so far), intersectP against tmax
+            const float limit = __shfl_sync(FULL, ANY ? tmax : fminf(tmax, bound), owner);
+            float t = INF;
+            bool last = false, hit = false;
+            if (act) {
+                // tri_test of record k (past the end of a leaf: another leaf's, or the array's padding)
+                const float4* tri = s.tris + 3 * (size_t)k;
+                const float4 a = __ldg(tri), b = __ldg(tri + 1), c = __ldg(tri + 2);
+                const int ow = warp0 + owner;
+                last = b.w != 0.0f;
+                const float3 e1 = make_float3(b.x, b.y, b.z), e2 = make_float3(c.x, c.y, c.z);
+                const float3 rd = make_float3(object[3][ow], object[4][ow], object[5][ow]);
+                const float3 pv = xcross(rd, e2);
+                const float det = xdot(e1, pv);
+                const float rdet = __frcp_rn(det);
+                const float3 tv = make_float3(xs(object[0][ow], a.x), xs(object[1][ow], a.y), xs(object[2][ow], a.z));
+                const float u = xm(rdet, xdot(tv, pv));
+                const float3 qv = xcross(tv, e1);
+                const float v = xm(rdet, xdot(rd, qv));
+                t = xm(rdet, xdot(e2, qv));
+                hit = !(det > -TRI_EPS && det < TRI_EPS) && !(u < 0.0f || u > 1.0f) &&
+                      !(v < 0.0f || xa(u, v) > 1.0f) && t > TRI_EPS && t < limit && t > tmin;
+            }
+            const unsigned ends = __ballot_sync(FULL, last);
+            if ((ends >> (lane - j)) & ((1u << j) - 1u)) hit = false;   // the leaf ended before this lane
+            else if (act) st.tri_tests++;
+            const unsigned hits = __ballot_sync(FULL, hit);
+            const int from = mine ? rank << shift : 0;                  // first lane of this lane's leaf's group
+            const bool my_hit = mine && ((hits >> from) & gmask), my_end = (ends >> from) & gmask;
+            const int first = ~cur;
+            if (mine) {
+                if (ANY && my_hit) {
+                    occluded = true;
+                    cur = DONE;
+                } else if (my_end) {
+                    cur = pop();
+                } else {
+                    cur -= width;   // the leaf's next triangles
+                }
+            }
+            if (!ANY && hits) {
+                // the group's closest hit, the first among equals
+                if (!hit) t = INF;
+                int jm = j;
+                for (int w = 1; w < width; w <<= 1) {
+                    const float t2 = __shfl_xor_sync(FULL, t, w);
+                    const int j2 = __shfl_xor_sync(FULL, jm, w);
+                    if (t2 < t || (t2 == t && j2 < jm)) {
+                        t = t2;
+                        jm = j2;
+                    }
+                }
+                const float ht = __shfl_sync(FULL, t, from);
+                const int hj = __shfl_sync(FULL, jm, from);
+                if (my_hit) {
+                    bound = ht;
+                    slot = first + hj;
+                }
+            }
+            leaves = __ballot_sync(FULL, is_leaf());
+            if (8 * __popc(leaves) < live) break;
+        }
+        // ---- instances
+        if (cur == LEAVE) {
+            // merge its closest hit (tlas.cu:116-121), back to the world ray
+            if (!ANY) {
+                if (slot >= 0 && bound < best_t) {
+                    best_t = bound;
+                    best_inst = inst;
+                    best_slot = slot;
+                }
+                bound = fminf(bound0, best_t);
             }
             inst = -1;
-            r = w;
-        } else {
-            const int e = top != NONE ? top : stack[--sp];
-            top = NONE;
-            if (e >= 0) {
-                // interior node of the TLAS or of the instance's BLAS
-                const bool in_blas = inst >= 0;
-                const BvhNode nd = load_node((in_blas ? s.nodes : s.tlas) + e);
-                const float cull = ANY ? INF : (in_blas ? loc.t : best.t);
-                const float tmx = (ANY || !in_blas) ? tmax0 : fminf(tmax0, loc.t);
-                bool h1, h2;
-                float t1, t2;
-                node_slabs(nd, r, tmin, tmx, &h1, &t1, &h2, &t2);
-                st.box_tests += 2;
-                const bool p1 = h1 && t1 < cull, p2 = h2 && t2 < cull;
-                if (in_blas ? (sp - base + 1 > BLAS_STACK) : (sp + 1 > TLAS_STACK)) {
-                    st.overflow++;
-                    sp = in_blas ? base : 0;   // the reference's stack would overflow: end this level
-                } else {
-                    const int c1 = nd.d.y ? (in_blas ? leaf_code(e, 0) : -nd.d.x - 1) : nd.d.x;
-                    const int c2 = nd.d.w ? (in_blas ? leaf_code(e, 1) : -nd.d.z - 1) : nd.d.z;
-                    // near child popped first: the far one goes to memory, the
-                    // near one stays in the register
-                    const bool far1 = t1 > t2;
-                    const int ca = far1 ? c1 : c2, cb = far1 ? c2 : c1;
-                    const bool pa = far1 ? p1 : p2, pb = far1 ? p2 : p1;
-                    if (pa && pb) stack[sp++] = ca;
-                    // the child visited next: a BLAS leaf starts at once, its
-                    // triangle range is in this node (no push, pop, setup step)
-                    const int cn = pb ? (far1 ? 1 : 0) : (far1 ? 0 : 1);
-                    const int ncount = cn ? nd.d.w : nd.d.y;
-                    if ((pa || pb) && in_blas && ncount > 0) {
-                        first = cn ? nd.d.z : nd.d.x;
-                        count = ncount;
-                        top = NONE;
-                    } else {
-                        top = pb ? cb : (pa ? ca : NONE);
-                    }
-                }
-            } else if (inst < 0) {
-                // entering an instance (TLAS leaf): object-space ray (Ray::transform)
-                inst = -e - 1;
-                const InstRec& ir = s.inst[inst];
-                const MeshRec m = s.meshes[ir.mesh];
-                const float4 inv[3] = {__ldg(&ir.inv[0]), __ldg(&ir.inv[1]), __ldg(&ir.inv[2])};
-                r = transform_xray(w, inv);
-                st.inst_xforms++;
-                base = sp;
-                loc.t = INF;
-                loc.tri = -1;
-                loc.u = loc.v = 0.0f;
-                if (m.node_root < 0) {
-                    first = m.leaf_first;
-                    count = m.leaf_count;
-                } else {
-                    top = m.node_root;
-                }
-            } else {
-                // BLAS leaf: its triangle range is read back from the parent node
-                const int c = -e - 1;
-                const int4 d = __ldg(reinterpret_cast<const int4*>(s.nodes + (c >> 1)) + 3);
-                first = (c & 1) ? d.z : d.x;
-                count = (c & 1) ? d.w : d.y;
-            }
+            nodes = s.tlas;
+            o = make_float3(world[0][tid], world[1][tid], world[2][tid]);
+            inv = make_float3(world[3][tid], world[4][tid], world[5][tid]);
+            d = make_float3(world[6][tid], world[7][tid], world[8][tid]);
+            cur = pop();
+        } else if (cur < 0 && cur > DEAD && inst < 0) {
+            // entering one (TLAS leaf): object-space ray (Ray::transform)
+            inst = ~cur;
+            const InstRec& ir = s.inst[inst];
+            const float4 m[3] = {__ldg(&ir.inv[0]), __ldg(&ir.inv[1]), __ldg(&ir.inv[2])};
+            XRay w;
+            w.o = o;
+            w.d = d;
+            const XRay r = transform_xray(w, m);
+            o = r.o;
+            inv = r.inv;
+            d = r.d;
+            object[0][tid] = o.x; object[1][tid] = o.y; object[2][tid] = o.z;
+            object[3][tid] = d.x; object[4][tid] = d.y; object[5][tid] = d.z;
+            st.inst_xforms++;
+            push(LEAVE);
+            nodes = s.nodes;
+            bound = bound0;
+            slot = -1;
+            cur = ir.root;
         }
     }
 }

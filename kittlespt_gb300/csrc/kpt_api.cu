@@ -1057,6 +1057,15 @@ static void stage_mark(kpt_context* c, int stage) {
     f->n++;
 }
 
+// The camera rays' closest hits and what follows from them (the miss and hit
+// lists, the visible surface).
+static void enqueue_primary(kpt_context* c, const FrameParams& F) {
+    const int np = c->W * c->H;
+    k_primary<<<persistent_grid(c, (const void*)k_primary, TRACE_BLOCK), TRACE_BLOCK, 0, c->stream>>>(F);
+    k_primary_surface<<<(np + PATH_BLOCK - 1) / PATH_BLOCK, PATH_BLOCK, 0, c->stream>>>(F);
+    c->launches += 2;
+}
+
 // The path stage: camera rays and their sky, then the wave(s) of paths level
 // by level, the queued sky and the ordered accumulation of every sample.
 // camera rays and their sky
@@ -1066,9 +1075,9 @@ static void enqueue_camera(kpt_context* c, const FrameParams& F) {
     cudaMemsetAsync(c->counts.p, 0, 4 * sizeof(int), s);
     stage_mark(c, KPT_STAGE_CAMERA);
     k_sky_constants<<<1, 32, 0, s>>>(F, c->sun_radiance.p);
-    k_primary<<<primary_blocks(c->W, c->H), PATH_BLOCK, 0, s>>>(F);
+    enqueue_primary(c, F);
     k_primary_sky<<<persistent_grid(c, (const void*)k_primary_sky, PATH_BLOCK), PATH_BLOCK, 0, s>>>(F);
-    c->launches += 3;
+    c->launches += 2;
 }
 
 // the start of a wave: its level counters cleared; with `mark`, the sky
@@ -1847,9 +1856,9 @@ static kpt_status adjoint_run(kpt_context* c, int sample0, int nsamples, const f
     KPT_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork[0], 0));
     k_adjoint_constants<<<1, 32, 0, c->side>>>(F, A);
     KPT_CUDA(cudaEventRecord(c->ev_join[0], c->side));
-    k_primary<<<primary_blocks(c->W, c->H), PATH_BLOCK, 0, s>>>(F);
+    enqueue_primary(c, F);
     k_adjoint_miss<<<c->sm_count, PATH_BLOCK, smem, s>>>(F, A);
-    c->launches += 4;
+    c->launches += 3;
     if (rec) {
         // the frozen-path records: one thread replays one sample
         KPT_CUDA(cudaStreamWaitEvent(s, c->ev_join[0], 0));
@@ -1987,7 +1996,7 @@ kpt_status kpt_adjoint_forward_device(kpt_context* c, int sample0, int nsamples,
     KPT_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork[0], 0));
     k_adjoint_constants<<<1, 32, 0, c->side>>>(F, A);
     KPT_CUDA(cudaEventRecord(c->ev_join[0], c->side));
-    k_primary<<<primary_blocks(c->W, c->H), PATH_BLOCK, 0, s>>>(F);
+    enqueue_primary(c, F);
     k_adjoint_miss<<<c->sm_count, PATH_BLOCK, smem, s>>>(F, A);   // the missing pixels' image
     for (int l = 0; l <= D; ++l) {
         if (l > 0) k_extend<<<g_ext, TRACE_BLOCK, 0, s>>>(F, l);
@@ -1997,7 +2006,7 @@ kpt_status kpt_adjoint_forward_device(kpt_context* c, int sample0, int nsamples,
     k_adj_sky<<<g_vtx, PATH_BLOCK, 0, s>>>(F, A, 0);
     k_adj_sweep<<<grid, PATH_BLOCK, smem, s>>>(F, A, 0);   // the hit pixels' image
     KPT_CUDA(cudaStreamWaitEvent(s, c->ev_join[0], 0));
-    c->launches += 7 + 3 * D;
+    c->launches += 6 + 3 * D;
     KPT_CUDA(cudaGetLastError());
     kpt_context::AdjForward& K = c->adj_fwd;
     K.F = F;

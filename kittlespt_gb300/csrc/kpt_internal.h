@@ -10,13 +10,8 @@ constexpr int PATH_BLOCK = 128;    // threads per block of the shading kernels
 constexpr int SHADE_MAX_BLOCK = 256;   // largest block k_shade is launched with (kpt_tuning.shade_block)
 constexpr int SHADE_WINDOW = 2048;     // largest window of paths k_shade regroups by lobe family (kpt_tuning.group_lobes)
 constexpr int TRACE_BLOCK = 128;   // threads per block of the ray kernels
-// k_primary: a warp traces a TILE_W x (32 / TILE_W) tile of pixels, a
-// block of PATH_BLOCK = 128 threads a 2 x 2 arrangement of them
-#ifndef KPT_TILE_W
-#define KPT_TILE_W 8
-#endif
-constexpr int TILE_W = KPT_TILE_W, TILE_H = 32 / KPT_TILE_W;
-inline int primary_blocks(int W, int H) { return ((W + 2 * TILE_W - 1) / (2 * TILE_W)) * ((H + 2 * TILE_H - 1) / (2 * TILE_H)); }
+// tiles of pixels that the lanes of a warp take together in the camera stage
+constexpr int TILE_W = 8, TILE_H = 4;
 #ifndef KPT_TRACE_MIN_BLOCKS
 #define KPT_TRACE_MIN_BLOCKS 8
 #endif
@@ -76,7 +71,8 @@ struct FrameParams {
     int* hit_list;             // [H*W] pixels whose camera ray hits, compacted
     int* hit_index;            // [H*W] position in hit_list, -1 for a miss
     int* miss_list;            // [H*W] pixels whose camera ray misses, compacted
-    int* counts;               // [0] hits, [1] misses, [2] queued sky evaluations (zeroed per frame)
+    int* counts;               // [0] hits, [1] misses, [2] queued sky evaluations, [3] fetch counter of the
+                               // camera rays (zeroed per frame)
     float4* pixel_sky;         // [H*W] sky radiance (times LeSun) of a missing camera ray
     float4* radiance;          // [hits][nsamples] path radiance before clamping (item = hit * nsamples + sample)
     float4* sky_queue;         // [2 per entry] (item bits, direction), (throughput, 0)
@@ -201,6 +197,7 @@ struct BatchQueues {
 
 // kernels (kpt_path.cu, fast maths)
 __global__ void k_primary(FrameParams F);
+__global__ void k_primary_surface(FrameParams F);
 __global__ void k_primary_sky(FrameParams F);
 __global__ void k_shade(FrameParams F, int level, long long wave0);        // blocks of <= PATH_BLOCK threads
 __global__ void k_shade_wide(FrameParams F, int level, long long wave0);   // blocks of <= SHADE_MAX_BLOCK threads

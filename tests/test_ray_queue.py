@@ -2,7 +2,8 @@
 the oracle bit for bit: leaves of 1 to 9 triangles and one of 40 (a group of
 lanes tests 4 or 8 of a leaf at a time), queues of fewer rays than the grid
 has warps, of about one ray per warp and of several warps' worth, ray ranges
-that end at, before and after a hit, and meshes whose root is a leaf."""
+that end at, before and after a hit, meshes whose root is a leaf, and the
+camera rays' tiles over ragged images."""
 
 import numpy as np
 import pytest
@@ -10,7 +11,7 @@ import pytest
 from kittlespt_gb300 import scenes as S
 from oracle import oracle as O
 
-from tests.test_gpu_parity import bits, global_prim, make_renderer
+from tests.test_gpu_parity import bits, global_prim, make_renderer, render_samples
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -111,3 +112,19 @@ def test_occlusion_ranges(which, n):
     finally:
         r.shutdown()
     np.testing.assert_array_equal(out.cpu().numpy() != 0, t < tmax)
+
+
+@pytest.mark.parametrize("w,h", [(8, 4), (9, 5), (1, 33), (7, 3), (257, 2), (40, 31)])
+def test_camera_tiles(w, h):
+    """Every pixel of images that 8 x 4 tiles cover exactly, with narrow and
+    low tiles at the edges, or only with those: first hits and albedo."""
+    sc = S.scene_small(w, h, 1, 1)
+    ref = O.Scene(sc).render_samples(0, 1)
+    r = make_renderer(sc)
+    try:
+        rad, hit, alb = render_samples(r, sc, 1)
+    finally:
+        r.shutdown()
+    np.testing.assert_array_equal(global_prim(sc, hit[..., 0], hit[..., 1]), ref["first_hit"][..., 0])
+    on = ref["first_hit"][..., 0] >= 0
+    np.testing.assert_array_equal(bits(alb[..., :3][on]), bits(ref["albedo"][on][..., :3]))

@@ -84,14 +84,10 @@ __device__ __forceinline__ MatFactors mat_factors(const SceneView& s, const Surf
 
 // d(sun radiance)/d(sky parameters): the Nishita radiance towards the sun is
 // a per-frame constant (k_sky_constants), so is its Jacobian (in double
-// precision, see nishita_jacobian_d).
-__global__ void k_adjoint_constants(FrameParams F, AdjParams A) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const SkyParams& P = F.sky;
-        float3 J[SKY_PARAMS];
-        nishita_jacobian_d(P, make_float3(0.0f, P.earth_r + 1.0f, 0.0f), P.sun_dir, J);
-        for (int i = 0; i < SKY_PARAMS; ++i) A.sun_J[i] = J[i];
-    }
+// precision; one block).
+__global__ void __launch_bounds__(JACOBIAN_BLOCK) k_adjoint_constants(FrameParams F, AdjParams A) {
+    const SkyParams& P = F.sky;
+    nishita_jacobian_block(P, make_float3(0.0f, P.earth_r + 1.0f, 0.0f), P.sun_dir, A.sun_J);
 }
 
 // Sky radiance and its Jacobian for a list of directions (tests and tools):
@@ -826,6 +822,9 @@ __global__ void __launch_bounds__(TRACE_BLOCK, TRACE_MIN_BLOCKS) k_adj_shadow(Fr
     int stack[STACK_WORDS];
     TraceStats st = {0, 0, 0, 0};
     int* lc = F.level_counts + LEVEL_WORDS * level;
+    // the escapes cannot grow while this kernel runs (k_adj_shade(level) has
+    // ended, k_adj_shade(level + 1) waits for it): their number ends level's range
+    if (blockIdx.x == 0 && threadIdx.x == 0) lc[5] = *A.esc_count;
     AdjShadowQueue q{F.shadow, A.vis + (size_t)level * F.cap, lc[1], F.cap};
     trace_queue<true>(F.scene, lc[1] + lc[2], lc + 4, q, st, stack);
 }
@@ -840,13 +839,16 @@ static __device__ __noinline__ void sky_jacobian_now(const SkyParams& P, float3 
     for (int q = 0; q < SKY_PARAMS; ++q) atomicAdd(slots + q, (double)wdot(w, J[q]));
 }
 
-// The sky radiance at the end of every escaped path of the wave (the
-// forward's march), for k_adj_sweep.
-__global__ void __launch_bounds__(PATH_BLOCK) k_adj_sky(FrameParams F, AdjParams A, long long) {
+// The sky radiance at the end of the paths that escaped at `level` (the
+// forward's march), for k_adj_sweep: from the end of level - 1's escapes to
+// the number k_adj_shadow(level) recorded.
+__global__ void __launch_bounds__(PATH_BLOCK) k_adj_sky(FrameParams F, AdjParams A, int level) {
     const SkyParams& P = F.sky;
     const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);
-    const int n = *A.esc_count;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const int* mark = F.level_counts + 5;
+    const int n = mark[LEVEL_WORDS * level];
+    for (int q = mark[LEVEL_WORDS * (level - 1)] + blockIdx.x * blockDim.x + threadIdx.x; q < n;
+         q += gridDim.x * blockDim.x) {
         const int i = A.esc[q];
         const float3 s = nishita(P, obs, xyz3(A.vend[2 * (size_t)i]));
         A.vsky[i] = make_float4(s.x, s.y, s.z, 0.0f);

@@ -375,6 +375,120 @@ static __device__ __noinline__ void nishita_jacobian_d(const SkyParams& P, float
     for (int i = 0; i < SKY_PARAMS; ++i) J[i] = make_float3((float)j[i][0], (float)j[i][1], (float)j[i][2]);
 }
 
+// nishita_jacobian_d by one block of JACOBIAN_BLOCK threads, every sum in its
+// order: 16 x 8 threads take the light samples and 16 the view samples, 16
+// sum each view sample's light samples and optical depths and form its
+// transmittances, 30 sum the integrals over the view samples.  One thread
+// doing all of it took 572 us -- a serial chain of ~400 double-precision
+// exponentials and square roots, and most of a small gradient evaluation;
+// this takes 34 us.
+__device__ __forceinline__ void nishita_jacobian_block(const SkyParams& P, float3 of, float3 df, float3* J) {
+    __shared__ double light[4][16][8];     // per light sample: depths and their height derivatives (R, M)
+    __shared__ bool above[16][8];          // the sample is above the ground
+    __shared__ double view[4][16];         // per view sample: pR, pM, dpR, dpM
+    __shared__ double depth[4][16];        // sr, sm, dsr, dsm
+    __shared__ double trans[16][3];
+    __shared__ bool lit[16];
+    __shared__ double sums[30];
+    const int tid = threadIdx.x;
+    const D3 o = d3(of), d = d3(df), sun = d3(P.sun_dir);
+    double te, tx, tmin = 0.0, tmax = 1.0e300;
+    if (!sphere_hit_d(o, d, P.atm_r, &te, &tx) || tx < 0.0) {
+        if (tid < SKY_PARAMS) J[tid] = make_float3(0.0f, 0.0f, 0.0f);
+        return;
+    }
+    if (te > tmin && te > 0.0) tmin = te;
+    if (tx < tmax) tmax = tx;
+    const double sR[3] = {P.sigma_r.x, P.sigma_r.y, P.sigma_r.z}, sM = P.sigma_m, tM = (double)P.sigma_m + P.sigma_am;
+    const double hr = P.h_r, hm = P.h_m, er = P.earth_r;
+    const double step = (tmax - tmin) / 16.0, half = 0.5 * step;
+    if (tid < 144) {
+        const bool sun_side = tid < 128;
+        const int i = sun_side ? tid >> 3 : tid - 128, j = tid & 7;
+        double t = tmin;
+        for (int k = 0; k < i; ++k) t += step;
+        const double s = t + half;
+        const D3 sp = {o.x + s * d.x, o.y + s * d.y, o.z + s * d.z};
+        if (sun_side) {
+            double lte, ltx;
+            sphere_hit_d(sp, sun, P.atm_r, &lte, &ltx);
+            const double lstep = ltx / 8.0;
+            const double ls = (j + 0.5) * lstep;
+            const D3 q = {sp.x + ls * sun.x, sp.y + ls * sun.y, sp.z + ls * sun.z};
+            const double altl = sqrt(ddot(q, q)) - er;
+            const double eR = exp(-altl / hr) * lstep, eM = exp(-altl / hm) * lstep;
+            above[i][j] = !(altl < 0.0);
+            light[0][i][j] = eR;
+            light[1][i][j] = eM;
+            light[2][i][j] = eR * altl / (hr * hr);
+            light[3][i][j] = eM * altl / (hm * hm);
+        } else {
+            const double alt = sqrt(ddot(sp, sp)) - er;
+            const double pR = exp(-alt / hr) * step, pM = exp(-alt / hm) * step;
+            view[0][i] = pR;
+            view[1][i] = pM;
+            view[2][i] = pR * alt / (hr * hr);
+            view[3][i] = pM * alt / (hm * hm);
+        }
+    }
+    __syncthreads();
+    if (tid < 16) {
+        double own[4] = {0.0, 0.0, 0.0, 0.0}, sunward[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int k = 0; k <= tid; ++k)
+            for (int q = 0; q < 4; ++q) own[q] += view[q][k];
+        bool all = true;
+        for (int k = 0; k < 8; ++k) {
+            all = all && above[tid][k];
+            for (int q = 0; q < 4; ++q) sunward[q] += light[q][tid][k];
+        }
+        lit[tid] = all;
+        const double sr = own[0] + sunward[0], sm = own[1] + sunward[1];
+        depth[0][tid] = sr;
+        depth[1][tid] = sm;
+        depth[2][tid] = own[2] + sunward[2];
+        depth[3][tid] = own[3] + sunward[3];
+        for (int c = 0; c < 3; ++c) trans[tid][c] = exp(-(sR[c] * sr + tM * sm));
+    }
+    __syncthreads();
+    if (tid < 30) {
+        // integral of the transmittance (kind 0) or of its derivative for parameter kind - 1, channel c,
+        // over the Rayleigh (species 0) or Mie density
+        const int c = tid % 3, species = (tid / 3) & 1, kind = tid / 6;
+        double acc = 0.0;
+        for (int i = 0; i < 16; ++i) {
+            if (!lit[i]) continue;
+            const double Tr = trans[i][c], p = view[species][i];
+            if (kind == 0) {
+                acc += Tr * p;
+                continue;
+            }
+            const double dtau = kind == 1 ? depth[0][i] : kind == 2 ? depth[1][i] : kind == 3 ? sR[c] * depth[2][i] : tM * depth[3][i];
+            const double dTr = Tr == 0.0 ? 0.0 : -Tr * dtau;
+            acc += dTr * p;
+            if (kind == 3 + species) acc += Tr * view[2 + species][i];
+        }
+        sums[tid] = acc;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        const double mu = ddot(d, sun);
+        const double rp = 3.0 * (1.0 + mu * mu) / (16.0 * 3.14159265358979323846);
+        const double g = 0.76;
+        const double den = (8.0 * 3.14159265358979323846) * ((2.0 + g * g) * pow(1.0 + g * g - 2.0 * g * mu, 1.5));
+        const double mp = 3.0 * ((1.0 - g * g) * (1.0 + mu * mu)) / den;
+        const double K = 6.0e5 * (double)P.sun_emission;
+        auto I = [&](int kind, int species, int c) { return sums[6 * kind + 3 * species + c]; };
+        double j[SKY_PARAMS][3] = {};
+        for (int c = 0; c < 3; ++c) {
+            j[SKY_RAYLEIGH_R + c][c] = ((I(0, 0, c) + sR[c] * I(1, 0, c)) * rp + sM * I(1, 1, c) * mp) * K;
+            j[SKY_MIE][c] = (sR[c] * I(2, 0, c) * rp + (I(0, 1, c) + sM * I(2, 1, c)) * mp) * K;
+            j[SKY_RAYLEIGH_H][c] = (sR[c] * I(3, 0, c) * rp + sM * I(3, 1, c) * mp) * K;
+            j[SKY_MIE_H][c] = (sR[c] * I(4, 0, c) * rp + sM * I(4, 1, c) * mp) * K;
+        }
+        for (int i = 0; i < SKY_PARAMS; ++i) J[i] = make_float3((float)j[i][0], (float)j[i][1], (float)j[i][2]);
+    }
+}
+
 // nishita_jacobian_d in single precision, with the geometry rewritten so
 // that nothing cancels: the altitude of o + s d is h / (sqrt(R^2 + h) + R)
 // with h = |o + s d|^2 - R^2 = (|o|^2 - R^2) + s (2 o.d + s d.d) formed from

@@ -1776,6 +1776,62 @@ kpt_status kpt_set_tuning(kpt_context* c, const kpt_tuning* t) {
 
 static int adjoint_params(const kpt_context* c) { return 4 * (int)c->materials.size() + ADJ_SKY_PARAMS; }
 
+// What precedes the replay's waves: the sky's constants, the sun's
+// double-precision Jacobian (only the sweep reads it) beside the camera rays
+// on the sky stream, and there too, once the missing pixels are listed, what
+// they give.
+static kpt_status adjoint_camera(kpt_context* c, const FrameParams& F, const AdjParams& A, size_t smem) {
+    cudaStream_t s = c->stream;
+    k_sky_constants<<<1, 32, 0, s>>>(F, c->sun_radiance.p);
+    KPT_CUDA(cudaEventRecord(c->ev_fork[0], s));
+    KPT_CUDA(cudaStreamWaitEvent(c->sky, c->ev_fork[0], 0));
+    k_adjoint_constants<<<1, JACOBIAN_BLOCK, 0, c->sky>>>(F, A);
+    enqueue_primary(c, F);
+    KPT_CUDA(cudaEventRecord(c->ev_fork[0], s));
+    KPT_CUDA(cudaStreamWaitEvent(c->sky, c->ev_fork[0], 0));
+    k_adjoint_miss<<<c->sm_count, PATH_BLOCK, smem, c->sky>>>(F, A);
+    c->launches += 3;
+    return KPT_OK;
+}
+
+// The replay of the wave starting at item w0, level by level, as the frame's
+// paths: the shadow rays of level l on the side stream beside the extension
+// rays of level l + 1 (joined before k_adj_shade(l + 1), which reuses their
+// buffer), the sky of the paths that escaped at l on the sky stream after
+// them.  Ends with the stream waiting for both.
+static kpt_status adjoint_wave(kpt_context* c, const FrameParams& F, const AdjParams& A, long long w0) {
+    cudaStream_t s = c->stream;
+    const int D = F.max_depth;
+    const int g_ext = persistent_grid(c, (const void*)k_extend, TRACE_BLOCK);
+    const int g_shd = persistent_grid(c, (const void*)k_adj_shadow, TRACE_BLOCK);
+    const int g_vtx = persistent_grid(c, (const void*)k_adj_shade, PATH_BLOCK);
+    const int g_sky = persistent_grid(c, (const void*)k_adj_sky, PATH_BLOCK);
+    c->levels_depth = D;   // kpt_get_level_counts then reports the replay's last wave
+    KPT_CUDA(cudaMemsetAsync(c->level_counts.p, 0, sizeof(int) * LEVEL_WORDS * (size_t)(D + 2), s));
+    KPT_CUDA(cudaMemsetAsync(A.vis, 0, (size_t)(D + 1) * F.cap, s));
+    KPT_CUDA(cudaMemsetAsync(A.esc_count, 0, sizeof(int), s));
+    for (int l = 0; l <= D; ++l) {
+        if (l > 0) {
+            k_extend<<<g_ext, TRACE_BLOCK, 0, s>>>(F, l);
+            KPT_CUDA(cudaStreamWaitEvent(s, c->ev_join[l - 1], 0));
+        }
+        k_adj_shade<<<g_vtx, PATH_BLOCK, 0, s>>>(F, A, l, w0);
+        KPT_CUDA(cudaEventRecord(c->ev_fork[l], s));
+        KPT_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork[l], 0));
+        k_adj_shadow<<<g_shd, TRACE_BLOCK, 0, c->side>>>(F, A, l);
+        KPT_CUDA(cudaEventRecord(c->ev_join[l], c->side));
+        if (l > 0) {   // no path has left the scene at level 0
+            KPT_CUDA(cudaStreamWaitEvent(c->sky, c->ev_join[l], 0));
+            k_adj_sky<<<g_sky, PATH_BLOCK, 0, c->sky>>>(F, A, l);
+        }
+        c->launches += l > 0 ? 4 : 2;
+    }
+    KPT_CUDA(cudaStreamWaitEvent(s, c->ev_join[D], 0));
+    KPT_CUDA(cudaEventRecord(c->ev_sky, c->sky));
+    KPT_CUDA(cudaStreamWaitEvent(s, c->ev_sky, 0));
+    return KPT_OK;
+}
+
 static kpt_status adjoint_run(kpt_context* c, int sample0, int nsamples, const float* adjoint, double* grad,
                               float* image, AdjRec* rec, int max_rec) {
     c->adj_fwd.valid = false;
@@ -1849,19 +1905,12 @@ static kpt_status adjoint_run(kpt_context* c, int sample0, int nsamples, const f
     int per_sm = 0;
     KPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PATH_BLOCK, smem));
     const int grid = std::max(1, per_sm) * c->sm_count;
-    k_sky_constants<<<1, 32, 0, s>>>(F, c->sun_radiance.p);
-    // the sun's double-precision Jacobian (one thread) on the side stream: only
-    // the replay's sweep (or the records kernel) reads it
-    KPT_CUDA(cudaEventRecord(c->ev_fork[0], s));
-    KPT_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork[0], 0));
-    k_adjoint_constants<<<1, 32, 0, c->side>>>(F, A);
-    KPT_CUDA(cudaEventRecord(c->ev_join[0], c->side));
-    enqueue_primary(c, F);
-    k_adjoint_miss<<<c->sm_count, PATH_BLOCK, smem, s>>>(F, A);
-    c->launches += 3;
+    st = adjoint_camera(c, F, A, smem);
+    if (st != KPT_OK) return st;
     if (rec) {
         // the frozen-path records: one thread replays one sample
-        KPT_CUDA(cudaStreamWaitEvent(s, c->ev_join[0], 0));
+        KPT_CUDA(cudaEventRecord(c->ev_sky, c->sky));
+        KPT_CUDA(cudaStreamWaitEvent(s, c->ev_sky, 0));
         k_adjoint_rec<<<grid, PATH_BLOCK, smem, s>>>(F, A);
         c->launches += 1;
     } else {
@@ -1869,24 +1918,11 @@ static kpt_status adjoint_run(kpt_context* c, int sample0, int nsamples, const f
         // waves find no work when fewer do): per level the vertices, their
         // shadow rays and the continuations, then every sample's sweep
         const long long items = (long long)np * nsamples;
-        const int g_ext = persistent_grid(c, (const void*)k_extend, TRACE_BLOCK);
-        const int g_shd = persistent_grid(c, (const void*)k_adj_shadow, TRACE_BLOCK);
-        const int g_vtx = persistent_grid(c, (const void*)k_adj_shade, PATH_BLOCK);
-        c->levels_depth = D;   // kpt_get_level_counts then reports the replay's last wave
         for (long long w0 = 0; w0 < items; w0 += F.cap) {
-            KPT_CUDA(cudaMemsetAsync(c->level_counts.p, 0, sizeof(int) * LEVEL_WORDS * (size_t)(D + 2), s));
-            KPT_CUDA(cudaMemsetAsync(A.vis, 0, (size_t)(D + 1) * F.cap, s));
-            KPT_CUDA(cudaMemsetAsync(A.esc_count, 0, sizeof(int), s));
-            for (int l = 0; l <= D; ++l) {
-                if (l > 0) k_extend<<<g_ext, TRACE_BLOCK, 0, s>>>(F, l);
-                k_adj_shade<<<g_vtx, PATH_BLOCK, 0, s>>>(F, A, l, w0);
-                k_adj_shadow<<<g_shd, TRACE_BLOCK, 0, s>>>(F, A, l);
-                c->launches += l > 0 ? 3 : 2;
-            }
-            k_adj_sky<<<g_vtx, PATH_BLOCK, 0, s>>>(F, A, w0);
-            KPT_CUDA(cudaStreamWaitEvent(s, c->ev_join[0], 0));
+            st = adjoint_wave(c, F, A, w0);
+            if (st != KPT_OK) return st;
             k_adj_sweep<<<grid, PATH_BLOCK, smem, s>>>(F, A, w0);
-            c->launches += 2;
+            c->launches += 1;
         }
     }
     if (A.skyq) {
@@ -1977,36 +2013,16 @@ kpt_status kpt_adjoint_forward_device(kpt_context* c, int sample0, int nsamples,
     cudaStream_t s = c->stream;
     KPT_CUDA(cudaMemsetAsync(image, 0, sizeof(float4) * (size_t)np, s));
     KPT_CUDA(cudaMemsetAsync(c->counts.p, 0, 4 * sizeof(int), s));
-    KPT_CUDA(cudaMemsetAsync(c->level_counts.p, 0, sizeof(int) * LEVEL_WORDS * (size_t)(D + 2), s));
-    KPT_CUDA(cudaMemsetAsync(A.vis, 0, (size_t)(D + 1) * F.cap, s));
-    KPT_CUDA(cudaMemsetAsync(A.esc_count, 0, sizeof(int), s));
     for (const void* k : {(const void*)k_adj_sweep, (const void*)k_adjoint_miss})
         KPT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     KPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adj_sweep, PATH_BLOCK, smem));
     const int grid = std::max(1, per_sm) * c->sm_count;
-    const int g_ext = persistent_grid(c, (const void*)k_extend, TRACE_BLOCK);
-    const int g_shd = persistent_grid(c, (const void*)k_adj_shadow, TRACE_BLOCK);
-    const int g_vtx = persistent_grid(c, (const void*)k_adj_shade, PATH_BLOCK);
-    c->levels_depth = D;
-    k_sky_constants<<<1, 32, 0, s>>>(F, c->sun_radiance.p);
-    // the sun's double-precision Jacobian (one thread; it depends on the sky
-    // parameters only) on the side stream beside the replay, for the sweep
-    KPT_CUDA(cudaEventRecord(c->ev_fork[0], s));
-    KPT_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork[0], 0));
-    k_adjoint_constants<<<1, 32, 0, c->side>>>(F, A);
-    KPT_CUDA(cudaEventRecord(c->ev_join[0], c->side));
-    enqueue_primary(c, F);
-    k_adjoint_miss<<<c->sm_count, PATH_BLOCK, smem, s>>>(F, A);   // the missing pixels' image
-    for (int l = 0; l <= D; ++l) {
-        if (l > 0) k_extend<<<g_ext, TRACE_BLOCK, 0, s>>>(F, l);
-        k_adj_shade<<<g_vtx, PATH_BLOCK, 0, s>>>(F, A, l, 0);
-        k_adj_shadow<<<g_shd, TRACE_BLOCK, 0, s>>>(F, A, l);
-    }
-    k_adj_sky<<<g_vtx, PATH_BLOCK, 0, s>>>(F, A, 0);
+    st = adjoint_camera(c, F, A, smem);   // with the missing pixels' image
+    if (st == KPT_OK) st = adjoint_wave(c, F, A, 0);
+    if (st != KPT_OK) return st;
     k_adj_sweep<<<grid, PATH_BLOCK, smem, s>>>(F, A, 0);   // the hit pixels' image
-    KPT_CUDA(cudaStreamWaitEvent(s, c->ev_join[0], 0));
-    c->launches += 6 + 3 * D;
+    c->launches += 1;
     KPT_CUDA(cudaGetLastError());
     kpt_context::AdjForward& K = c->adj_fwd;
     K.F = F;
@@ -2055,8 +2071,12 @@ kpt_status kpt_adjoint_backward_device(kpt_context* c, const float* adjoint, dou
     KPT_CUDA(cudaMemsetAsync(A.skyq_count, 0, sizeof(int), s));
     KPT_CUDA(cudaMemsetAsync(A.skyqf_count, 0, sizeof(int), s));
     // (the sun's Jacobian, A.sun_J, came with the forward call)
-    k_adjoint_miss<<<c->sm_count, PATH_BLOCK, smem, s>>>(F, A);
+    KPT_CUDA(cudaEventRecord(c->ev_fork[0], s));
+    KPT_CUDA(cudaStreamWaitEvent(c->sky, c->ev_fork[0], 0));
+    k_adjoint_miss<<<c->sm_count, PATH_BLOCK, smem, c->sky>>>(F, A);
+    KPT_CUDA(cudaEventRecord(c->ev_sky, c->sky));
     k_adj_sweep<<<grid, PATH_BLOCK, smem, s>>>(F, A, 0);
+    KPT_CUDA(cudaStreamWaitEvent(s, c->ev_sky, 0));
     KPT_CUDA(cudaEventRecord(c->ev_fork[0], s));
     KPT_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork[0], 0));
     k_adjoint_sky_f<<<c->sm_count * 4, PATH_BLOCK, 0, c->side>>>(F, A);

@@ -81,7 +81,8 @@ struct FrameParams {
     PrimaryRec* hits;          // [cap] closest hits of the paths entering a level
     ShadowRec* shadow;         // [cap] shadow rays of a level: sun rays from the front, light rays from the back
     int* level_counts;         // [LEVEL_WORDS * (max_depth + 2)] zeroed per wave; word 5: sky queue
-                               // length after level l (of level max_depth + 1: at the wave's start)
+                               // length after level l (of level max_depth + 1: at the wave's start),
+                               // in the adjoint replay the wave's escapes after level l
     PathRec* unsorted;         // [cap] k_shade's continuations before the octant sort, null: no sort
     int* octants;              // [16 * (max_depth + 2)] per level: paths per direction octant, cursors
     int cap;
@@ -92,6 +93,7 @@ struct FrameParams {
 // path-replay adjoint (kpt_adjoint.cu)
 
 constexpr int ADJ_MAX_VERTICES = 17;   // max_depth <= 16
+constexpr int JACOBIAN_BLOCK = 160;    // threads of k_adjoint_constants
 constexpr int ADJ_SKY_PARAMS = 6;      // Rayleigh r, g, b, Mie, Rayleigh height, Mie height
 
 // One path vertex as the replay saw it, everything that is held fixed (for
@@ -231,7 +233,7 @@ __global__ void k_adjoint_sky_f(FrameParams F, AdjParams A);
 __global__ void k_adj_shade(FrameParams F, AdjParams A, int level, long long wave0);
 __global__ void k_adj_shadow(FrameParams F, AdjParams A, int level);
 __global__ void k_adj_sweep(FrameParams F, AdjParams A, long long wave0);
-__global__ void k_adj_sky(FrameParams F, AdjParams A, long long wave0);
+__global__ void k_adj_sky(FrameParams F, AdjParams A, int level);
 // kpt_post.cu (IEEE): clamp and add the samples of each pixel in sample order
 // Temporal accumulation (kernels.cu:164-327): per instance, the matrices of
 // computeVelocity and testReprojection for one frame, rows of column-major

@@ -24,7 +24,7 @@ __device__ __forceinline__ float ggx_D_grad(float alpha, float3 wm, float* dD) {
     if (floor) a = fmaxf(a, 1.0e-3f);
     float a2 = Sqr(a);
     float ndh = Sqr(saturatef_(wm.z));
-    float b = (float)((double)ndh * ((double)a2 - 1.0) + 1.0);
+    float b = ggx_b(ndh, a2);
     float D = a2 / (PI_F * Sqr(b));
     // dD/da2 = (b - 2 a2 ndh) / (pi b^3); a2 = alpha^2 unless floored
     *dD = floor ? 0.0f : ((b - 2.0f * a2 * ndh) / (PI_F * b * b * b)) * (2.0f * a);

@@ -545,7 +545,8 @@ __global__ void __launch_bounds__(PATH_BLOCK) k_adjoint_rec(FrameParams F, AdjPa
 
 __device__ __forceinline__ float3 xyz3(float4 v) { return make_float3(v.x, v.y, v.z); }
 
-__global__ void __launch_bounds__(PATH_BLOCK, 6) k_adj_shade(FrameParams F, AdjParams A, int level, long long wave0) {
+// (held to 96 registers: at 80 the same gradient takes 6.61 ms, not 6.52; at 128, 6.56)
+__global__ void __launch_bounds__(PATH_BLOCK, 5) k_adj_shade(FrameParams F, AdjParams A, int level, long long wave0) {
     constexpr int MV = ADJ_MAX_VERTICES;
     const SceneView& s = F.scene;
     const SkyParams& P = F.sky;
@@ -855,17 +856,87 @@ __global__ void __launch_bounds__(PATH_BLOCK) k_adj_sky(FrameParams F, AdjParams
     }
 }
 
+// Adds the lanes' v (to the gradients of material mat's four parameters) to
+// the block's sums: per material among the lanes of the full warp, one
+// exchange that leaves each quarter of the warp one parameter to sum, six
+// double additions and four atomic adds.  (Lanes without a vertex: mat < 0.)
+__device__ __forceinline__ void grad_add_warp(double* sg, int mat, const float* v) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    unsigned todo = __ballot_sync(FULL, mat >= 0 && (v[0] != 0.0f || v[1] != 0.0f || v[2] != 0.0f || v[3] != 0.0f));
+    while (todo) {
+        const int m = __shfl_sync(FULL, mat, __ffs(todo) - 1);
+        const bool mine = mat == m;
+        todo &= ~__ballot_sync(FULL, mine);
+        const bool high = lane & 16, odd = lane & 8;
+        // parameters 0, 1 stay in the low half of the warp, 2, 3 in the high half
+        const float k0 = mine ? (high ? v[2] : v[0]) : 0.0f, k1 = mine ? (high ? v[3] : v[1]) : 0.0f;
+        const float s0 = mine ? (high ? v[0] : v[2]) : 0.0f, s1 = mine ? (high ? v[1] : v[3]) : 0.0f;
+        const float r0 = __shfl_xor_sync(FULL, s0, 16), r1 = __shfl_xor_sync(FULL, s1, 16);
+        const double d0 = (double)k0 + (double)r0, d1 = (double)k1 + (double)r1;
+        double d = odd ? d1 : d0;
+        d += __shfl_xor_sync(FULL, odd ? d0 : d1, 8);
+        d += __shfl_xor_sync(FULL, d, 4);
+        d += __shfl_xor_sync(FULL, d, 2);
+        d += __shfl_xor_sync(FULL, d, 1);
+        if ((lane & 7) == 0 && d != 0.0) atomicAdd(sg + 4 * m + (lane >> 3), d);
+    }
+}
+
+// Adds each lane's c to image[p]: neighbouring lanes of one pixel (items are
+// pixel-major) are summed first.  Lanes without a sample: p < 0.
+__device__ __forceinline__ void image_add_warp(float4* image, int p, float3 c) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int q = __shfl_down_sync(FULL, p, o);
+        const float x = __shfl_down_sync(FULL, c.x, o), y = __shfl_down_sync(FULL, c.y, o), z = __shfl_down_sync(FULL, c.z, o);
+        if (lane + o < 32 && q == p) {
+            c.x += x;
+            c.y += y;
+            c.z += z;
+        }
+    }
+    const int before = __shfl_up_sync(FULL, p, 1);
+    if (p >= 0 && (lane == 0 || before != p)) {
+        atomicAdd(&image[p].x, c.x);
+        atomicAdd(&image[p].y, c.y);
+        atomicAdd(&image[p].z, c.z);
+    }
+}
+
+// dLoss/d(radiance of the sample) of path radiance L at pixel p: the adjoint
+// image on the unclamped channels, over the samples.
+__device__ __forceinline__ float3 sample_weight(const AdjParams& A, int p, float3 L, float inv_n, float3* clamped) {
+    float3 msk;
+    *clamped = make_float3(clamp_out(L.x, &msk.x), clamp_out(L.y, &msk.y), clamp_out(L.z, &msk.z));
+    if (!A.adjoint) return make_float3(0.0f, 0.0f, 0.0f);
+    const float4 a = A.adjoint[p];
+    return make_float3(a.x, a.y, a.z) * msk * inv_n;
+}
+
+// Queues the sky Jacobian of an escaped path (its last direction and
+// throughput) with its gradient weight.
+__device__ __forceinline__ void queue_escape(const AdjParams& A, const SkyParams& P, float3 obs, float3 d, float3 beta,
+                                             float3 g, double* sky_slots) {
+    const float3 gb = wmul(g, beta);
+    const bool band = sky_in_band(P, d);
+    const bool done = band ? sky_defer(A, d, gb) : sky_push(A.skyqf, A.skyqf_count, A.skyqf_cap, d, gb);
+    if (!done) sky_jacobian_now(P, obs, d, band, gb, sky_slots);
+}
+
 // Every sample of the wave: its radiance from the vertex records (the
 // forward's sum), clamp, image, and the reverse sweep into the gradients.
-// the sweep and the vertex replay are held to 64 and 85 registers: left to
-// 193 and 110 they keep 8 and 16 warps per SM on latency-bound loads (the
-// sweep's spills cost less than the warps it gains)
+// Forward half: bound by the latency of the records' loads (held to 64
+// registers: left to 193 it keeps 8 warps per SM); backward half: by the FP64
+// pipe (72% busy, 1/64 of the FP32 rate).  512x512x32 samples, depth 6: 278 us
+// and 541 us; with an atomic add per lane, parameter and image channel, 363
+// and 784.
 __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjParams A, long long wave0) {
     extern __shared__ double sg[];
     const int ng = 4 * A.nmat + ADJ_SKY_PARAMS;
     grad_begin(sg, ng);
-    GradAcc acc{sg};
-    double gsky[SKY_PARAMS] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     // the sun light samples' weights, summed: their sky gradient is linear in
     // the sun's Jacobian, applied once at the end
     double cs0 = 0.0, cs1 = 0.0, cs2 = 0.0;
@@ -877,99 +948,102 @@ __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjP
     const long long left = (long long)nhit * F.nsamples - wave0;
     const int n = (int)(left < 0 ? 0 : (left < cap ? left : cap));
     const float inv_n = 1.0f / (float)F.nsamples;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const long long item = wave0 + i;
-        const int p = F.hit_list[item / F.nsamples];
-        const float4 e0 = A.vend[2 * (size_t)i], e1 = A.vend[2 * (size_t)i + 1];
-        const int nv = __float_as_int(e0.w);
-        const bool escaped = __float_as_int(e1.w) != 0;
-        const float3 d_end = xyz3(e0), b_end = xyz3(e1);
-        const float3 s_end = escaped ? xyz3(A.vsky[i]) : make_float3(0.0f, 0.0f, 0.0f);
+    // whole warps: every lane takes part in the warp's sums
+    for (int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += gridDim.x * blockDim.x) {
+        const int i = i0 + (threadIdx.x & 31);
+        const bool in = i < n;
+        int p = -1, nv = 0;
+        float3 g = make_float3(0.0f, 0.0f, 0.0f), R = g, Lc = g;
         // c of vertex k: its emission, plus its light sample where visible
-        auto vertex_c = [&](int k, float4 emit, bool* vis_nee) {
+        auto vertex_c = [&](const float4* v, float4 emit, bool vis) {
             const float3 c = xyz3(emit);
-            const int nee = __float_as_int(emit.w);
-            *vis_nee = nee != 0 && A.vis[(size_t)k * cap + i] != 0;
-            if (!*vis_nee) return c;
-            const float3 fcos = xyz3(A.vr[((size_t)k * cap + i) * AV_FIELDS + AV_FCOS]);
-            const float3 kk = xyz3(A.vr[((size_t)k * cap + i) * AV_FIELDS + AV_K]);
-            return nee == 1 ? c + fcos * sun_rad * kk.x : c + fcos * kk;
+            if (!vis) return c;
+            const float3 fcos = xyz3(v[AV_FCOS]);
+            const float3 kk = xyz3(v[AV_K]);
+            return __float_as_int(emit.w) == 1 ? c + fcos * sun_rad * kk.x : c + fcos * kk;
         };
-        // the path's radiance: summed over its vertices, or (the backward
-        // half of a split adjoint) as the forward half stored it
-        float3 L = make_float3(0.0f, 0.0f, 0.0f);
-        if (A.lpath_ready) {
-            L = xyz3(A.lpath[i]);
-        } else {
+        if (in) {
+            const long long item = wave0 + i;
+            p = F.hit_list[item / F.nsamples];
+            const float4 e0 = A.vend[2 * (size_t)i], e1 = A.vend[2 * (size_t)i + 1];
+            nv = __float_as_int(e0.w);
+            const bool escaped = __float_as_int(e1.w) != 0;
+            const float3 d_end = xyz3(e0), b_end = xyz3(e1);
+            const float3 s_end = escaped ? xyz3(A.vsky[i]) : make_float3(0.0f, 0.0f, 0.0f);
+            // the path's radiance: summed over its vertices, or (the backward
+            // half of a split adjoint) as the forward half stored it
+            float3 L = make_float3(0.0f, 0.0f, 0.0f);
+            if (A.lpath_ready) {
+                L = xyz3(A.lpath[i]);
+            } else {
 #pragma unroll 1
-            for (int k = 0; k < nv; ++k) {
-                bool v;
-                const float3 b = xyz3(A.vr[((size_t)k * cap + i) * AV_FIELDS + AV_BETA]);
-                L = L + b * vertex_c(k, A.vr[((size_t)k * cap + i) * AV_FIELDS + AV_EMIT], &v);
-            }
-            if (escaped) L = L + b_end * s_end;
-            if (A.lpath) A.lpath[i] = make_float4(L.x, L.y, L.z, 0.0f);
-        }
-        float3 msk;
-        const float3 Lc = make_float3(clamp_out(L.x, &msk.x), clamp_out(L.y, &msk.y), clamp_out(L.z, &msk.z));
-        if (A.image) {
-            atomicAdd(&A.image[p].x, Lc.x * inv_n);
-            atomicAdd(&A.image[p].y, Lc.y * inv_n);
-            atomicAdd(&A.image[p].z, Lc.z * inv_n);
-        }
-        if (!A.adjoint) continue;   // the forward half of a split adjoint: the image only
-        const float4 a = A.adjoint[p];
-        const float3 g = make_float3(a.x, a.y, a.z) * msk * inv_n;
-        if (!nonzero(g)) continue;
-        float3 R = escaped ? s_end : make_float3(0.0f, 0.0f, 0.0f);
-        if (escaped) {
-            const float3 gb = wmul(g, b_end);
-            const bool band = sky_in_band(P, d_end);
-            const bool done = band ? sky_defer(A, d_end, gb)
-                                   : sky_push(A.skyqf, A.skyqf_count, A.skyqf_cap, d_end, gb);
-            if (!done) sky_jacobian_now(P, obs, d_end, band, gb, sg + 4 * A.nmat);
-        }
-#pragma unroll 1
-        for (int k = nv - 1; k >= 0; --k) {
-            const size_t o = (size_t)k * cap + i;
-            const float4 b4 = A.vr[o * AV_FIELDS + AV_BETA];
-            bool v;
-            const float3 ck = vertex_c(k, A.vr[o * AV_FIELDS + AV_EMIT], &v);
-            float3 dca = make_float3(0.0f, 0.0f, 0.0f), dcr = dca, cs = dca;
-            if (v) {
-                const int nee = __float_as_int(A.vr[o * AV_FIELDS + AV_EMIT].w);
-                const float3 kk = xyz3(A.vr[o * AV_FIELDS + AV_K]);
-                const float3 da = xyz3(A.vr[o * AV_FIELDS + AV_DA]), dl = xyz3(A.vr[o * AV_FIELDS + AV_DAL]);
-                if (nee == 1) {
-                    dca = da * sun_rad * kk.x;
-                    dcr = dl * sun_rad * kk.x;
-                    cs = xyz3(A.vr[o * AV_FIELDS + AV_FCOS]) * kk.x;
-                } else {
-                    dca = da * kk;
-                    dcr = dl * kk;
+                for (int k = 0; k < nv; ++k) {
+                    const size_t o = (size_t)k * cap + i;
+                    const float4* v = A.vr + o * AV_FIELDS;
+                    const float3 b = xyz3(v[AV_BETA]);
+                    const float4 emit = v[AV_EMIT];
+                    const bool vis = A.vis[o] != 0 && __float_as_int(emit.w) != 0;
+                    L = L + b * vertex_c(v, emit, vis);
                 }
+                if (escaped) L = L + b_end * s_end;
+                if (A.lpath) A.lpath[i] = make_float4(L.x, L.y, L.z, 0.0f);
             }
-            const float3 gb = wmul(g, xyz3(b4));
-            const float3 dwa = xyz3(A.vr[o * AV_FIELDS + AV_DWA]), dwr = xyz3(A.vr[o * AV_FIELDS + AV_DWR]);
-            const float3 ta = wmul(gb, dca + wmul(dwa, R));
-            const int m4 = 4 * __float_as_int(b4.w);
-            acc.add(m4 + 0, ta.x);
-            acc.add(m4 + 1, ta.y);
-            acc.add(m4 + 2, ta.z);
-            acc.add(m4 + 3, wdot(gb, dcr + wmul(dwr, R)));
-            if (nonzero(cs)) {
-                const float3 gs = wmul(gb, cs);
-                cs0 += gs.x;
-                cs1 += gs.y;
-                cs2 += gs.z;
+            g = sample_weight(A, p, L, inv_n, &Lc);
+            if (A.adjoint) {
+                R = s_end;
+                if (!nonzero(g)) nv = 0;
+                else if (escaped)
+                    queue_escape(A, P, obs, d_end, b_end, g, sg + 4 * A.nmat);
             }
-            R = ck + xyz3(A.vr[o * AV_FIELDS + AV_W]) * R;
+        }
+        if (A.image) image_add_warp(A.image, p, Lc * inv_n);
+        if (!A.adjoint) continue;   // the forward half of a split adjoint: the image only
+#pragma unroll 1
+        for (int k = __reduce_max_sync(0xffffffffu, nv) - 1; k >= 0; --k) {
+            int mat = -1;
+            float add[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (k < nv) {
+                const size_t o = (size_t)k * cap + i;
+                const float4* v = A.vr + o * AV_FIELDS;
+                const float4 b4 = v[AV_BETA], emit = v[AV_EMIT];
+                const bool vis = A.vis[o] != 0 && __float_as_int(emit.w) != 0;
+                const float3 wk = xyz3(v[AV_W]), dwa = xyz3(v[AV_DWA]), dwr = xyz3(v[AV_DWR]);
+                const float3 ck = vertex_c(v, emit, vis);
+                float3 dca = make_float3(0.0f, 0.0f, 0.0f), dcr = dca, cs = dca;
+                if (vis) {
+                    const float3 kk = xyz3(v[AV_K]);
+                    const float3 da = xyz3(v[AV_DA]), dl = xyz3(v[AV_DAL]);
+                    if (__float_as_int(emit.w) == 1) {
+                        dca = da * sun_rad * kk.x;
+                        dcr = dl * sun_rad * kk.x;
+                        cs = xyz3(v[AV_FCOS]) * kk.x;
+                    } else {
+                        dca = da * kk;
+                        dcr = dl * kk;
+                    }
+                }
+                const float3 gb = wmul(g, xyz3(b4));
+                const float3 ta = wmul(gb, dca + wmul(dwa, R));
+                mat = __float_as_int(b4.w);
+                add[0] = ta.x;
+                add[1] = ta.y;
+                add[2] = ta.z;
+                add[3] = wdot(gb, dcr + wmul(dwr, R));
+                if (nonzero(cs)) {
+                    const float3 gs = wmul(gb, cs);
+                    cs0 += gs.x;
+                    cs1 += gs.y;
+                    cs2 += gs.z;
+                }
+                R = ck + wk * R;
+            }
+            grad_add_warp(sg, mat, add);
         }
     }
     if (!A.adjoint) return;   // uniform over the block: the image only, no gradient
     for (int q = 0; q < SKY_PARAMS; ++q) {   // one shared add per warp per sky parameter
         const float3 J = A.sun_J[q];
-        double v = gsky[q] + cs0 * J.x + cs1 * J.y + cs2 * J.z;
+        double v = cs0 * J.x + cs1 * J.y + cs2 * J.z;
         for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
         if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(sg + 4 * A.nmat + q, v);
     }

@@ -1117,6 +1117,32 @@ static void enqueue_path_end(kpt_context* c, const FrameParams& F) {
     c->launches += 1;
 }
 
+// The level (>= 2) from which k_tail takes a wave's paths one by one, above
+// max_depth: none.  It pays while fewer than about 60,000 paths enter it (four
+// per resident warp of the ray kernels: 1920x1080x2 over 64 instances 3.30 ms
+// per level, 3.19 from a level of 75,837 paths, 3.28 from one of 232,618;
+// 640x360x1 over 16 spheres 1.19 and 1.10 ms from one of 50,799).  The host
+// knows the wave's items only; of them at most about 22, 12 and 5% enter
+// levels 2, 3 and 4 and half as many each later one (convex objects under an
+// open sky lose paths sooner and could start earlier, for 1-3% of the frame).
+static int tail_level(const FrameParams& F) {
+    const double items = std::min<double>((double)F.W * F.H * F.nsamples, (double)F.cap);
+    const double most[] = {0.3e6, 0.55e6, 1.25e6};   // items of a wave whose tail starts at 2, 3, 4
+    int l = 2;
+    for (double limit = most[0]; items > limit; ++l) limit = l + 1 <= 4 ? most[l - 1] : 2.0 * limit;
+    return l < F.max_depth ? l : F.max_depth + 1;
+}
+
+// The tail from level l of the paths whose hits are known and the light
+// samples of the level before added, and the sky its paths end in.
+static void enqueue_tail(kpt_context* c, const FrameParams& F, int l) {
+    k_tail<<<persistent_grid(c, (const void*)k_tail, TRACE_BLOCK), TRACE_BLOCK, 0, c->stream>>>(F, l);
+    cudaEventRecord(c->ev_fork[l], c->stream);
+    cudaStreamWaitEvent(c->sky, c->ev_fork[l], 0);
+    k_sky_queue<<<persistent_grid(c, (const void*)k_sky_queue, PATH_BLOCK), PATH_BLOCK, 0, c->sky>>>(F, l, true);
+    c->launches += 2;
+}
+
 static void enqueue_paths(kpt_context* c, const FrameParams& F) {
     cudaStream_t s = c->stream;
     const int np = c->W * c->H;
@@ -1131,13 +1157,19 @@ static void enqueue_paths(kpt_context* c, const FrameParams& F) {
     // streams, joined before k_shade(l + 1); serial when stages are timed
     const bool fork = c->tf == nullptr && c->ev_fork.size() >= (size_t)D + 1;
     const int g_sky = persistent_grid(c, (const void*)k_sky_queue, PATH_BLOCK);
+    const int tail = fork ? tail_level(F) : D + 1;
     for (long long w0 = 0; w0 < items; w0 += F.cap) {
         enqueue_wave_start(c, F, fork);
-        for (int l = 0; l <= D; ++l) {
+        for (int l = 0; l <= std::min(D, tail); ++l) {
             if (l > 0) {
                 stage_mark(c, KPT_STAGE_EXTEND);
                 k_extend<<<g_ext, TRACE_BLOCK, 0, s>>>(F, l);
                 if (fork) cudaStreamWaitEvent(s, c->ev_join[l - 1], 0);
+            }
+            if (l == tail) {   // (after k_shadow(l - 1): both add to the paths' radiance)
+                enqueue_tail(c, F, l);
+                c->launches += 1;
+                break;
             }
             stage_mark(c, KPT_STAGE_SHADE);
             enqueue_shade(c, F, l, w0);
@@ -1149,7 +1181,7 @@ static void enqueue_paths(kpt_context* c, const FrameParams& F) {
                 cudaEventRecord(c->ev_join[l], c->side);
                 // k_shade(l)'s sky entries are final (their paths ended)
                 cudaStreamWaitEvent(c->sky, c->ev_join[l], 0);
-                k_sky_queue<<<g_sky, PATH_BLOCK, 0, c->sky>>>(F, l);
+                k_sky_queue<<<g_sky, PATH_BLOCK, 0, c->sky>>>(F, l, false);
                 c->launches += 1;
             } else {
                 k_shadow<<<g_shd, TRACE_BLOCK, 0, s>>>(F, l);
@@ -1163,7 +1195,7 @@ static void enqueue_paths(kpt_context* c, const FrameParams& F) {
             }
         }
         if (fork) {
-            cudaStreamWaitEvent(s, c->ev_join[D], 0);
+            if (tail > D) cudaStreamWaitEvent(s, c->ev_join[D], 0);
             cudaEventRecord(c->ev_sky, c->sky);
             cudaStreamWaitEvent(s, c->ev_sky, 0);
         }
@@ -1172,7 +1204,7 @@ static void enqueue_paths(kpt_context* c, const FrameParams& F) {
     }
     if (!fork) {
         stage_mark(c, KPT_STAGE_SKY);
-        k_sky_queue<<<g_sky, PATH_BLOCK, 0, s>>>(F, -1);
+        k_sky_queue<<<g_sky, PATH_BLOCK, 0, s>>>(F, -1, false);
         c->launches += 1;
     }
     enqueue_path_end(c, F);
@@ -2301,8 +2333,11 @@ static kpt_status submit_shared(kpt_batch* b, int n, kpt_context* const* jobs, c
         J.ninst = c->view.ninst;
         J.inst_base = b->m_inst_base[j];
         J.cap = F[j].cap;
-        J.max_depth = F[j].max_depth;
-        D = std::max(D, F[j].max_depth);
+        // levels below `shaded` are shaded and their shadow rays traced by the
+        // batch, extension rays up to level `extended`; then the job's tail
+        J.shaded = std::min(tail_level(F[j]), F[j].max_depth + 1);
+        J.extended = std::min(J.shaded, F[j].max_depth);
+        D = std::max(D, J.extended);
     }
     KPT_CUDA(b->d_jobs.upload(b->h_jobs.data(), n, b->stream));
     KPT_CUDA(b->d_queues.ensure(2 * (size_t)(n + 1) + 2));
@@ -2330,15 +2365,37 @@ static kpt_status submit_shared(kpt_batch* b, int n, kpt_context* const* jobs, c
             enqueue_camera(c, F[j]);
             enqueue_wave_start(c, F[j], true);
         }
+        // a job's end: its sky, ray counts, accumulation and post chain
+        auto finish = [&](int j) {
+            kpt_context* c = jobs[j];
+            cudaEventRecord(c->ev_sky, c->sky);
+            cudaStreamWaitEvent(c->stream, c->ev_sky, 0);
+            k_count_rays<<<1, 32, 0, c->stream>>>(F[j]);
+            c->launches += 1;
+            enqueue_path_end(c, F[j]);
+            enqueue_post(c, F[j], c->frame_index + spp[j], c->settings.frame_delta_ms);
+            cudaEventRecordWithFlags(b->ev_end[j], c->stream, cudaEventRecordExternal);
+            cudaEventRecord(b->ev_dep[j], c->stream);
+        };
         for (int l = 0; l <= D; ++l) {
+            bool shading = false, extending = false;
             for (int j = 0; j < n; ++j) {
                 kpt_context* c = jobs[j];
-                if (F[j].max_depth < l) continue;
+                const int shaded = b->h_jobs[j].shaded;
+                if (shaded < l || l > F[j].max_depth) continue;
                 if (l > 0) cudaStreamWaitEvent(c->stream, b->ev_level, 0);
+                if (l == shaded) {   // the rest of the job's levels, path by path
+                    enqueue_tail(c, F[j], l);
+                    finish(j);
+                    continue;
+                }
                 enqueue_shade(c, F[j], l, 0);
                 cudaEventRecord(c->ev_fork[l], c->stream);
                 cudaStreamWaitEvent(b->stream, c->ev_fork[l], 0);
+                shading = true;
+                extending = extending || b->h_jobs[j].extended > l;
             }
+            if (!shading) break;
             k_batch_level<<<1, 32, 0, b->stream>>>(Q, l);
             cudaEventRecord(b->ev_counts, b->stream);
             cudaStreamWaitEvent(b->side, b->ev_counts, 0);
@@ -2346,29 +2403,20 @@ static kpt_status submit_shared(kpt_batch* b, int n, kpt_context* const* jobs, c
             cudaEventRecord(b->ev_shadow, b->side);
             for (int j = 0; j < n; ++j) {
                 kpt_context* c = jobs[j];
-                if (F[j].max_depth < l) continue;
+                if (b->h_jobs[j].shaded <= l) continue;
                 // the level's sky entries are final (their paths ended)
                 cudaStreamWaitEvent(c->sky, b->ev_shadow, 0);
-                k_sky_queue<<<persistent_grid(c, (const void*)k_sky_queue, PATH_BLOCK), PATH_BLOCK, 0, c->sky>>>(F[j], l);
+                k_sky_queue<<<persistent_grid(c, (const void*)k_sky_queue, PATH_BLOCK), PATH_BLOCK, 0, c->sky>>>(
+                    F[j], l, false);
                 c->launches += 2;   // its shading and sky of the level
             }
-            if (l < D) k_extend_batch<<<g_ext, TRACE_BLOCK, 0, b->stream>>>(b->m_view, Q, l + 1, b->d_counters.p);
+            if (extending) k_extend_batch<<<g_ext, TRACE_BLOCK, 0, b->stream>>>(b->m_view, Q, l + 1, b->d_counters.p);
             cudaStreamWaitEvent(b->stream, b->ev_shadow, 0);
             cudaEventRecord(b->ev_level, b->stream);
-            // the jobs whose last level this was: their sky, ray counts,
-            // accumulation and post chain
-            for (int j = 0; j < n; ++j) {
-                kpt_context* c = jobs[j];
+            for (int j = 0; j < n; ++j) {   // the jobs whose last level this was
                 if (F[j].max_depth != l) continue;
-                cudaStreamWaitEvent(c->stream, b->ev_shadow, 0);
-                cudaEventRecord(c->ev_sky, c->sky);
-                cudaStreamWaitEvent(c->stream, c->ev_sky, 0);
-                k_count_rays<<<1, 32, 0, c->stream>>>(F[j]);
-                c->launches += 1;
-                enqueue_path_end(c, F[j]);
-                enqueue_post(c, F[j], c->frame_index + spp[j], c->settings.frame_delta_ms);
-                cudaEventRecordWithFlags(b->ev_end[j], c->stream, cudaEventRecordExternal);
-                cudaEventRecord(b->ev_dep[j], c->stream);
+                cudaStreamWaitEvent(jobs[j]->stream, b->ev_shadow, 0);
+                finish(j);
             }
         }
         for (int j = 0; j < n; ++j) cudaStreamWaitEvent(b->stream, b->ev_dep[j], 0);

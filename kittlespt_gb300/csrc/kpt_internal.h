@@ -19,6 +19,9 @@ constexpr int TILE_W = 8, TILE_H = 4;
 // budget must allow (8: at most 64 registers, 32 warps per SM)
 constexpr int TRACE_MIN_BLOCKS = KPT_TRACE_MIN_BLOCKS;
 
+// k_tail, which also shades: 128 registers (80: an 853x481x3 frame 1.16 ms, not 1.14)
+constexpr int TAIL_MIN_BLOCKS = 4;
+
 // Closest hit of a pixel's camera ray (the same for every sample: the
 // reference discards its filter jitter, kernels.cu:397-402).
 struct __align__(16) PrimaryRec {
@@ -44,7 +47,8 @@ struct __align__(16) ShadowRec {
 
 // per-level counters of a wave, LEVEL_WORDS ints per level: paths entering
 // the level, sun shadow rays, light shadow rays, then the fetch counters of
-// the extension and shadow ray queues
+// the extension and shadow ray queues, the sky queue's mark, the fetch counter
+// of a tail that starts there
 constexpr int LEVEL_WORDS = 8;
 
 // Everything the kernels of one frame read; passed by value.
@@ -183,7 +187,9 @@ struct __align__(16) BatchJob {
     int* level_counts;
     const int* counts;              // counts[2]: the job's sky queue length
     int tlas_root;                  // merged TLAS: root node, or -(instance) - 1
-    int ninst, inst_base, cap, max_depth, pad[3];
+    int ninst, inst_base, cap;
+    int shaded, extended;           // levels shaded in the batch: 0 .. shaded - 1; extension rays up to `extended`
+    int pad[2];
 };
 
 // The ray queues of one level of a batch: the prefix sums of the jobs'
@@ -211,7 +217,8 @@ __global__ void k_count_rays(FrameParams F);   // adds the wave's ray counts to 
 __global__ void k_sort_count(FrameParams F, int level);     // octant histogram of the paths entering level
 __global__ void k_sort_scatter(FrameParams F, int level);   // paths entering level, grouped by octant
 __global__ void k_shadow(FrameParams F, int level);
-__global__ void k_sky_queue(FrameParams F, int level);
+__global__ void k_tail(const __grid_constant__ FrameParams F, int level0);   // the levels from level0 on, path by path
+__global__ void k_sky_queue(FrameParams F, int level, bool rest);
 __global__ void k_sky_constants(FrameParams F, float3* sun_radiance);
 // a batch's queues: after every job's k_shade(level), the extension rays of
 // level + 1 and the shadow rays of level (one block)

@@ -669,6 +669,168 @@ __global__ void __launch_bounds__(TRACE_BLOCK, TRACE_MIN_BLOCKS) k_shadow(FrameP
 }
 
 // ---------------------------------------------------------------------------
+// The tail of a wave: from `level` on, each lane takes one path from its hit to
+// its end -- shades the vertex, traces its shadow ray, adds the light sample,
+// traces the continuation, and so on -- instead of every path waiting at each
+// level for the longest ray of the level.  The later levels of a wave hold few
+// rays and last as long as the longest of them: an 853x481x3 frame of depth 8
+// takes 1.32 ms level by level and 1.18 with a tail from level 4 (1.14 from 2),
+// 256x256x1 of depth 4 0.38 and 0.35, 640x360x2 of depth 5 0.68 and 0.62.
+// What bounds it is the longest chain of rays and vertices.  Each path's events
+// are those of the wave, in its order: the same shading code, the radiance of
+// its item receiving emission, light sample and sky one after the other.
+
+// One vertex's outcomes (shade_vertex), kept for the lane's next rays.
+struct TailSink {
+    const FrameParams& F;
+    PathRec* slot;      // the path's record, rewritten at every vertex
+    float4* contrib;    // its light sample's radiance
+    int* here;          // level_counts of the vertex's level
+    bool shadowed, more;
+    float3 so, sd;      // the shadow ray
+    float stmax;
+    __device__ __forceinline__ void sky(int item, float3 d, float3 beta, float3) {
+        const int q = group_append(F.counts + 2);
+        F.sky_queue[2 * (size_t)q] = make_float4(__int_as_float(item), d.x, d.y, d.z);
+        F.sky_queue[2 * (size_t)q + 1] = make_float4(beta.x, beta.y, beta.z, 0.0f);
+    }
+    __device__ __forceinline__ void radiance(int item, float3 L) {
+        F.radiance[item] = make_float4(L.x, L.y, L.z, 0.0f);
+    }
+    __device__ __forceinline__ void shadow(const Surf& si, float3 target, float3 c, int, bool sun) {
+        shadow_ray(si, target, so, sd, stmax);
+        *contrib = make_float4(c.x, c.y, c.z, 0.0f);
+        shadowed = true;
+        atomicAdd(here + (sun ? 1 : 2), 1);
+    }
+    __device__ __forceinline__ void next(const PathRec& pr) {
+        *slot = pr;
+        more = true;
+        atomicAdd(here + LEVEL_WORDS, 1);
+    }
+};
+
+// Shades the vertex at `level` of the path in slot i, found at hit h, out of
+// line: inlined into the traversal's loop the compiler rounds some light
+// samples differently from the wave's shading.
+struct TailVertex {
+    float3 so, sd;
+    float stmax;
+    int item;
+    bool shadowed, more;
+};
+static __device__ __noinline__ void tail_shade(const FrameParams& F, int level, PathRec* paths, int i,
+                                               const PrimaryRec& h, TailVertex* out) {
+    const PathRec pr = paths[i];
+    const int item = __float_as_int(pr.beta_item.w);
+    const float4 l4 = F.radiance[item];
+    TailSink sink{F, paths + i, &F.shadow[i].contrib, F.level_counts + LEVEL_WORDS * level, false, false};
+    shade_vertex(F, level, h, make_float3(pr.o_pb.x, pr.o_pb.y, pr.o_pb.z),
+                 make_float3(pr.d_seed.x, pr.d_seed.y, pr.d_seed.z),
+                 make_float3(pr.beta_item.x, pr.beta_item.y, pr.beta_item.z),
+                 make_float3(pr.prev.x, pr.prev.y, pr.prev.z), make_float3(l4.x, l4.y, l4.z), pr.o_pb.w,
+                 __float_as_uint(pr.d_seed.w), item, sink);
+    out->so = sink.so;
+    out->sd = sink.sd;
+    out->stmax = sink.stmax;
+    out->item = item;
+    out->shadowed = sink.shadowed;
+    out->more = sink.more;
+}
+
+__global__ void __launch_bounds__(TRACE_BLOCK, TAIL_MIN_BLOCKS) k_tail(const __grid_constant__ FrameParams F, int level0) {
+    constexpr unsigned FULL = 0xffffffffu;
+    using T = Traversal<RAYS_MIXED>;
+    __shared__ TraceShared sh;
+    int stack[STACK_WORDS];
+    TraceStats st = {0, 0, 0, 0}, st_any = {0, 0, 0, 0};
+    int* const lc = F.level_counts + LEVEL_WORDS * level0;
+    const int n = lc[0];
+    PathRec* const paths = F.paths[level0 & 1];
+    const int lane = threadIdx.x & 31;
+    const int lanes = queue_lanes(n);
+    const int batch = min(F.scene.fetch_batch, (lanes + 3) / 4);
+    T r(F.scene, sh, st, st_any, stack, 0.0f, n > 0 && lane < lanes);
+    int i = -1, level = level0;   // the lane's path (its slot), the level it enters next or is at
+    bool more = false;            // it goes on after its shadow ray
+    while (n > 0) {
+        const unsigned idle = __ballot_sync(FULL, r.cur == T::DONE), dead = __ballot_sync(FULL, r.cur == T::DEAD);
+        if (idle && ((idle | dead) == FULL || __popc(idle) >= batch)) {
+            const bool mine = r.cur == T::DONE;
+            // lanes whose path has ended take the next one, at its hit
+            const unsigned want = __ballot_sync(FULL, mine && i < 0);
+            int base = 0;
+            if (lane == 0 && want) base = atomicAdd(lc + 6, __popc(want));
+            base = __shfl_sync(FULL, base, 0);
+            if (mine) {
+                bool shade = false, go = false;
+                PrimaryRec h;
+                float3 wo, wd;
+                if (i < 0) {
+                    i = base + __popc(want & ((1u << lane) - 1u));
+                    if (i < n) {
+                        h = F.hits[i];
+                        level = level0;
+                        shade = true;
+                    } else {
+                        r.cur = T::DEAD;
+                    }
+                } else if (r.any) {   // its shadow ray is done
+                    if (!r.occluded) {
+                        const int item = __float_as_int(F.shadow[i].d_item.w);
+                        const float4 c = F.shadow[i].contrib;
+                        const float4 L = F.radiance[item];
+                        F.radiance[item] = make_float4(L.x + c.x, L.y + c.y, L.z + c.z, 0.0f);
+                    }
+                    go = more;
+                } else {              // its continuation's hit
+                    const Hit q = r.result();
+                    h.t = q.t;
+                    h.u = q.u;
+                    h.v = q.v;
+                    h.inst = q.inst;
+                    h.tri = q.tri;
+                    shade = true;
+                }
+                bool any = false;
+                float tmax = __int_as_float(0x7f800000);
+                if (shade) {
+                    TailVertex v;
+                    tail_shade(F, level, paths, i, h, &v);
+                    ++level;
+                    more = go = v.more;
+                    if (v.shadowed) {
+                        F.shadow[i].d_item.w = __int_as_float(v.item);
+                        any = go = true;
+                        wo = v.so;
+                        wd = v.sd;
+                        tmax = v.stmax;
+                    }
+                }
+                if (go) {
+                    if (!any) {
+                        const float4 a = paths[i].o_pb, b = paths[i].d_seed;
+                        wo = make_float3(a.x, a.y, a.z);
+                        wd = make_float3(b.x, b.y, b.z);
+                    }
+                    r.any = any;
+                    r.tmax = tmax;
+                    r.bound0 = next_up(tmax);
+                    r.start(wo, wd);
+                } else if (r.cur != T::DEAD) {
+                    i = -1;   // the path has ended
+                }
+            }
+            continue;
+        }
+        if (dead == FULL) break;
+        r.step(32 - __popc(idle | dead));
+    }
+    flush_stats(st, F.counters);
+    flush_stats(st_any, F.counters ? F.counters + 8 : nullptr);
+}
+
+// ---------------------------------------------------------------------------
 // Temporal accumulation in the reference GPU build's arithmetic
 // (kpt_settings.temporal_arith = 1): computeVelocity, testReprojection and
 // reprojectAccumulate (kernels.cu:164-223, 299-327) with the matrix
@@ -867,13 +1029,13 @@ __global__ void k_batch_level(BatchQueues Q, int level) {
         int e = 0, sh = 0;
         if (j < Q.njobs) {
             const BatchJob& J = Q.jobs[j];
-            if (level <= J.max_depth) {
+            if (level < J.shaded) {
                 int* lc = J.level_counts + LEVEL_WORDS * level;
                 sh = lc[1] + lc[2];
                 // the job's sky queue cannot grow before its k_shade(level + 1):
                 // its length ends level's range (as k_shadow records it)
                 lc[5] = J.counts[2];
-                if (level + 1 <= J.max_depth) e = J.level_counts[LEVEL_WORDS * (level + 1)];
+                if (level + 1 <= J.extended) e = J.level_counts[LEVEL_WORDS * (level + 1)];
             }
         }
         for (int o = 1; o < 32; o <<= 1) {
@@ -1028,13 +1190,14 @@ __global__ void k_merge_inst(const InstRec* src, int n, InstRec* dst, int mesh_a
 // sky * throughput of every path that left the scene, added to its sample:
 // the whole queue (level < 0), or the entries k_shade(level) appended, from
 // the end of level - 1's range (the wave's starting length for level 0) to
-// the length k_shadow(level) recorded
-__global__ void __launch_bounds__(PATH_BLOCK) k_sky_queue(FrameParams F, int level) {
+// the length k_shadow(level) recorded; `rest`: to the queue's end (after
+// k_tail(level))
+__global__ void __launch_bounds__(PATH_BLOCK) k_sky_queue(FrameParams F, int level, bool rest) {
     int i0 = 0, n = F.counts[2];
     if (level >= 0) {
         const int* mark = F.level_counts + 5;
         i0 = mark[LEVEL_WORDS * (level > 0 ? level - 1 : F.max_depth + 1)];
-        n = mark[LEVEL_WORDS * level];
+        if (!rest) n = mark[LEVEL_WORDS * level];
     }
     const SkyParams& P = F.sky;
     const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);

@@ -404,126 +404,112 @@ __device__ __forceinline__ Hit hit_at(const SceneView& s, int inst, int slot, fl
     return h;
 }
 
-template <bool ANY, class Src, bool ROOTS = false>
-__device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next, Src& src, TraceStats& st,
-                                            int* stack) {
-    constexpr unsigned FULL = 0xffffffffu;
+// Shared memory of a block's rays.
+struct TraceShared {
+    float world[9][TRACE_BLOCK];    // world ray: origin, reciprocal direction, direction
+    float object[6][TRACE_BLOCK];   // ray in its instance: origin, direction
+    int top[STACK_SHARED][TRACE_BLOCK];
+    int owners[TRACE_BLOCK];
+};
+
+// What the rays of a queue are: closest hits, any hits, or each its own kind.
+enum RayKind { RAYS_CLOSEST, RAYS_ANY, RAYS_MIXED };
+
+// One lane's ray and the steps of its warp (every lane of a full warp calls
+// step() together).
+template <RayKind KIND>
+struct Traversal {
+    static constexpr unsigned FULL = 0xffffffffu;
     // what a lane does next (cur, and the entries of its stack): an interior
     // node (>= 0), a leaf (~its first triangle, or ~instance in the TLAS), or
     // leave the instance, store the result, nothing more (the queue is empty)
-    constexpr int LEAVE = (int)0x80000000, DONE = (int)0x80000001, DEAD = (int)0x80000002;
-    const float INF = __int_as_float(0x7f800000);
-    __shared__ float world[9][TRACE_BLOCK];    // world ray: origin, reciprocal direction, direction
-    __shared__ float object[6][TRACE_BLOCK];   // ray in its instance: origin, direction
-    __shared__ int top[STACK_SHARED][TRACE_BLOCK];
-    __shared__ int owners[TRACE_BLOCK];
-    if (n <= 0) return;
-    const int tid = threadIdx.x, lane = tid & 31, warp0 = tid & ~31;
-    const float tmin = src.tmin();
-    // a queue of fewer rays than the grid has lanes is spread over all its
-    // warps: short queues are bound by the latency of their longest rays,
-    // which other rays of the warp prolong (1021 rays 88 -> 29 us, the 65k
-    // paths of a 256x256 frame 0.85 -> 0.42 ms with this and the above)
-    const int warps = gridDim.x * (TRACE_BLOCK / 32);
-    int cur = lane < (n + warps - 1) / warps ? DONE : DEAD;
-    int ray = -1;                       // queue entry
+    static constexpr int LEAVE = (int)0x80000000, DONE = (int)0x80000001, DEAD = (int)0x80000002;
+    const SceneView& s;
+    TraceShared& sh;
+    TraceStats& st;                     // (RAYS_MIXED: of the closest-hit rays)
+    TraceStats& st_any;                 // RAYS_MIXED: of the any-hit rays
+    int* stack;
+    const float tmin;
+    const int tid, lane;
+    int cur;
     int inst = -1;                      // instance being traversed, -1: in the TLAS
     int sp = 0;
-    float tmax = INF;
-    float bound0 = INF, bound = INF;    // boxes entered at or beyond are culled: of the ray, now
-    float best_t = INF;                 // closest hit of the ray: instance, triangle record
+    float tmax;
+    float bound0, bound;                // boxes entered at or beyond are culled: of the ray, now
+    float best_t;                       // closest hit of the ray: instance, triangle record
     int best_inst = -1, best_slot = -1;
     int slot = -1;                      // closest hit in the instance (its distance is `bound`), -1: none
-    bool occluded = false;              // ANY: a triangle blocked the ray
-    const BvhNode* nodes = s.tlas;
-    float3 o = make_float3(0.0f, 0.0f, 0.0f), inv = o, d = o;   // the ray in the space being traversed
-    auto push = [&](int e) {
-        if (sp < STACK_SHARED) top[sp][tid] = e;
+    bool occluded = false;              // any hit: a triangle blocked the ray
+    bool any = KIND == RAYS_ANY;
+    const BvhNode* nodes;
+    float3 o, inv, d;                   // the ray in the space being traversed
+
+    __device__ __forceinline__ Traversal(const SceneView& s_, TraceShared& sh_, TraceStats& st_, TraceStats& st_any_,
+                                         int* stack_, float tmin_, bool alive)
+        : s(s_), sh(sh_), st(st_), st_any(st_any_), stack(stack_), tmin(tmin_), tid(threadIdx.x),
+          lane(threadIdx.x & 31), cur(alive ? DONE : DEAD) {
+        tmax = bound0 = bound = best_t = __int_as_float(0x7f800000);
+        nodes = s.tlas;
+        o = inv = d = make_float3(0.0f, 0.0f, 0.0f);
+    }
+    __device__ __forceinline__ void push(int e) {
+        if (sp < STACK_SHARED) sh.top[sp][tid] = e;
         else stack[sp] = e;
         ++sp;
-    };
-    auto pop = [&]() {
+    }
+    __device__ __forceinline__ int pop() {
         --sp;
         int e;
-        if (sp < STACK_SHARED) e = top[sp][tid];
+        if (sp < STACK_SHARED) e = sh.top[sp][tid];
         else e = stack[sp];
         return e;
-    };
-    auto is_leaf = [&]() { return cur < 0 && cur > DEAD && inst >= 0; };
-    for (;;) {
-        // ---- rays that are done wait until fetch_batch lanes of the warp
-        // are (or nobody else works), then store their results and fetch and
-        // set up their next rays together
-        const unsigned idle = __ballot_sync(FULL, cur == DONE), dead = __ballot_sync(FULL, cur == DEAD);
-        if (idle && ((idle | dead) == FULL || __popc(idle) >= s.fetch_batch)) {
-            bool more = false;
-            float3 wo, wd;
-            if (cur == DONE && ray >= 0) {
-                if (ANY) {
-                    src.any(ray, occluded);
-                } else {
-                    Hit h;
-                    h.t = best_t;
-                    h.inst = h.tri = -1;
-                    h.u = h.v = 0.0f;
-                    if (best_inst >= 0)
-                        h = hit_at(s, best_inst, best_slot, best_t,
-                                   make_float3(world[0][tid], world[1][tid], world[2][tid]),
-                                   make_float3(world[6][tid], world[7][tid], world[8][tid]));
-                    more = src.closest(ray, h, wo, wd);
-                }
-            }
-            const unsigned want = __ballot_sync(FULL, cur == DONE && !more);
-            int base = 0;
-            if (lane == 0 && want) base = atomicAdd(next, __popc(want));
-            base = __shfl_sync(FULL, base, 0);
-            if (cur == DONE) {
-                if (!more) {
-                    ray = base + __popc(want & ((1u << lane) - 1u));
-                    if (ray < n) {
-                        src.ray(ray, wo, wd, tmax);
-                        bound0 = next_up(tmax);
-                        more = true;
-                    } else {
-                        cur = DEAD;
-                    }
-                }
-                if (more) {
-                    // a new ray: the TLAS root box (TLAS::intersect, tlas.cu:60-75), then its root
-                    const XRay w = make_xray(wo, wd);
-                    o = w.o;
-                    inv = w.inv;
-                    d = w.d;
-                    world[0][tid] = o.x; world[1][tid] = o.y; world[2][tid] = o.z;
-                    world[3][tid] = inv.x; world[4][tid] = inv.y; world[5][tid] = inv.z;
-                    world[6][tid] = d.x; world[7][tid] = d.y; world[8][tid] = d.z;
-                    best_t = INF;
-                    best_inst = -1;
-                    bound = bound0;
-                    inst = -1;
-                    occluded = false;
-                    nodes = s.tlas;
-                    sp = 0;
-                    push(DONE);
-                    float4 lo, hi;
-                    int root, ninst;
-                    if constexpr (ROOTS) {
-                        src.root(ray, lo, hi, root, ninst);
-                    } else {
-                        lo = s.tlas_lo;
-                        hi = s.tlas_hi;
-                        root = s.tlas_root_leaf ? ~0 : 0;
-                        ninst = s.ninst;
-                    }
-                    float te;
-                    st.box_tests++;
-                    if (ninst > 0 && slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, w, tmin, tmax, &te)) cur = root;
-                }
-            }
-            continue;
-        }
-        if (dead == FULL) break;
-        const int live = 32 - __popc(idle | dead);
+    }
+    __device__ __forceinline__ bool is_leaf() const { return cur < 0 && cur > DEAD && inst >= 0; }
+    __device__ __forceinline__ bool any_hit() const { return KIND == RAYS_MIXED ? any : KIND == RAYS_ANY; }
+
+    // a new ray: the TLAS root box (TLAS::intersect, tlas.cu:60-75), then its root
+    __device__ __forceinline__ void start(float3 wo, float3 wd, float4 lo, float4 hi, int root, int ninst) {
+        const XRay w = make_xray(wo, wd);
+        o = w.o;
+        inv = w.inv;
+        d = w.d;
+        sh.world[0][tid] = o.x; sh.world[1][tid] = o.y; sh.world[2][tid] = o.z;
+        sh.world[3][tid] = inv.x; sh.world[4][tid] = inv.y; sh.world[5][tid] = inv.z;
+        sh.world[6][tid] = d.x; sh.world[7][tid] = d.y; sh.world[8][tid] = d.z;
+        best_t = __int_as_float(0x7f800000);
+        best_inst = -1;
+        bound = bound0;
+        inst = -1;
+        occluded = false;
+        nodes = s.tlas;
+        sp = 0;
+        push(DONE);
+        cur = DONE;
+        float te;
+        (KIND == RAYS_MIXED && any ? st_any : st).box_tests++;
+        if (ninst > 0 && slab(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, w, tmin, tmax, &te)) cur = root;
+    }
+    __device__ __forceinline__ void start(float3 wo, float3 wd) {
+        start(wo, wd, s.tlas_lo, s.tlas_hi, s.tlas_root_leaf ? ~0 : 0, s.ninst);
+    }
+
+    // the closest hit of the ray that is done
+    __device__ __forceinline__ Hit result() const {
+        Hit h;
+        h.t = best_t;
+        h.inst = h.tri = -1;
+        h.u = h.v = 0.0f;
+        if (best_inst >= 0)
+            h = hit_at(s, best_inst, best_slot, best_t,
+                       make_float3(sh.world[0][tid], sh.world[1][tid], sh.world[2][tid]),
+                       make_float3(sh.world[6][tid], sh.world[7][tid], sh.world[8][tid]));
+        return h;
+    }
+
+    // nodes, leaves, instances; live: lanes of the warp with a ray on its way
+    __device__ __forceinline__ void step(int live) {
+        const float INF = __int_as_float(0x7f800000);
+        const int warp0 = tid & ~31;
         // ---- interior nodes of the TLAS or of an instance's BLAS, until fewer
         // than half of the live lanes step (3/8: 6.38 ms, 5/8: as 1/2, none: 7.4)
         while (cur >= 0) {
@@ -542,7 +528,7 @@ __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next
             const float x2 = fminf(fminf(fmaxf(l2x, h2x), fmaxf(l2y, h2y)), fmaxf(l2z, h2z));
             const bool p1 = t1 <= x1 && x1 >= tmin && t1 < bound;
             const bool p2 = t2 <= x2 && x2 >= tmin && t2 < bound;
-            st.box_tests += 2;
+            (KIND == RAYS_MIXED && any ? st_any : st).box_tests += 2;
             const int r1 = __float_as_int(refs.x), r2 = __float_as_int(refs.z);
             const int c1 = __float_as_int(refs.y) ? ~r1 : r1, c2 = __float_as_int(refs.w) ? ~r2 : r2;
             // the near child is next, the far one on the stack
@@ -561,14 +547,14 @@ __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next
             const unsigned gmask = (1u << width) - 1u;
             const int rank = __popc(leaves & ((1u << lane) - 1u));
             const bool mine = is_leaf() && rank < (32 >> shift);   // this lane's leaf is in the round
-            if (mine) owners[warp0 + rank] = lane;
+            if (mine) sh.owners[warp0 + rank] = lane;
             __syncwarp(FULL);
             const int g = lane >> shift, j = lane & (width - 1);   // group of lanes, its triangle
             const bool act = g < nleaf;
-            const int owner = act ? owners[warp0 + g] : 0;
+            const int owner = act ? sh.owners[warp0 + g] : 0;
             const int k = ~__shfl_sync(FULL, cur, owner) + j;
             // BLAS2::intersect tests against min(tmax, closest so far), intersectP against tmax
-            const float limit = __shfl_sync(FULL, ANY ? tmax : fminf(tmax, bound), owner);
+            const float limit = __shfl_sync(FULL, any_hit() ? tmax : fminf(tmax, bound), owner);
             float t = INF;
             bool last = false, hit = false;
             if (act) {
@@ -578,11 +564,12 @@ __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next
                 const int ow = warp0 + owner;
                 last = b.w != 0.0f;
                 const float3 e1 = make_float3(b.x, b.y, b.z), e2 = make_float3(c.x, c.y, c.z);
-                const float3 rd = make_float3(object[3][ow], object[4][ow], object[5][ow]);
+                const float3 rd = make_float3(sh.object[3][ow], sh.object[4][ow], sh.object[5][ow]);
                 const float3 pv = xcross(rd, e2);
                 const float det = xdot(e1, pv);
                 const float rdet = __frcp_rn(det);
-                const float3 tv = make_float3(xs(object[0][ow], a.x), xs(object[1][ow], a.y), xs(object[2][ow], a.z));
+                const float3 tv = make_float3(xs(sh.object[0][ow], a.x), xs(sh.object[1][ow], a.y),
+                                              xs(sh.object[2][ow], a.z));
                 const float u = xm(rdet, xdot(tv, pv));
                 const float3 qv = xcross(tv, e1);
                 const float v = xm(rdet, xdot(rd, qv));
@@ -591,14 +578,20 @@ __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next
                       !(v < 0.0f || xa(u, v) > 1.0f) && t > TRI_EPS && t < limit && t > tmin;
             }
             const unsigned ends = __ballot_sync(FULL, last);
-            if ((ends >> (lane - j)) & ((1u << j) - 1u)) hit = false;   // the leaf ended before this lane
-            else if (act) st.tri_tests++;
+            const bool tested = act && !((ends >> (lane - j)) & ((1u << j) - 1u));   // the leaf reaches this lane
+            hit = hit && tested;
             const unsigned hits = __ballot_sync(FULL, hit);
             const int from = mine ? rank << shift : 0;                  // first lane of this lane's leaf's group
             const bool my_hit = mine && ((hits >> from) & gmask), my_end = (ends >> from) & gmask;
+            if constexpr (KIND == RAYS_MIXED) {   // counted for the ray's kind, by its owner
+                const unsigned t_mask = __ballot_sync(FULL, tested);
+                if (mine) (any ? st_any : st).tri_tests += __popc((t_mask >> from) & gmask);
+            } else if (tested) {
+                st.tri_tests++;
+            }
             const int first = ~cur;
             if (mine) {
-                if (ANY && my_hit) {
+                if (any_hit() && my_hit) {
                     occluded = true;
                     cur = DONE;
                 } else if (my_end) {
@@ -607,7 +600,7 @@ __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next
                     cur -= width;   // the leaf's next triangles
                 }
             }
-            if (!ANY && hits) {
+            if (KIND != RAYS_ANY && hits) {
                 // the group's closest hit, the first among equals
                 if (!hit) t = INF;
                 int jm = j;
@@ -621,7 +614,7 @@ __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next
                 }
                 const float ht = __shfl_sync(FULL, t, from);
                 const int hj = __shfl_sync(FULL, jm, from);
-                if (my_hit) {
+                if (my_hit && !any_hit()) {
                     bound = ht;
                     slot = first + hj;
                 }
@@ -632,7 +625,7 @@ __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next
         // ---- instances
         if (cur == LEAVE) {
             // merge its closest hit (tlas.cu:116-121), back to the world ray
-            if (!ANY) {
+            if (KIND != RAYS_ANY) {
                 if (slot >= 0 && bound < best_t) {
                     best_t = bound;
                     best_inst = inst;
@@ -642,9 +635,9 @@ __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next
             }
             inst = -1;
             nodes = s.tlas;
-            o = make_float3(world[0][tid], world[1][tid], world[2][tid]);
-            inv = make_float3(world[3][tid], world[4][tid], world[5][tid]);
-            d = make_float3(world[6][tid], world[7][tid], world[8][tid]);
+            o = make_float3(sh.world[0][tid], sh.world[1][tid], sh.world[2][tid]);
+            inv = make_float3(sh.world[3][tid], sh.world[4][tid], sh.world[5][tid]);
+            d = make_float3(sh.world[6][tid], sh.world[7][tid], sh.world[8][tid]);
             cur = pop();
         } else if (cur < 0 && cur > DEAD && inst < 0) {
             // entering one (TLAS leaf): object-space ray (Ray::transform)
@@ -658,15 +651,80 @@ __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next
             o = r.o;
             inv = r.inv;
             d = r.d;
-            object[0][tid] = o.x; object[1][tid] = o.y; object[2][tid] = o.z;
-            object[3][tid] = d.x; object[4][tid] = d.y; object[5][tid] = d.z;
-            st.inst_xforms++;
+            sh.object[0][tid] = o.x; sh.object[1][tid] = o.y; sh.object[2][tid] = o.z;
+            sh.object[3][tid] = d.x; sh.object[4][tid] = d.y; sh.object[5][tid] = d.z;
+            (KIND == RAYS_MIXED && any ? st_any : st).inst_xforms++;
             push(LEAVE);
             nodes = s.nodes;
             bound = bound0;
             slot = -1;
             cur = ir.root;
         }
+    }
+};
+
+// Lanes of a warp that take rays of a queue of n: a queue of fewer rays than
+// the grid has lanes is spread over all its warps -- short queues are bound
+// by the latency of their longest rays, which other rays of the warp prolong
+// (1021 rays 88 -> 27 us, the 65k paths of a 256x256 frame 0.85 -> 0.42 ms
+// with this and the above).
+__device__ __forceinline__ int queue_lanes(int n) {
+    const int warps = gridDim.x * (TRACE_BLOCK / 32);
+    return (n + warps - 1) / warps;
+}
+
+template <bool ANY, class Src, bool ROOTS = false>
+__device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next, Src& src, TraceStats& st,
+                                            int* stack) {
+    constexpr unsigned FULL = 0xffffffffu;
+    using T = Traversal<ANY ? RAYS_ANY : RAYS_CLOSEST>;
+    __shared__ TraceShared sh;
+    if (n <= 0) return;
+    const int lane = threadIdx.x & 31;
+    T r(s, sh, st, st, stack, src.tmin(), lane < queue_lanes(n));
+    int ray = -1;   // queue entry
+    for (;;) {
+        // rays that are done wait until fetch_batch lanes of the warp are (or
+        // nobody else works), then store their results and fetch and set up
+        // their next rays together
+        const unsigned idle = __ballot_sync(FULL, r.cur == T::DONE), dead = __ballot_sync(FULL, r.cur == T::DEAD);
+        if (idle && ((idle | dead) == FULL || __popc(idle) >= s.fetch_batch)) {
+            bool more = false;
+            float3 wo, wd;
+            if (r.cur == T::DONE && ray >= 0) {
+                if (ANY) src.any(ray, r.occluded);
+                else more = src.closest(ray, r.result(), wo, wd);
+            }
+            const unsigned want = __ballot_sync(FULL, r.cur == T::DONE && !more);
+            int base = 0;
+            if (lane == 0 && want) base = atomicAdd(next, __popc(want));
+            base = __shfl_sync(FULL, base, 0);
+            if (r.cur == T::DONE) {
+                if (!more) {
+                    ray = base + __popc(want & ((1u << lane) - 1u));
+                    if (ray < n) {
+                        src.ray(ray, wo, wd, r.tmax);
+                        r.bound0 = next_up(r.tmax);
+                        more = true;
+                    } else {
+                        r.cur = T::DEAD;
+                    }
+                }
+                if (more) {
+                    if constexpr (ROOTS) {
+                        float4 lo, hi;
+                        int root, ninst;
+                        src.root(ray, lo, hi, root, ninst);
+                        r.start(wo, wd, lo, hi, root, ninst);
+                    } else {
+                        r.start(wo, wd);
+                    }
+                }
+            }
+            continue;
+        }
+        if (dead == FULL) break;
+        r.step(32 - __popc(idle | dead));
     }
 }
 

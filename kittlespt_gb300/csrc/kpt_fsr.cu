@@ -9,11 +9,9 @@
 // The unit is compiled without fast maths and without contraction
 // (-fmad=false): every float operation rounds once, in the reference's order,
 // and the reference's double-precision literals (0.5, .4, 1.5625, .29, 1. /
-// lob, 4. * lobe + 1., the RCAS limit) keep their double results, so the
-// images are bit for bit those of the reference compiled for the host.  FP64
-// is slow on this GPU, so where a float form provably rounds to the same
-// float it replaces the double one (each case says why); the rest stays in
-// double.
+// lob, 4. * lobe + 1., the RCAS limit) keep their results rounded to float,
+// formed in float -- FP64 is slow on this GPU -- by forms that round to the
+// same float (each says why).
 // Reads go through textureReadBilinear's rule (device_texture_buffer.cuh:
 // 42-80): the pixel position truncated toward zero, texels clamped to the
 // image, lerps with the remainder (negative at the top and left edges).
@@ -43,22 +41,64 @@ __device__ __forceinline__ float3 bilinear3(const float4* img, int w, int h, flo
 }
 
 // luma times two of the reference, y + 0.5 * (x + z), evaluated there in
-// double and rounded to float.  When halving s = x + z is exact in float, the
-// float sum y + s/2 is the same float: the exact sum rounded once, and where
-// double cannot hold the exact sum (exponents more than 29 apart) the
-// smaller term is below half a float ulp of the larger either way.  A
-// subnormal s takes the double form.
-__device__ __forceinline__ float luma2(float3 c) {
-    const float s = c.x + c.z, h = 0.5f * s;
-    if (h + h == s) return c.y + h;
-    return (float)((double)c.y + 0.5 * (double)s);
-}
+// double and rounded to float: half of 2 y + s, whose float sum is twice the
+// rounded y + s / 2 (for sums
+// below 2^128; a subnormal result's sum is exact and the halving rounds once).
+__device__ __forceinline__ float luma2(float3 c) { return 0.5f * (2.0f * c.y + (c.x + c.z)); }
 
 // clamp(q, 0, 1) of helper_math, fmaxf(0, fminf(q, 1)), which gives 1 for a
 // NaN q (0 / 0 on a flat row or column of lumas); spelled out so that the
 // NaN case cannot become a saturation (which gives 0)
 __device__ __forceinline__ float clamp01(float q) {
     return isnan(q) ? 1.0f : fmaxf(0.0f, fminf(q, 1.0f));
+}
+
+// The reference's double-precision weights, stretch and lobe, rounded to
+// float: float sums and products with their exact rounding errors, h + l
+// within e of the exact value.  Where h + l - e and h + l + e round to
+// different floats (one input in 2^16 or fewer and NaN, but one length in 60 for
+// the lobe: .29 = 29 / 100 brings each 50th near a tie) the double form
+// decides, so the result is its float always (tests/fsr_exact_sums.c).  All in double,
+// EASU to 1920x1080 held the FP64 pipe, 1/64 of the float rate, at 84% and
+// took 318 us; in float 127 us.
+__device__ __forceinline__ float rounded(float h, float l, float e, bool& sure) {
+    const float lo = h + (l - e), hi = h + (l + e);
+    sure = sure && lo == hi;
+    return lo;
+}
+__device__ __forceinline__ float2 two_sum(float a, float b) {
+    const float s = a + b, t = s - a;
+    return make_float2(s, (a - (s - t)) + (b - t));
+}
+struct EasuWeights { float w00, w10, w01; };   // (1 - x) (1 - y), x (1 - y), (1 - x) y
+__device__ __forceinline__ EasuWeights easu_weights(float x, float y) {
+    const float2 u = two_sum(1.0f, -x), v = two_sum(1.0f, -y);
+    const float p = u.x * v.x, q = x * v.x, r = u.x * y;
+    bool sure = true;
+    EasuWeights W;
+    W.w00 = rounded(p, fmaf(u.x, v.y, fmaf(u.y, v.x, fmaf(u.x, v.x, -p))), p * 0x1p-44f, sure);
+    W.w10 = rounded(q, fmaf(x, v.y, fmaf(x, v.x, -q)), q * 0x1p-44f, sure);
+    W.w01 = rounded(r, fmaf(u.y, y, fmaf(u.x, y, -r)), r * 0x1p-44f, sure);
+    if (!sure) {
+        W.w00 = (float)((1.0 - (double)x) * (1.0 - (double)y));
+        W.w10 = (float)((double)x * (1.0 - (double)y));
+        W.w01 = (float)((1.0 - (double)x) * (double)y);
+    }
+    return W;
+}
+constexpr float C29 = 0.29f, CL29 = 0x1.1eb852p-27f;   // 0.29 (double) in two floats
+// 1 + (s - 1) len and the lobe 0.5 - 0.29 len
+__device__ __forceinline__ void easu_shape(float s, float len, float& stretched, float& lobe) {
+    const float2 a = two_sum(s, -1.0f);
+    const float p = a.x * len, q = C29 * len;
+    const float2 r = two_sum(1.0f, p), t = two_sum(0.5f, -q);
+    bool sure = true;
+    stretched = rounded(r.x, r.y + fmaf(a.y, len, fmaf(a.x, len, -p)), 0x1p-44f, sure);
+    lobe = rounded(t.x, t.y - fmaf(CL29, len, fmaf(C29, len, -q)), 0x1p-46f, sure);
+    if (!sure) {
+        stretched = (float)(1.0 + ((double)s - 1.0) * (double)len);
+        lobe = (float)(0.5 - 0.29 * (double)len);
+    }
 }
 
 // FsrEasuSetF (upscale.cuh:101-130): gradient direction and edge length of
@@ -187,9 +227,10 @@ __global__ void k_easu(const float4* src, int sw, int sh, float4* dst, int dw, i
 
     float2 dir = make_float2(0.0f, 0.0f);
     float len = 0.0f;
-    easu_set(dir, len, (float)((1.0 - (double)ppx) * (1.0 - (double)ppy)), bL, eL, fL, gL, jL);
-    easu_set(dir, len, (float)((double)ppx * (1.0 - (double)ppy)), cL, fL, gL, hL, kL);
-    easu_set(dir, len, (float)((1.0 - (double)ppx) * (double)ppy), fL, iL, jL, kL, nL);
+    const EasuWeights W = easu_weights(ppx, ppy);
+    easu_set(dir, len, W.w00, bL, eL, fL, gL, jL);
+    easu_set(dir, len, W.w10, cL, fL, gL, hL, kL);
+    easu_set(dir, len, W.w01, fL, iL, jL, kL, nL);
     easu_set(dir, len, ppx * ppy, gL, jL, kL, lL, oL);
 
     // normalise the direction (1 / sqrt, both correctly rounded), shape the
@@ -202,16 +243,15 @@ __global__ void k_easu(const float4* src, int sw, int sh, float4* dst, int dw, i
     dir.x = zro ? 1.0f : dir.x;
     dir.x *= dirR;
     dir.y *= dirR;
-    len = (float)((double)len * 0.5);
+    len = len * 0.5f;
     len *= len;
     const float stretch = (dir.x * dir.x + dir.y * dir.y) / fmaxf(fabsf(dir.x), fabsf(dir.y));
     EasuKernel K;
     K.dir = dir;
     // 1. - .5 * len and 1. / lob in double give the float forms' results for
-    // every float len in [0, 1] and lob in [0.2, 0.51] (checked
-    // exhaustively); .29 * len and the stretch term stay in double
-    K.len2 = make_float2((float)(1.0 + ((double)stretch - 1.0) * (double)len), 1.0f - 0.5f * len);
-    K.lob = (float)(0.5 - 0.29 * (double)len);
+    // every float len in [0, 1] and lob in [0.2, 0.51] (checked exhaustively)
+    K.len2.y = 1.0f - 0.5f * len;
+    easu_shape(stretch, len, K.len2.x, K.lob);
     K.clp = 1.0f / K.lob;
     K.ppx = ppx;
     K.ppy = ppy;

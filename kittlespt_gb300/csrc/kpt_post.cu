@@ -321,10 +321,42 @@ __device__ __forceinline__ float srgb_enc(float v) {  // color.cuh:421-426
     return (v <= 0.0031308f) ? __fmul_rn(12.92f, v) : __fsub_rn(__fmul_rn(__fadd_rn(1.0f, 0.055f), powf(v, __fdiv_rn(1.0f, 2.4f))), 0.055f);
 }
 
+// Y (1 - cx - cy) / cy, the reference's double-precision expression rounded to
+// float.  In double it kept the FP64 pipe, 1/64 of the float rate, at 71%
+// (73 us at 1920x1080, in float 64).  Here as float sums and products with
+// their exact rounding errors and a quotient corrected once, within 2^-44 of
+// the exact value; where that does not decide the rounding (about one input in
+// 2^20), or a product's error could leave the float range (a luminance outside
+// [2^-40, 2^60], a chromaticity outside the gamut or not a number: black
+// pixels), the double form does, so the result is its float always
+// (tests/fsr_exact_sums.c).
+__device__ __forceinline__ float2 two_sum(float a, float b) {
+    const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+    return make_float2(s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t)));
+}
+__device__ __forceinline__ float luminance_z(float Y, float cx, float cy) {
+    if (Y >= 0x1p-40f && Y <= 0x1p60f && cy >= 0x1p-10f && cy <= 1.0f && cx >= 0.0f && cx <= 1.0f) {
+        const float2 a = two_sum(1.0f, -cx), b = two_sum(a.x, -cy);
+        const float2 m = two_sum(b.x, __fadd_rn(a.y, b.y));
+        const float p = __fmul_rn(Y, m.x), pl = __fmaf_rn(Y, m.y, __fmaf_rn(Y, m.x, -p));
+        const float rc = __frcp_rn(cy), q = __fmul_rn(p, rc);
+        const float l = __fmul_rn(__fadd_rn(__fmaf_rn(-q, cy, p), pl), rc), e = __fmul_rn(fabsf(q), 0x1p-44f);
+        const float lo = __fadd_rn(q, __fsub_rn(l, e)), hi = __fadd_rn(q, __fadd_rn(l, e));
+        if (lo == hi) return lo;
+    }
+    return (float)((double)Y * (1.0 - (double)cx - (double)cy) / (double)cy);
+}
+
 // computePostProcess (kernels.cu:475-504) with Film / AgX (film.cuh:79-194).
+// The exposure range's logarithms, the same for every pixel, are taken once
+// per block.
 __global__ void k_tonemap(int W, int H, const float4* render, const float4* bloom, int use_bloom, float final_blend,
                           const ExposureState* st, float fixed_scalar, int auto_exposure, float white_ev, float black_ev,
                           float4* image) {
+    __shared__ float range[2];
+    if (threadIdx.y == 0 && threadIdx.x < 2)
+        range[threadIdx.x] = log2f(__fmul_rn(exp2f(threadIdx.x ? white_ev : black_ev), 0.18f));
+    __syncthreads();
     int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= W || y >= H) return;
     int sx = (int)__fmul_rn(__fdiv_rn(__fadd_rn((float)x, 0.5f), (float)W), (float)W);
@@ -340,12 +372,12 @@ __global__ void k_tonemap(int W, int H, const float4* render, const float4* bloo
     float Y = __fmul_rn(Yv, expo), cx = __fmul_rn(X, inv), cy = __fmul_rn(Yv, inv);
     float X2 = __fdiv_rn(__fmul_rn(Y, cx), cy);
     float Y2 = Y;
-    float Z2 = (float)((double)Y * (1.0 - (double)cx - (double)cy) / (double)cy);
+    float Z2 = luminance_z(Y, cx, cy);
     float r = dot3(3.2404542f, -1.5371385f, -0.4985314f, X2, Y2, Z2);
     float g = dot3(-0.9692660f, 1.8760108f, 0.0415560f, X2, Y2, Z2);
     float b = dot3(0.0556434f, -0.2040259f, 1.0572252f, X2, Y2, Z2);
     // AgX (film.cuh:79-172)
-    const float mn = log2f(__fmul_rn(exp2f(black_ev), 0.18f)), mx = log2f(__fmul_rn(exp2f(white_ev), 0.18f));
+    const float mn = range[0], mx = range[1];
     const float dr = __fsub_rn(mx, mn);
     float r2 = fmaxf(dot3(0.6274f, 0.3293f, 0.0433f, r, g, b), 0.0f);
     float g2 = fmaxf(dot3(0.0691f, 0.9195f, 0.0113f, r, g, b), 0.0f);

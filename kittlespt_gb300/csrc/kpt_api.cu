@@ -85,6 +85,7 @@ struct kpt_context {
     // on it once k_shadow(l) has ended, beside the later levels
     cudaStream_t sky = nullptr;
     cudaEvent_t ev_sky = nullptr;
+    cudaEvent_t ev_branch[6] = {};   // a frame's other forks and joins (BRANCH_*)
     std::vector<cudaEvent_t> ev_fork, ev_join;
     uint64_t launches = 0;
 
@@ -294,6 +295,8 @@ kpt_status kpt_create(int device, kpt_context** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->sky, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_sky, cudaEventDisableTiming);
+    for (cudaEvent_t& ev : c->ev_branch)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         delete c;
         return fail(KPT_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
@@ -349,6 +352,8 @@ kpt_status kpt_destroy(kpt_context* c) {
     for (auto* v : {&c->ev_fork, &c->ev_join})
         for (cudaEvent_t e : *v) cudaEventDestroy(e);
     if (c->ev_sky) cudaEventDestroy(c->ev_sky);
+    for (cudaEvent_t ev : c->ev_branch)
+        if (ev) cudaEventDestroy(ev);
     if (c->sky) cudaStreamDestroy(c->sky);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -1066,30 +1071,48 @@ static void enqueue_primary(kpt_context* c, const FrameParams& F) {
     c->launches += 2;
 }
 
-// The path stage: camera rays and their sky, then the wave(s) of paths level
-// by level, the queued sky and the ordered accumulation of every sample.
-// camera rays and their sky
-static void enqueue_camera(kpt_context* c, const FrameParams& F) {
-    cudaStream_t s = c->stream;
-    c->levels_depth = F.max_depth;
-    cudaMemsetAsync(c->counts.p, 0, 4 * sizeof(int), s);
-    stage_mark(c, KPT_STAGE_CAMERA);
-    k_sky_constants<<<1, 32, 0, s>>>(F, c->sun_radiance.p);
-    enqueue_primary(c, F);
-    k_primary_sky<<<persistent_grid(c, (const void*)k_primary_sky, PATH_BLOCK), PATH_BLOCK, 0, s>>>(F);
-    c->launches += 2;
+// `to` continues after what `from` holds now
+enum { BRANCH_START, BRANCH_SUN, BRANCH_HITS, BRANCH_COUNT, BRANCH_RENDER, BRANCH_EXPOSURE };
+static void branch(kpt_context* c, int which, cudaStream_t from, cudaStream_t to) {
+    cudaEventRecord(c->ev_branch[which], from);
+    cudaStreamWaitEvent(to, c->ev_branch[which], 0);
 }
 
-// the start of a wave: its level counters cleared; with `mark`, the sky
-// queue's length recorded as where its level 0 begins
-static void enqueue_wave_start(kpt_context* c, const FrameParams& F, bool mark) {
-    cudaStream_t s = c->stream;
+// the start of a wave on stream s: its level counters cleared (among them
+// where in the sky queue its level 0 begins, 0 in a frame's first wave); with
+// `mark`, that is set to the sky queue's length
+static void enqueue_wave_start(kpt_context* c, const FrameParams& F, bool mark, cudaStream_t s) {
     const int D = F.max_depth;
     cudaMemsetAsync(c->level_counts.p, 0, sizeof(int) * LEVEL_WORDS * (size_t)(D + 2), s);
     if (mark)
         cudaMemcpyAsync(c->level_counts.p + LEVEL_WORDS * (D + 1) + 5, c->counts.p + 2, sizeof(int),
                         cudaMemcpyDeviceToDevice, s);
     if (F.unsorted) cudaMemsetAsync(c->octants.p, 0, sizeof(int) * 16 * (size_t)(D + 2), s);
+}
+
+// The path stage: camera rays and their sky, then the wave(s) of paths level
+// by level, the queued sky and the ordered accumulation of every sample.
+// Here the camera rays, their sky and the start of the first wave.  With
+// `fork`, the sun's radiance and the first wave's counters (due at the first
+// shading) are made beside the camera rays, and the camera rays' sky (due at
+// the accumulation) beside the paths: in line they, the ray counts and the
+// image's own pass took 30 us of a 256x256 frame (352 us, now 325).
+static void enqueue_camera(kpt_context* c, const FrameParams& F, bool fork) {
+    cudaStream_t s = c->stream, sky = fork ? c->sky : s;
+    c->levels_depth = F.max_depth;
+    stage_mark(c, KPT_STAGE_CAMERA);
+    if (fork) branch(c, BRANCH_START, s, sky);
+    k_sky_constants<<<1, 32, 0, sky>>>(F, c->sun_radiance.p);
+    enqueue_wave_start(c, F, false, sky);
+    if (fork) cudaEventRecord(c->ev_branch[BRANCH_SUN], sky);
+    cudaMemsetAsync(c->counts.p, 0, 4 * sizeof(int), s);
+    enqueue_primary(c, F);
+    if (fork) {
+        branch(c, BRANCH_HITS, s, sky);
+        cudaStreamWaitEvent(s, c->ev_branch[BRANCH_SUN], 0);
+    }
+    k_primary_sky<<<persistent_grid(c, (const void*)k_primary_sky, PATH_BLOCK), PATH_BLOCK, 0, sky>>>(F);
+    c->launches += 2;
 }
 
 // the shading of level l of the wave starting at item w0
@@ -1109,11 +1132,23 @@ static void enqueue_shade(kpt_context* c, const FrameParams& F, int l, long long
     }
 }
 
-// the ordered accumulation of every sample
-static void enqueue_path_end(kpt_context* c, const FrameParams& F) {
+// a wave's ray counts, on the stream of its shadow rays; with what the sky
+// stream still holds, joined into the context's stream
+static void enqueue_wave_end(kpt_context* c, const FrameParams& F) {
+    k_count_rays<<<1, 32, 0, c->side>>>(F);
+    branch(c, BRANCH_COUNT, c->side, c->stream);
+    cudaEventRecord(c->ev_sky, c->sky);
+    cudaStreamWaitEvent(c->stream, c->ev_sky, 0);
+    c->launches += 1;
+}
+
+// The ordered accumulation of every sample and, for a frame (total_samples of
+// them so far) whose image is not first blended over time, that image.
+static void enqueue_path_end(kpt_context* c, const FrameParams& F, int total_samples) {
     const int np = c->W * c->H;
     stage_mark(c, KPT_STAGE_ACCUMULATE);
-    k_accumulate<<<(np + 255) / 256, 256, 0, c->stream>>>(F);
+    float4* render = total_samples > 0 && !c->settings.temporal_accumulation ? c->render.p : nullptr;
+    k_accumulate<<<(np + 255) / 256, 256, 0, c->stream>>>(F, (float)total_samples, render);
     c->launches += 1;
 }
 
@@ -1138,16 +1173,16 @@ static int tail_level(const FrameParams& F) {
 static void enqueue_tail(kpt_context* c, const FrameParams& F, int l) {
     k_tail<<<persistent_grid(c, (const void*)k_tail, TRACE_BLOCK), TRACE_BLOCK, 0, c->stream>>>(F, l);
     cudaEventRecord(c->ev_fork[l], c->stream);
+    cudaStreamWaitEvent(c->side, c->ev_fork[l], 0);
     cudaStreamWaitEvent(c->sky, c->ev_fork[l], 0);
     k_sky_queue<<<persistent_grid(c, (const void*)k_sky_queue, PATH_BLOCK), PATH_BLOCK, 0, c->sky>>>(F, l, true);
     c->launches += 2;
 }
 
-static void enqueue_paths(kpt_context* c, const FrameParams& F) {
+static void enqueue_paths(kpt_context* c, const FrameParams& F, int total_samples) {
     cudaStream_t s = c->stream;
     const int np = c->W * c->H;
     const int D = F.max_depth;
-    enqueue_camera(c, F);
     const int g_ext = persistent_grid(c, (const void*)k_extend, TRACE_BLOCK);
     const int g_shd = persistent_grid(c, (const void*)k_shadow, TRACE_BLOCK);
     // every pixel may hit: the last waves find no work when fewer do
@@ -1158,8 +1193,9 @@ static void enqueue_paths(kpt_context* c, const FrameParams& F) {
     const bool fork = c->tf == nullptr && c->ev_fork.size() >= (size_t)D + 1;
     const int g_sky = persistent_grid(c, (const void*)k_sky_queue, PATH_BLOCK);
     const int tail = fork ? tail_level(F) : D + 1;
+    enqueue_camera(c, F, fork);
     for (long long w0 = 0; w0 < items; w0 += F.cap) {
-        enqueue_wave_start(c, F, fork);
+        if (w0 > 0) enqueue_wave_start(c, F, fork, s);
         for (int l = 0; l <= std::min(D, tail); ++l) {
             if (l > 0) {
                 stage_mark(c, KPT_STAGE_EXTEND);
@@ -1195,19 +1231,18 @@ static void enqueue_paths(kpt_context* c, const FrameParams& F) {
             }
         }
         if (fork) {
-            if (tail > D) cudaStreamWaitEvent(s, c->ev_join[D], 0);
-            cudaEventRecord(c->ev_sky, c->sky);
-            cudaStreamWaitEvent(s, c->ev_sky, 0);
+            enqueue_wave_end(c, F);
+        } else {
+            k_count_rays<<<1, 32, 0, s>>>(F);
+            c->launches += 1;
         }
-        k_count_rays<<<1, 32, 0, s>>>(F);
-        c->launches += 1;
     }
     if (!fork) {
         stage_mark(c, KPT_STAGE_SKY);
         k_sky_queue<<<g_sky, PATH_BLOCK, 0, s>>>(F, -1, false);
         c->launches += 1;
     }
-    enqueue_path_end(c, F);
+    enqueue_path_end(c, F, total_samples);
 }
 
 static kpt_status ready(kpt_context* c) {
@@ -1242,9 +1277,11 @@ static void update_thresholds(kpt_context* c) {
 // The frame: enqueued on the context stream (captured into a graph).
 static void enqueue_temporal(kpt_context* c, const FrameParams& F);
 
-// what follows the path stage: temporal blend or resolve, exposure, upscale,
-// bloom, tonemap, lens effects
-static void enqueue_post(kpt_context* c, const FrameParams& F, int total_samples, float delta_ms) {
+// What follows the path stage: temporal blend, exposure, upscale, bloom,
+// tonemap, lens effects.  The exposure (due at the tonemap) is measured beside
+// the upscale and the bloom chain, where it is in line when stages are timed
+// (853x481: 28 us of 1.18 ms).
+static void enqueue_post(kpt_context* c, const FrameParams& F, float delta_ms) {
     cudaStream_t s = c->stream;
     const int np = c->W * c->H;
     stage_mark(c, KPT_STAGE_POST);
@@ -1252,11 +1289,12 @@ static void enqueue_post(kpt_context* c, const FrameParams& F, int total_samples
         enqueue_temporal(c, F);
         // modulateSamples of the blended image (kernels.cu:453-472)
         k_resolve<<<(np + 255) / 256, 256, 0, s>>>(np, c->thist[0].p, c->albedo.p, 1.0f, c->render.p);
-    } else {
-        k_resolve<<<(np + 255) / 256, 256, 0, s>>>(np, c->acc.p, c->albedo.p, (float)total_samples, c->render.p);
+        c->launches += 1;
     }
-    c->launches += 1;
+    const bool beside = c->tf == nullptr;
     if (c->settings.auto_exposure) {
+        cudaStream_t x = beside ? c->side : s;
+        if (beside) branch(c, BRANCH_RENDER, s, x);
         ExposureIn in{};
         in.aperture = c->exposure.aperture;
         in.ev_comp = c->exposure.ev_comp;
@@ -1267,9 +1305,10 @@ static void enqueue_post(kpt_context* c, const FrameParams& F, int total_samples
         in.min_shutter = c->exposure.min_shutter;
         in.max_shutter = c->exposure.max_shutter;
         in.delta_ms = delta_ms;
-        cudaMemsetAsync(c->hist.p, 0, 256 * sizeof(unsigned long long), s);
-        k_histogram<<<(np + 255) / 256, 256, 0, s>>>(c->W, c->H, c->render.p, c->thresholds.p, c->hist.p);
-        k_exposure<<<1, 32, 0, s>>>(c->hist.p, c->expo_state.p, in);
+        cudaMemsetAsync(c->hist.p, 0, 256 * sizeof(unsigned long long), x);
+        k_histogram<<<(np + 255) / 256, 256, 0, x>>>(c->W, c->H, c->render.p, c->thresholds.p, c->hist.p);
+        k_exposure<<<1, 256, 0, x>>>(c->hist.p, c->expo_state.p, in);
+        if (beside) cudaEventRecord(c->ev_branch[BRANCH_EXPOSURE], x);
         c->launches += 2;
     }
     // launchUpscaleComputeKernel (kernels.cu:84-104): bilinear, or with FSR
@@ -1310,6 +1349,7 @@ static void enqueue_post(kpt_context* c, const FrameParams& F, int total_samples
     double lavg = (10.0 / 0.65) * ((N * N) / ((double)c->exposure.iso * (double)c->exposure.shutter));
     float fixed_scalar = (float)(0.18 / lavg);
     const bool fx = c->settings.postprocess_effects != 0;
+    if (beside && c->settings.auto_exposure) cudaStreamWaitEvent(s, c->ev_branch[BRANCH_EXPOSURE], 0);
     k_tonemap<<<dim3((c->OW + 15) / 16, (c->OH + 15) / 16), dim3(16, 16), 0, s>>>(
         c->OW, c->OH, out, bloom0, bloom0 != nullptr, c->settings.bloom_final_blend, c->expo_state.p, fixed_scalar,
         c->settings.auto_exposure, c->exposure.white_ev, c->exposure.black_ev, fx ? c->backbuf.p : c->image.p);
@@ -1323,8 +1363,8 @@ static void enqueue_post(kpt_context* c, const FrameParams& F, int total_samples
 }
 
 static void enqueue_frame(kpt_context* c, const FrameParams& F, int total_samples, float delta_ms) {
-    enqueue_paths(c, F);
-    enqueue_post(c, F, total_samples, delta_ms);
+    enqueue_paths(c, F, total_samples);
+    enqueue_post(c, F, delta_ms);
 }
 
 // Host-side work of a frame, outside any capture: TLAS rebuild, exposure
@@ -1606,7 +1646,7 @@ kpt_status kpt_render_samples_device(kpt_context* c, int sample0, int nsamples, 
     F.sample_out = reinterpret_cast<float4*>(radiance);
     F.first_hit = reinterpret_cast<int4*>(first_hit);
     F.albedo = reinterpret_cast<float4*>(albedo);
-    enqueue_paths(c, F);
+    enqueue_paths(c, F, 0);
     KPT_CUDA(cudaGetLastError());
     return KPT_OK;
 }
@@ -2362,18 +2402,14 @@ static kpt_status submit_shared(kpt_batch* b, int n, kpt_context* const* jobs, c
         for (int j = 0; j < n; ++j) {
             kpt_context* c = jobs[j];
             cudaStreamWaitEvent(c->stream, b->ev_fork, 0);
-            enqueue_camera(c, F[j]);
-            enqueue_wave_start(c, F[j], true);
+            enqueue_camera(c, F[j], true);
         }
         // a job's end: its sky, ray counts, accumulation and post chain
         auto finish = [&](int j) {
             kpt_context* c = jobs[j];
-            cudaEventRecord(c->ev_sky, c->sky);
-            cudaStreamWaitEvent(c->stream, c->ev_sky, 0);
-            k_count_rays<<<1, 32, 0, c->stream>>>(F[j]);
-            c->launches += 1;
-            enqueue_path_end(c, F[j]);
-            enqueue_post(c, F[j], c->frame_index + spp[j], c->settings.frame_delta_ms);
+            enqueue_wave_end(c, F[j]);
+            enqueue_path_end(c, F[j], c->frame_index + spp[j]);
+            enqueue_post(c, F[j], c->settings.frame_delta_ms);
             cudaEventRecordWithFlags(b->ev_end[j], c->stream, cudaEventRecordExternal);
             cudaEventRecord(b->ev_dep[j], c->stream);
         };
@@ -2415,7 +2451,7 @@ static kpt_status submit_shared(kpt_batch* b, int n, kpt_context* const* jobs, c
             cudaEventRecord(b->ev_level, b->stream);
             for (int j = 0; j < n; ++j) {   // the jobs whose last level this was
                 if (F[j].max_depth != l) continue;
-                cudaStreamWaitEvent(jobs[j]->stream, b->ev_shadow, 0);
+                cudaStreamWaitEvent(jobs[j]->side, b->ev_shadow, 0);
                 finish(j);
             }
         }

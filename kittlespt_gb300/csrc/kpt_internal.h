@@ -287,7 +287,8 @@ struct TemporalParams {
 };
 __global__ void k_temporal(TemporalParams T);       // kpt_post.cu, IEEE
 __global__ void k_temporal_gpu(TemporalParams T);   // kpt_path.cu, the reference GPU build's arithmetic
-__global__ void k_accumulate(FrameParams F);
+// with `render`, also the image sum / total_samples * albedo
+__global__ void k_accumulate(FrameParams F, float total_samples, float4* render);
 __global__ void k_sky(SkyParams P, int n, const float3* dirs, float3* out);
 __global__ void k_trace(SceneView s, int n, const float3* o, const float3* d, float tmin, float tmax,
                         int* inst, int* tri, float* t, float2* uv, int* next, unsigned long long* counters);

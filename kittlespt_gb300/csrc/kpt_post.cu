@@ -26,11 +26,29 @@
 
 namespace kpt {
 
+__device__ __forceinline__ float qbyte(float v) {  // floatToByte then byteToFloat (packing.cuh:10-18)
+    v = fmaxf(0.0f, fminf(v, 1.0f));
+    uint32_t b = (uint32_t)__fmul_rn(v, 255.0f) & 0xFFu;
+    return __fdiv_rn((float)b, 255.0f);
+}
+
+__device__ __forceinline__ float4 resolve(float4 a, float4 al, float nsamples) {
+    return make_float4(__fmul_rn(__fdiv_rn(a.x, nsamples), qbyte(al.x)),
+                       __fmul_rn(__fdiv_rn(a.y, nsamples), qbyte(al.y)),
+                       __fmul_rn(__fdiv_rn(a.z, nsamples), qbyte(al.z)), 1.0f);
+}
+
+__global__ void k_resolve(int npix, const float4* acc, const float4* albedo, float nsamples, float4* render) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < npix) render[i] = resolve(acc[i], albedo[i], nsamples);
+}
+
 // RGBSpectrum::clampOutput (color.cuh:295-302) of every sample, added to the
 // pixel's accumulation in sample order (integrator.cuh:406-415), as the
 // reference accumulates one frame per sample.  Samples of a pixel whose camera
-// ray misses all equal the pixel's sky radiance.
-__global__ void k_accumulate(FrameParams F) {
+// ray misses all equal the pixel's sky radiance.  With `render`, the image too
+// (a launch of its own and a pass over the sum otherwise).
+__global__ void k_accumulate(FrameParams F, float total_samples, float4* render) {
     const int npix = F.W * F.H;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npix) return;
@@ -49,6 +67,7 @@ __global__ void k_accumulate(FrameParams F) {
         if (F.sample_out) F.sample_out[(size_t)k * npix + p] = L;
     }
     if (F.acc) F.acc[p] = make_float4(acc.x, acc.y, acc.z, 1.0f);
+    if (render) render[p] = resolve(acc, F.albedo[p], total_samples);
 }
 
 // --- temporal accumulation (kernels.cu:164-327) ------------------------------
@@ -138,21 +157,6 @@ __global__ void k_temporal(TemporalParams T) {
     T.hist_out[p] = out;
 }
 
-__device__ __forceinline__ float qbyte(float v) {  // floatToByte then byteToFloat (packing.cuh:10-18)
-    v = fmaxf(0.0f, fminf(v, 1.0f));
-    uint32_t b = (uint32_t)__fmul_rn(v, 255.0f) & 0xFFu;
-    return __fdiv_rn((float)b, 255.0f);
-}
-
-__global__ void k_resolve(int npix, const float4* acc, const float4* albedo, float nsamples, float4* render) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npix) return;
-    float4 a = acc[i], al = albedo[i];
-    render[i] = make_float4(__fmul_rn(__fdiv_rn(a.x, nsamples), qbyte(al.x)),
-                            __fmul_rn(__fdiv_rn(a.y, nsamples), qbyte(al.y)),
-                            __fmul_rn(__fdiv_rn(a.z, nsamples), qbyte(al.z)), 1.0f);
-}
-
 __device__ __forceinline__ float metering(int W, int H, int x, int y) {  // histogram.cu:35-48
     int cx = (int)__fdiv_rn((float)W, 2.0f), cy = (int)__fdiv_rn((float)H, 2.0f);
     float dx = (float)(cx - x), dy = (float)(cy - y);
@@ -208,11 +212,27 @@ __global__ void __launch_bounds__(256) k_histogram(int W, int H, const float4* r
     if (sh[threadIdx.x]) atomicAdd(&hist[threadIdx.x], sh[threadIdx.x]);
 }
 
-__global__ void k_exposure(const unsigned long long* hist, ExposureState* st, ExposureIn in) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    unsigned long long total = 0, wsum = 0;
-    for (int b = 0; b < 256; ++b) { total += hist[b]; wsum += hist[b] * (unsigned long long)b; }
-    double nonblack = (double)(total - hist[0]) / 16777216.0;
+// One block of 256 threads, a bin each; the sums are whole numbers, so their
+// order is free.  The rest is one thread's chain of double-precision functions.
+__global__ void __launch_bounds__(256) k_exposure(const unsigned long long* hist, ExposureState* st, ExposureIn in) {
+    __shared__ unsigned long long sums[2][8];
+    const unsigned long long mine = hist[threadIdx.x];
+    unsigned long long total = threadIdx.x ? mine : 0, wsum = mine * threadIdx.x;   // bin 0 is black
+    for (int o = 16; o > 0; o >>= 1) {
+        total += __shfl_down_sync(0xffffffffu, total, o);
+        wsum += __shfl_down_sync(0xffffffffu, wsum, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sums[0][threadIdx.x >> 5] = total;
+        sums[1][threadIdx.x >> 5] = wsum;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; ++w) {
+        total += sums[0][w];
+        wsum += sums[1][w];
+    }
+    double nonblack = (double)total / 16777216.0;
     if (nonblack < 0.001) nonblack = 0.001;
     double avg_bin = ((double)wsum / 16777216.0) / nonblack;
     double range = (double)in.white_ev - (double)in.black_ev;

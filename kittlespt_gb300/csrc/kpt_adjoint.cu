@@ -843,17 +843,23 @@ static __device__ __noinline__ void sky_jacobian_now(const SkyParams& P, float3 
 // The sky radiance at the end of the paths that escaped at `level` (the
 // forward's march), for k_adj_sweep: from the end of level - 1's escapes to
 // the number k_adj_shadow(level) recorded.
-__global__ void __launch_bounds__(PATH_BLOCK) k_adj_sky(FrameParams F, AdjParams A, int level) {
+template <int LANES>
+__device__ __forceinline__ void adj_sky(const FrameParams& F, const AdjParams& A, int q0, int n) {
     const SkyParams& P = F.sky;
     const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);
-    const int* mark = F.level_counts + 5;
-    const int n = mark[LEVEL_WORDS * level];
-    for (int q = mark[LEVEL_WORDS * (level - 1)] + blockIdx.x * blockDim.x + threadIdx.x; q < n;
-         q += gridDim.x * blockDim.x) {
+    sky_spread<LANES>(q0, n, [&](int q, bool first) {
         const int i = A.esc[q];
-        const float3 s = nishita(P, obs, xyz3(A.vend[2 * (size_t)i]));
-        A.vsky[i] = make_float4(s.x, s.y, s.z, 0.0f);
-    }
+        const float3 s = nishita<LANES>(P, obs, xyz3(A.vend[2 * (size_t)i]));
+        if (first) A.vsky[i] = make_float4(s.x, s.y, s.z, 0.0f);
+    });
+}
+__global__ void __launch_bounds__(PATH_BLOCK) k_adj_sky(FrameParams F, AdjParams A, int level) {
+    const int* mark = F.level_counts + 5;
+    const int q0 = mark[LEVEL_WORDS * (level - 1)], n = mark[LEVEL_WORDS * level];
+    const int lanes = sky_lanes(n - q0, gridDim.x * blockDim.x);
+    if (lanes == 8) adj_sky<8>(F, A, q0, n);
+    else if (lanes == 2) adj_sky<2>(F, A, q0, n);
+    else adj_sky<1>(F, A, q0, n);
 }
 
 // Adds the lanes' v (to the gradients of material mat's four parameters) to

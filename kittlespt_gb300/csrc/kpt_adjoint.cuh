@@ -591,66 +591,72 @@ static __device__ __noinline__ float3 nishita_grad(const SkyParams& P, float3 o,
         if (te > tmin && te > 0.0f) tmin = te;
         if (tx < tmax) tmax = tx;
     }
-    const float step = xm(xs(tmax, tmin), 0.0625f);
+    const SkyIeee A(P);
+    const float step = SkyIeee::part(tmin, tmax);
     const float3 tR = make_float3(xa(P.sigma_r.x, 0.0f), xa(P.sigma_r.y, 0.0f), xa(P.sigma_r.z, 0.0f));
     const float tM = xa(P.sigma_m, P.sigma_am);
     const float half = xm(step, 0.5f);
-    const float ihr2 = 1.0f / (P.h_r * P.h_r), ihm2 = 1.0f / (P.h_m * P.h_m);
+    const float2 ih2 = make_float2(1.0f / (P.h_r * P.h_r), 1.0f / (P.h_m * P.h_m));
     float t = tmin;
-    float3 iR = make_float3(0.0f, 0.0f, 0.0f), iM = make_float3(0.0f, 0.0f, 0.0f);
-    // derivatives of iR, iM: [0] d/d sigma_r (own channel), [1] d/d sigma_m, [2] d/d h_r, [3] d/d h_m
-    float3 diR[4], diM[4];
-    for (int k = 0; k < 4; ++k) diR[k] = diM[k] = make_float3(0.0f, 0.0f, 0.0f);
-    float oR = 0.0f, oM = 0.0f, doR = 0.0f, doM = 0.0f;   // doR = d oR / d h_r, doM = d oM / d h_m
+    // pairs: (Rayleigh, Mie)
+    float2 in[3] = {both(0.0f), both(0.0f), both(0.0f)};
+    // derivatives of in: [0] d/d sigma_r (own channel), [1] d/d sigma_m, [2] d/d h_r, [3] d/d h_m
+    float2 din[4][3];
+    for (int k = 0; k < 4; ++k) din[k][0] = din[k][1] = din[k][2] = both(0.0f);
+    float2 opt = both(0.0f), dopt = both(0.0f);   // dopt: d opt / d scale height
 #pragma unroll 1
     for (int i = 0; i < 16; ++i) {
-        float3 sp = xpoint(o, xa(t, half), d);
-        float alt = xs(__fsqrt_rn(xdot(sp, sp)), P.earth_r);
-        float pR = xm(expf(-alt * P.inv_h_r), step);
-        float pM = xm(expf(-alt * P.inv_h_m), step);
-        float dpR = pR * alt * ihr2, dpM = pM * alt * ihm2;   // d/d h of exp(-alt / h) * step
-        oR = xa(oR, pR);
-        oM = xa(oM, pM);
-        doR += dpR;
-        doM += dpM;
+        const float3 sp = xpoint(o, xa(t, half), d);
+        const float alt = xs(SkyIeee::radius(sp), P.earth_r);
+        const float2 p = __fmul2_rn(exp_pair(__fmul2_rn(both(alt), make_float2(A.nhr, A.nhm))), both(step));
+        const float2 dp = __fmul2_rn(__fmul2_rn(p, both(alt)), ih2);   // d/d h of exp(-alt / h) * step
+        opt = A.sum(opt, p);
+        dopt = A.sum(dopt, dp);
         float lte, ltx;
         sphere_hit(sp, P.sun_dir, P.atm_r, &lte, &ltx);
-        float lstep = xm(ltx, 0.125f);
-        float lhalf = xm(lstep, 0.5f);
-        float lt = 0.0f, lR = 0.0f, lM = 0.0f, dlR = 0.0f, dlM = 0.0f;
+        const float lstep = SkyIeee::eighth(ltx);
+        const float2 lhalf = both(xm(lstep, 0.5f)), len = both(lstep);
+        float lt = 0.0f;
+        float2 l = both(0.0f), dl = both(0.0f);
         int j;
 #pragma unroll
-        for (j = 0; j < 8; ++j) {
-            float3 spl = xpoint(sp, xa(lt, lhalf), P.sun_dir);
-            float altl = xs(__fsqrt_rn(xdot(spl, spl)), P.earth_r);
-            if (altl < 0.0f) break;
-            float eR = xm(expf(-altl * P.inv_h_r), lstep), eM = xm(expf(-altl * P.inv_h_m), lstep);
-            lR = xa(lR, eR);
-            lM = xa(lM, eM);
-            dlR += eR * altl * ihr2;
-            dlM += eM * altl * ihm2;
-            lt = xa(lt, lstep);
+        for (j = 0; j < 8; j += 2) {
+            const float lt1 = xa(lt, lstep);
+            const float2 u = __fadd2_rn(make_float2(lt, lt1), lhalf);
+            const float2 a = light_heights(A, P, sp, u);
+            if (a.x < 0.0f || a.y < 0.0f) break;
+            const float2 r = exp_pair(__fmul2_rn(a, both(A.nhr))), m = exp_pair(__fmul2_rn(a, both(A.nhm)));
+            const float2 e0 = __fmul2_rn(make_float2(r.x, m.x), len), e1 = __fmul2_rn(make_float2(r.y, m.y), len);
+            l = A.sum(A.sum(l, e0), e1);
+            dl = __ffma2_rn(__fmul2_rn(e0, both(a.x)), ih2, dl);
+            dl = __ffma2_rn(__fmul2_rn(e1, both(a.y)), ih2, dl);
+            lt = xa(lt1, lstep);
         }
         if (j == 8) {
-            float sr = xa(oR, lR), sm = xa(oM, lM);
-            float dsr = doR + dlR, dsm = doM + dlM;
-            float tmm = xm(tM, sm);
-            float3 tau = make_float3(xa(xm(tR.x, sr), tmm), xa(xm(tR.y, sr), tmm), xa(xm(tR.z, sr), tmm));
-            float3 Tr = make_float3(expf(-tau.x), expf(-tau.y), expf(-tau.z));
-            iR = make_float3(xa(iR.x, xm(Tr.x, pR)), xa(iR.y, xm(Tr.y, pR)), xa(iR.z, xm(Tr.z, pR)));
-            iM = make_float3(xa(iM.x, xm(Tr.x, pM)), xa(iM.y, xm(Tr.y, pM)), xa(iM.z, xm(Tr.z, pM)));
-            // d tau: sigma_r (own channel) sr; sigma_m sm; h_r sigma_r dsr; h_m tM dsm; dTr = -Tr dtau
-            const float3 dtau[4] = {make_float3(sr, sr, sr), make_float3(sm, sm, sm), tR * dsr,
-                                    make_float3(tM * dsm, tM * dsm, tM * dsm)};
-            for (int k = 0; k < 4; ++k) {
-                float3 dTr = -zmul(Tr, dtau[k]);
-                diR[k] = diR[k] + dTr * pR;
-                diM[k] = diM[k] + dTr * pM;
+            const float2 s = __fadd2_rn(opt, l), ds = __fadd2_rn(dopt, dl);
+            const float3 tau = SkyIeee::depth(tR, tM, s);
+            const float T[3] = {expf(-tau.x), expf(-tau.y), expf(-tau.z)};
+            // d tau: sigma_r (own channel) s.x; sigma_m s.y; h_r sigma_r ds.x; h_m tM ds.y; dT = -T dtau
+            const float hr[3] = {tR.x * ds.x, tR.y * ds.x, tR.z * ds.x}, hm = tM * ds.y;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                in[c] = A.add(in[c], both(T[c]), p);
+                const bool some = T[c] != 0.0f;
+                const float dtau[4] = {s.x, s.y, hr[c], hm};
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    din[k][c] = __ffma2_rn(both(some ? -(T[c] * dtau[k]) : -0.0f), p, din[k][c]);
+                din[2][c].x += some ? T[c] * dp.x : 0.0f;
+                din[3][c].y += some ? T[c] * dp.y : 0.0f;
             }
-            diR[2] = diR[2] + zmul(Tr, make_float3(dpR, dpR, dpR));
-            diM[3] = diM[3] + zmul(Tr, make_float3(dpM, dpM, dpM));
         }
         t = xa(t, step);
+    }
+    const float3 iR = make_float3(in[0].x, in[1].x, in[2].x), iM = make_float3(in[0].y, in[1].y, in[2].y);
+    float3 diR[4], diM[4];
+    for (int k = 0; k < 4; ++k) {
+        diR[k] = make_float3(din[k][0].x, din[k][1].x, din[k][2].x);
+        diM[k] = make_float3(din[k][0].y, din[k][1].y, din[k][2].y);
     }
     float mu = dot(d, P.sun_dir);
     float rp = (3.0f * (1.0f + Sqr(mu))) / (16.0f * PI_F);

@@ -925,6 +925,7 @@ kpt_status kpt_reset_accumulation(kpt_context* c) {
 
 static SkyParams sky_params(const kpt_environment& e) {
     SkyParams P{};
+    P.one = 1.0f;
     // getSunDirection (integrator.cuh:222-230), single precision as on the device
     float cp = cosf(e.sun_phi), sp = sinf(e.sun_phi), ct = cosf(e.sun_theta), st = sinf(e.sun_theta);
     float3 d = make_float3(cp * ct, st, sp * ct);
@@ -1749,7 +1750,11 @@ kpt_status kpt_sky_device(kpt_context* c, int n, const float* dirs, float* rgb) 
     if (!c || n < 0 || (n > 0 && (!dirs || !rgb))) return fail(KPT_ERR_INVALID, "kpt_sky_device: bad arguments");
     KPT_CUDA(cudaSetDevice(c->device));
     if (n == 0) return KPT_OK;
-    k_sky<<<(n + 127) / 128, 128, 0, c->stream>>>(frame_sky(c), n, (const float3*)dirs, (float3*)rgb);
+    // several lanes per direction where the GPU has the threads for them
+    const long long threads = (long long)persistent_grid(c, (const void*)k_sky, SKY_BLOCK) * SKY_BLOCK;
+    const int lanes = 8LL * n <= threads ? 8 : 2LL * n <= threads ? 2 : 1;
+    const int per_block = SKY_BLOCK / lanes;
+    k_sky<<<(n - 1) / per_block + 1, SKY_BLOCK, 0, c->stream>>>(frame_sky(c), n, lanes, (const float3*)dirs, (float3*)rgb);
     c->launches += 1;
     KPT_CUDA(cudaGetLastError());
     return KPT_OK;

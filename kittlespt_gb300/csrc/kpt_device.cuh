@@ -126,6 +126,7 @@ struct SkyParams {
     float cos_half_sun;       // LeSun threshold
     float sun_radius_m;       // physical radius of the sun disc at 1 AU
     float3 sun_radiance;      // Nishita radiance towards the sun (constant per frame)
+    float one;                // 1.0f, for sums that must not be fused with a product
     int gpu_arith;            // 1: sky and sun in the reference GPU build's arithmetic, 0: IEEE
 };
 

@@ -7,6 +7,7 @@
 namespace kpt {
 
 constexpr int PATH_BLOCK = 128;    // threads per block of the shading kernels
+constexpr int SKY_BLOCK = 64;
 constexpr int SHADE_MAX_BLOCK = 256;   // largest block k_shade is launched with (kpt_tuning.shade_block)
 constexpr int SHADE_WINDOW = 2048;     // largest window of paths k_shade regroups by lobe family (kpt_tuning.group_lobes)
 constexpr int TRACE_BLOCK = 128;   // threads per block of the ray kernels
@@ -289,7 +290,7 @@ __global__ void k_temporal(TemporalParams T);       // kpt_post.cu, IEEE
 __global__ void k_temporal_gpu(TemporalParams T);   // kpt_path.cu, the reference GPU build's arithmetic
 // with `render`, also the image sum / total_samples * albedo
 __global__ void k_accumulate(FrameParams F, float total_samples, float4* render);
-__global__ void k_sky(SkyParams P, int n, const float3* dirs, float3* out);
+__global__ void k_sky(SkyParams P, int n, int lanes, const float3* dirs, float3* out);
 __global__ void k_trace(SceneView s, int n, const float3* o, const float3* d, float tmin, float tmax,
                         int* inst, int* tri, float* t, float2* uv, int* next, unsigned long long* counters);
 __global__ void k_occluded(SceneView s, int n, const float3* o, const float3* d, float tmin, const float* tmax,

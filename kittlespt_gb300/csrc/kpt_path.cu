@@ -131,18 +131,26 @@ __global__ void __launch_bounds__(PATH_BLOCK) k_primary_surface(FrameParams F) {
 }
 
 // sky (times LeSun) of every pixel whose camera ray misses
-__global__ void __launch_bounds__(PATH_BLOCK) k_primary_sky(FrameParams F) {
-    const int n = F.counts[1];
+template <int LANES>
+__device__ __forceinline__ void primary_sky(const FrameParams& F, int n) {
     const SkyParams& P = F.sky;
     const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    sky_spread<LANES>(0, n, [&](int i, bool first) {
         int p = F.miss_list[i];
         XRay r = camera_ray(F, p % F.W, p / F.W);
-        float3 sk = nishita(P, obs, r.d) * le_sun(P, r.d);
+        float3 sk = nishita<LANES>(P, obs, r.d) * le_sun(P, r.d);
         float4 v = make_float4(sk.x, sk.y, sk.z, 0.0f);
-        F.pixel_sky[p] = v;
-        if (F.albedo) F.albedo[p] = v;
-    }
+        if (first) {
+            F.pixel_sky[p] = v;
+            if (F.albedo) F.albedo[p] = v;
+        }
+    });
+}
+__global__ void __launch_bounds__(PATH_BLOCK) k_primary_sky(FrameParams F) {
+    const int n = F.counts[1], lanes = sky_lanes(n, gridDim.x * blockDim.x);
+    if (lanes == 8) primary_sky<8>(F, n);
+    else if (lanes == 2) primary_sky<2>(F, n);
+    else primary_sky<1>(F, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -1187,6 +1195,19 @@ __global__ void k_merge_inst(const InstRec* src, int n, InstRec* dst, int mesh_a
     dst[i] = r;
 }
 
+template <int LANES>
+__device__ __forceinline__ void sky_queue(const FrameParams& F, int i0, int n) {
+    const SkyParams& P = F.sky;
+    const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);
+    sky_spread<LANES>(i0, n, [&](int i, bool first) {
+        float4 a = F.sky_queue[2 * (size_t)i], b = F.sky_queue[2 * (size_t)i + 1];
+        int item = __float_as_int(a.x);
+        float3 sk = nishita<LANES>(P, obs, make_float3(a.y, a.z, a.w));
+        if (!first) return;
+        float4 L = F.radiance[item];
+        F.radiance[item] = make_float4(L.x + sk.x * b.x, L.y + sk.y * b.y, L.z + sk.z * b.z, 0.0f);
+    });
+}
 // sky * throughput of every path that left the scene, added to its sample:
 // the whole queue (level < 0), or the entries k_shade(level) appended, from
 // the end of level - 1's range (the wave's starting length for level 0) to
@@ -1199,15 +1220,10 @@ __global__ void __launch_bounds__(PATH_BLOCK) k_sky_queue(FrameParams F, int lev
         i0 = mark[LEVEL_WORDS * (level > 0 ? level - 1 : F.max_depth + 1)];
         if (!rest) n = mark[LEVEL_WORDS * level];
     }
-    const SkyParams& P = F.sky;
-    const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);
-    for (int i = i0 + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float4 a = F.sky_queue[2 * (size_t)i], b = F.sky_queue[2 * (size_t)i + 1];
-        int item = __float_as_int(a.x);
-        float3 sk = nishita(P, obs, make_float3(a.y, a.z, a.w));
-        float4 L = F.radiance[item];
-        F.radiance[item] = make_float4(L.x + sk.x * b.x, L.y + sk.y * b.y, L.z + sk.z * b.z, 0.0f);
-    }
+    const int lanes = sky_lanes(n - i0, gridDim.x * blockDim.x);
+    if (lanes == 8) sky_queue<8>(F, i0, n);
+    else if (lanes == 2) sky_queue<2>(F, i0, n);
+    else sky_queue<1>(F, i0, n);
 }
 
 // The sun's constants in the reference GPU build's arithmetic (fast sine,
@@ -1226,16 +1242,24 @@ __global__ void k_sun_constants_gpu(float phi, float theta, float diameter, floa
 
 // Nishita radiance towards the sun: a per-frame constant.
 __global__ void k_sky_constants(FrameParams F, float3* sun_radiance) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const SkyParams& P = F.sky;
-        *sun_radiance = nishita(P, make_float3(0.0f, P.earth_r + 1.0f, 0.0f), P.sun_dir);
-    }
+    if (threadIdx.x >= 8 || blockIdx.x != 0) return;
+    const SkyParams& P = F.sky;
+    const float3 L = nishita<8>(P, make_float3(0.0f, P.earth_r + 1.0f, 0.0f), P.sun_dir);
+    if (threadIdx.x == 0) *sun_radiance = L;
 }
 
-// Sky radiance for a list of directions (tests and tools).
-__global__ void k_sky(SkyParams P, int n, const float3* dirs, float3* out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = nishita(P, make_float3(0.0f, P.earth_r + 1.0f, 0.0f), dirs[i]);
+// Sky radiance for a list of directions, `lanes` (8, 2 or 1) threads each.
+template <int LANES>
+__device__ __forceinline__ void sky_list(const SkyParams& P, int n, const float3* dirs, float3* out) {
+    sky_spread<LANES>(0, n, [&](int i, bool first) {
+        const float3 L = nishita<LANES>(P, make_float3(0.0f, P.earth_r + 1.0f, 0.0f), dirs[i]);
+        if (first) out[i] = L;
+    });
+}
+__global__ void __launch_bounds__(SKY_BLOCK) k_sky(SkyParams P, int n, int lanes, const float3* dirs, float3* out) {
+    if (lanes == 8) sky_list<8>(P, n, dirs, out);
+    else if (lanes == 2) sky_list<2>(P, n, dirs, out);
+    else sky_list<1>(P, n, dirs, out);
 }
 
 // ---------------------------------------------------------------------------

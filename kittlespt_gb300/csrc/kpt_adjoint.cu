@@ -106,19 +106,16 @@ __device__ __forceinline__ bool sky_in_band(const SkyParams& P, float3 d) {
     return fabsf(d.y) < 0.05f || dot(d, P.sun_dir) > 0.995f;
 }
 
-// Queues an escape's sky Jacobian (direction d) with its gradient weight w
-// in queue q (count, capacity cap); false when there is no queue or it is
-// full (the caller evaluates the Jacobian at once).
-__device__ __forceinline__ bool sky_push(float4* q, int* count, int cap, float3 d, float3 w) {
-    if (!q) return false;
-    const int i = atomicAdd(count, 1);
-    if (i >= cap) return false;
-    q[2 * (size_t)i] = make_float4(d.x, d.y, d.z, 0.0f);
-    q[2 * (size_t)i + 1] = make_float4(w.x, w.y, w.z, 0.0f);
-    return true;
-}
+// Queues an escape's double-precision sky Jacobian (direction d) with its
+// gradient weight w; false when there is no queue or it is full (the caller
+// evaluates the Jacobian at once).
 __device__ __forceinline__ bool sky_defer(const AdjParams& A, float3 d, float3 w) {
-    return sky_push(A.skyq, A.skyq_count, A.skyq_cap, d, w);
+    if (!A.skyq) return false;
+    const int i = atomicAdd(A.skyq_count, 1);
+    if (i >= A.skyq_cap) return false;
+    A.skyq[2 * (size_t)i] = make_float4(d.x, d.y, d.z, 0.0f);
+    A.skyq[2 * (size_t)i + 1] = make_float4(w.x, w.y, w.z, 0.0f);
+    return true;
 }
 
 // Pixels whose camera ray misses: every sample is sky(d) * LeSun(d).
@@ -430,14 +427,11 @@ __device__ __forceinline__ void adjoint_items(const FrameParams& F, const AdjPar
                 // The sky Jacobian at the escape: near the sun (Mie forward
                 // peak) and the horizon the single-precision march's
                 // derivatives are ill-conditioned, so there it is evaluated
-                // in double.  Both kinds are queued for batched kernels
-                // (k_adjoint_sky_d / _f), which march on full warps instead
-                // of the few lanes of a warp that escape together here.
+                // in double (queued, where there is a queue, for
+                // k_adjoint_sky_d).
                 const float3 gb = wmul(g, b_end);
                 const bool band = sky_in_band(P, d_end);
-                const bool done = band ? sky_defer(A, d_end, gb)
-                                       : sky_push(A.skyqf, A.skyqf_count, A.skyqf_cap, d_end, gb);
-                if (!done) {
+                if (!(band && sky_defer(A, d_end, gb))) {
                     float3 J_end[SKY_PARAMS];
                     if (band) nishita_jacobian_d(P, obs, d_end, J_end);
                     else nishita_grad(P, obs, d_end, J_end);
@@ -493,25 +487,18 @@ __device__ __forceinline__ void adjoint_block(const FrameParams& F, const AdjPar
 }
 
 
-// The deferred sky Jacobians: weight . J(d) per queued escape, summed into
-// the sky parameters' gradients; in double (DBL, the band near the horizon
-// and the sun) or single precision.
-template <bool DBL>
-__device__ __forceinline__ void sky_jacobians(const FrameParams& F, const float4* q, const int* count, int cap,
-                                              double* grad) {
+// The sky parameters' gradients summed over n entries: jacobian(i, J) gives
+// entry i's Jacobian and returns its weight.
+template <class Jacobian>
+__device__ __forceinline__ void sum_jacobians(int n, double* grad, Jacobian jacobian) {
     __shared__ double sg[SKY_PARAMS];
+    if ((int)(blockIdx.x * blockDim.x) >= n) return;   // the sums of blocks without entries would cost FP64 time too
     if (threadIdx.x < SKY_PARAMS) sg[threadIdx.x] = 0.0;
     __syncthreads();
-    const SkyParams& P = F.sky;
-    const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);
-    const int n = min(*count, cap);
     double gsky[SKY_PARAMS] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 a = q[2 * (size_t)i], b = q[2 * (size_t)i + 1];
         float3 J[SKY_PARAMS];
-        if (DBL) nishita_jacobian_s(P, obs, make_float3(a.x, a.y, a.z), J);
-        else nishita_grad(P, obs, make_float3(a.x, a.y, a.z), J);
-        const float3 w = make_float3(b.x, b.y, b.z);
+        const float3 w = jacobian(i, J);
         for (int k = 0; k < SKY_PARAMS; ++k) gsky[k] += wdot(w, J[k]);
     }
     for (int k = 0; k < SKY_PARAMS; ++k) {
@@ -523,11 +510,45 @@ __device__ __forceinline__ void sky_jacobians(const FrameParams& F, const float4
     if (threadIdx.x < SKY_PARAMS && sg[threadIdx.x] != 0.0) atomicAdd(grad + threadIdx.x, sg[threadIdx.x]);
 }
 
+// The deferred sky Jacobians (the band near the horizon and the sun, in
+// double).
 __global__ void __launch_bounds__(PATH_BLOCK) k_adjoint_sky_d(FrameParams F, AdjParams A) {
-    sky_jacobians<true>(F, A.skyq, A.skyq_count, A.skyq_cap, A.grad + 4 * A.nmat);
+    const SkyParams& P = F.sky;
+    const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);
+    sum_jacobians(min(*A.skyq_count, A.skyq_cap), A.grad + 4 * A.nmat, [&](int i, float3* J) {
+        const float4 a = A.skyq[2 * (size_t)i], b = A.skyq[2 * (size_t)i + 1];
+        nishita_jacobian_s(P, obs, make_float3(a.x, a.y, a.z), J);
+        return make_float3(b.x, b.y, b.z);
+    });
 }
-__global__ void __launch_bounds__(PATH_BLOCK) k_adjoint_sky_f(FrameParams F, AdjParams A) {
-    sky_jacobians<false>(F, A.skyqf, A.skyqf_count, A.skyqf_cap, A.grad + 4 * A.nmat);
+
+// A sky Jacobian's twelve values (a Rayleigh coefficient moves its own channel
+// only) in three float4s.
+__device__ __forceinline__ void store_jacobian(float4* v, const float3* J) {
+    v[0] = make_float4(J[SKY_RAYLEIGH_R].x, J[SKY_RAYLEIGH_G].y, J[SKY_RAYLEIGH_B].z, J[SKY_MIE].x);
+    v[1] = make_float4(J[SKY_MIE].y, J[SKY_MIE].z, J[SKY_RAYLEIGH_H].x, J[SKY_RAYLEIGH_H].y);
+    v[2] = make_float4(J[SKY_RAYLEIGH_H].z, J[SKY_MIE_H].x, J[SKY_MIE_H].y, J[SKY_MIE_H].z);
+}
+__device__ __forceinline__ void load_jacobian(const float4* v, float3* J) {
+    const float4 a = v[0], b = v[1], c = v[2];
+    J[SKY_RAYLEIGH_R] = make_float3(a.x, 0.0f, 0.0f);
+    J[SKY_RAYLEIGH_G] = make_float3(0.0f, a.y, 0.0f);
+    J[SKY_RAYLEIGH_B] = make_float3(0.0f, 0.0f, a.z);
+    J[SKY_MIE] = make_float3(a.w, b.x, b.y);
+    J[SKY_RAYLEIGH_H] = make_float3(b.z, b.w, c.x);
+    J[SKY_MIE_H] = make_float3(c.y, c.z, c.w);
+}
+
+// The single-precision sky Jacobians of the wave's other escapes, which
+// k_adj_sky stored, with the weights of k_adj_sweep.  (Summed in the sweep
+// itself, where half a warp's paths escape, they cost it 120 us of
+// 512x512x32 samples, here 110: both are bound by the FP64 additions.)
+__global__ void __launch_bounds__(PATH_BLOCK) k_adjoint_sky_w(AdjParams A) {
+    sum_jacobians(*A.skyw_count, A.grad + 4 * A.nmat, [&](int i, float3* J) {
+        const float4 w = A.skyw[i];
+        load_jacobian(A.vskyJ + 3 * (size_t)__float_as_int(w.w), J);
+        return make_float3(w.x, w.y, w.z);
+    });
 }
 __global__ void __launch_bounds__(PATH_BLOCK) k_adjoint_rec(FrameParams F, AdjParams A) { adjoint_block<true>(F, A); }
 
@@ -830,35 +851,36 @@ __global__ void __launch_bounds__(TRACE_BLOCK, TRACE_MIN_BLOCKS) k_adj_shadow(Fr
     trace_queue<true>(F.scene, lc[1] + lc[2], lc + 4, q, st, stack);
 }
 
-// An escape's sky Jacobian evaluated where it occurs (its queue is full):
-// weight . J added to the block's sky gradient slots.
-static __device__ __noinline__ void sky_jacobian_now(const SkyParams& P, float3 obs, float3 d, bool band, float3 w,
-                                                     double* slots) {
+// An escape's sky Jacobian in double evaluated where it occurs (the queue is
+// full): weight . J added to the block's sky gradient slots.
+static __device__ __noinline__ void sky_jacobian_now(const SkyParams& P, float3 obs, float3 d, float3 w, double* slots) {
     float3 J[SKY_PARAMS];
-    if (band) nishita_jacobian_d(P, obs, d, J);
-    else nishita_grad(P, obs, d, J);
+    nishita_jacobian_d(P, obs, d, J);
     for (int q = 0; q < SKY_PARAMS; ++q) atomicAdd(slots + q, (double)wdot(w, J[q]));
 }
 
 // The sky radiance at the end of the paths that escaped at `level` (the
-// forward's march), for k_adj_sweep: from the end of level - 1's escapes to
-// the number k_adj_shadow(level) recorded.
+// forward's march) and its single-precision Jacobian, which the same march
+// gives for a third more, for k_adj_sweep: from the end of level - 1's escapes
+// to the number k_adj_shadow(level) recorded.  (A march of its own per escape
+// in the backward half took 1070 us of 512x512x32 samples; this kernel went from 663 to 900.)
 template <int LANES>
 __device__ __forceinline__ void adj_sky(const FrameParams& F, const AdjParams& A, int q0, int n) {
     const SkyParams& P = F.sky;
     const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);
     sky_spread<LANES>(q0, n, [&](int q, bool first) {
         const int i = A.esc[q];
-        const float3 s = nishita<LANES>(P, obs, xyz3(A.vend[2 * (size_t)i]));
-        if (first) A.vsky[i] = make_float4(s.x, s.y, s.z, 0.0f);
+        float3 J[SKY_PARAMS];
+        const float3 s = nishita_grad<LANES>(P, obs, xyz3(A.vend[2 * (size_t)i]), J);
+        if (!first) return;
+        A.vsky[i] = make_float4(s.x, s.y, s.z, 0.0f);
+        store_jacobian(A.vskyJ + 3 * (size_t)i, J);
     });
 }
 __global__ void __launch_bounds__(PATH_BLOCK) k_adj_sky(FrameParams F, AdjParams A, int level) {
     const int* mark = F.level_counts + 5;
     const int q0 = mark[LEVEL_WORDS * (level - 1)], n = mark[LEVEL_WORDS * level];
-    const int lanes = sky_lanes(n - q0, gridDim.x * blockDim.x);
-    if (lanes == 8) adj_sky<8>(F, A, q0, n);
-    else if (lanes == 2) adj_sky<2>(F, A, q0, n);
+    if (8LL * (n - q0) <= (long long)gridDim.x * blockDim.x) adj_sky<8>(F, A, q0, n);
     else adj_sky<1>(F, A, q0, n);
 }
 
@@ -922,16 +944,6 @@ __device__ __forceinline__ float3 sample_weight(const AdjParams& A, int p, float
     return make_float3(a.x, a.y, a.z) * msk * inv_n;
 }
 
-// Queues the sky Jacobian of an escaped path (its last direction and
-// throughput) with its gradient weight.
-__device__ __forceinline__ void queue_escape(const AdjParams& A, const SkyParams& P, float3 obs, float3 d, float3 beta,
-                                             float3 g, double* sky_slots) {
-    const float3 gb = wmul(g, beta);
-    const bool band = sky_in_band(P, d);
-    const bool done = band ? sky_defer(A, d, gb) : sky_push(A.skyqf, A.skyqf_count, A.skyqf_cap, d, gb);
-    if (!done) sky_jacobian_now(P, obs, d, band, gb, sky_slots);
-}
-
 // Every sample of the wave: its radiance from the vertex records (the
 // forward's sum), clamp, image, and the reverse sweep into the gradients.
 // Forward half: bound by the latency of the records' loads (held to 64
@@ -942,6 +954,11 @@ __device__ __forceinline__ void queue_escape(const AdjParams& A, const SkyParams
 __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjParams A, long long wave0) {
     extern __shared__ double sg[];
     const int ng = 4 * A.nmat + ADJ_SKY_PARAMS;
+    const int cap = F.cap;
+    const int nhit = F.counts[0];
+    const long long left = (long long)nhit * F.nsamples - wave0;
+    const int n = (int)(left < 0 ? 0 : (left < cap ? left : cap));
+    if ((long long)blockIdx.x * blockDim.x >= n) return;   // (its sums would cost FP64 time)
     grad_begin(sg, ng);
     // the sun light samples' weights, summed: their sky gradient is linear in
     // the sun's Jacobian, applied once at the end
@@ -949,10 +966,6 @@ __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjP
     const SkyParams& P = F.sky;
     const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);
     const float3 sun_rad = *F.sun_radiance;
-    const int cap = F.cap;
-    const int nhit = F.counts[0];
-    const long long left = (long long)nhit * F.nsamples - wave0;
-    const int n = (int)(left < 0 ? 0 : (left < cap ? left : cap));
     const float inv_n = 1.0f / (float)F.nsamples;
     // whole warps: every lane takes part in the warp's sums
     for (int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += gridDim.x * blockDim.x) {
@@ -998,8 +1011,13 @@ __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjP
             if (A.adjoint) {
                 R = s_end;
                 if (!nonzero(g)) nv = 0;
-                else if (escaped)
-                    queue_escape(A, P, obs, d_end, b_end, g, sg + 4 * A.nmat);
+                else if (escaped) {
+                    const float3 gb = wmul(g, b_end);
+                    if (!sky_in_band(P, d_end))   // one per path slot: the queue has room
+                        A.skyw[atomicAdd(A.skyw_count, 1)] = make_float4(gb.x, gb.y, gb.z, __int_as_float(i));
+                    else if (!sky_defer(A, d_end, gb))
+                        sky_jacobian_now(P, obs, d_end, gb, sg + 4 * A.nmat);
+                }
             }
         }
         if (A.image) image_add_warp(A.image, p, Lc * inv_n);

@@ -581,7 +581,50 @@ static __device__ __noinline__ void nishita_jacobian_s(const SkyParams& P, float
     }
 }
 
+// What a view step adds to a march with derivatives: the transmittance towards
+// the sun T, the optical depths s = (Rayleigh, Mie) and their derivatives ds by
+// the scale heights, the air p of the step and its derivative dp.
+struct GradStep {
+    float3 T;
+    float2 s, ds, p, dp;
+};
+template <int LANES>
+__device__ __forceinline__ GradStep step_of(unsigned mask, const GradStep& G, int lane) {
+    GradStep R;
+    R.T = make_float3(__shfl_sync(mask, G.T.x, lane, LANES), __shfl_sync(mask, G.T.y, lane, LANES),
+                      __shfl_sync(mask, G.T.z, lane, LANES));
+    R.s = shfl_pair<LANES>(mask, G.s, lane);
+    R.ds = shfl_pair<LANES>(mask, G.ds, lane);
+    R.p = shfl_pair<LANES>(mask, G.p, lane);
+    R.dp = shfl_pair<LANES>(mask, G.dp, lane);
+    return R;
+}
+
+// The march's sums, (Rayleigh, Mie) per channel, and their derivatives:
+// [0] d/d sigma_r (own channel), [1] d/d sigma_m, [2] d/d h_r, [3] d/d h_m.
+struct GradSums {
+    float2 in[3], din[4][3];
+    __device__ __forceinline__ void add(const SkyIeee& A, float3 tR, float tM, const GradStep& G) {
+        // d tau: sigma_r (own channel) s.x; sigma_m s.y; h_r sigma_r ds.x; h_m tM ds.y; dT = -T dtau
+        const float T[3] = {G.T.x, G.T.y, G.T.z};
+        const float hr[3] = {tR.x * G.ds.x, tR.y * G.ds.x, tR.z * G.ds.x}, hm = tM * G.ds.y;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            in[c] = A.add(in[c], both(T[c]), G.p);
+            const bool some = T[c] != 0.0f;
+            const float dtau[4] = {G.s.x, G.s.y, hr[c], hm};
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                din[k][c] = __ffma2_rn(both(some ? -(T[c] * dtau[k]) : -0.0f), G.p, din[k][c]);
+            din[2][c].x += some ? T[c] * G.dp.x : 0.0f;
+            din[3][c].y += some ? T[c] * G.dp.y : 0.0f;
+        }
+    }
+};
+
 // nishita() with its derivatives: J[i] = dL/d(parameter i), i < SKY_PARAMS.
+// LANES as there: the steps' sums are in the march's order, whatever LANES.
+template <int LANES = 1>
 static __device__ __noinline__ float3 nishita_grad(const SkyParams& P, float3 o, float3 d, float3* J) {
     for (int i = 0; i < SKY_PARAMS; ++i) J[i] = make_float3(0.0f, 0.0f, 0.0f);
     float tmin = 0.0f, tmax = __int_as_float(0x7f800000);
@@ -597,21 +640,34 @@ static __device__ __noinline__ float3 nishita_grad(const SkyParams& P, float3 o,
     const float tM = xa(P.sigma_m, P.sigma_am);
     const float half = xm(step, 0.5f);
     const float2 ih2 = make_float2(1.0f / (P.h_r * P.h_r), 1.0f / (P.h_m * P.h_m));
+    const int lane = threadIdx.x & (LANES - 1);
+    const unsigned mask = ((1u << (LANES & 31)) - 1u) << (threadIdx.x & 31 & ~(LANES - 1));
     float t = tmin;
-    // pairs: (Rayleigh, Mie)
-    float2 in[3] = {both(0.0f), both(0.0f), both(0.0f)};
-    // derivatives of in: [0] d/d sigma_r (own channel), [1] d/d sigma_m, [2] d/d h_r, [3] d/d h_m
-    float2 din[4][3];
-    for (int k = 0; k < 4; ++k) din[k][0] = din[k][1] = din[k][2] = both(0.0f);
+#pragma unroll
+    for (int q = 0; q < LANES - 1; ++q) t = q < lane ? xa(t, step) : t;
+    GradSums S;
+    for (int c = 0; c < 3; ++c) S.in[c] = S.din[0][c] = S.din[1][c] = S.din[2][c] = S.din[3][c] = both(0.0f);
     float2 opt = both(0.0f), dopt = both(0.0f);   // dopt: d opt / d scale height
 #pragma unroll 1
-    for (int i = 0; i < 16; ++i) {
+    for (int i = 0; i < 16; i += LANES) {
+        GradStep G;
         const float3 sp = xpoint(o, xa(t, half), d);
         const float alt = xs(SkyIeee::radius(sp), P.earth_r);
-        const float2 p = __fmul2_rn(exp_pair(__fmul2_rn(both(alt), make_float2(A.nhr, A.nhm))), both(step));
-        const float2 dp = __fmul2_rn(__fmul2_rn(p, both(alt)), ih2);   // d/d h of exp(-alt / h) * step
-        opt = A.sum(opt, p);
-        dopt = A.sum(dopt, dp);
+        G.p = __fmul2_rn(exp_pair(__fmul2_rn(both(alt), make_float2(A.nhr, A.nhm))), both(step));
+        G.dp = __fmul2_rn(__fmul2_rn(G.p, both(alt)), ih2);   // d/d h of exp(-alt / h) * step
+        if (LANES == 1) {
+            opt = A.sum(opt, G.p);
+            dopt = A.sum(dopt, G.dp);
+        } else {   // the sums up to this lane's step, carried on from the last lane's
+#pragma unroll
+            for (int q = 0; q < LANES; ++q) {
+                const float2 p = shfl_pair<LANES>(mask, G.p, q), dp = shfl_pair<LANES>(mask, G.dp, q);
+                if (q <= lane) {
+                    opt = A.sum(opt, p);
+                    dopt = A.sum(dopt, dp);
+                }
+            }
+        }
         float lte, ltx;
         sphere_hit(sp, P.sun_dir, P.atm_r, &lte, &ltx);
         const float lstep = SkyIeee::eighth(ltx);
@@ -632,31 +688,34 @@ static __device__ __noinline__ float3 nishita_grad(const SkyParams& P, float3 o,
             dl = __ffma2_rn(__fmul2_rn(e1, both(a.y)), ih2, dl);
             lt = xa(lt1, lstep);
         }
-        if (j == 8) {
-            const float2 s = __fadd2_rn(opt, l), ds = __fadd2_rn(dopt, dl);
-            const float3 tau = SkyIeee::depth(tR, tM, s);
-            const float T[3] = {expf(-tau.x), expf(-tau.y), expf(-tau.z)};
-            // d tau: sigma_r (own channel) s.x; sigma_m s.y; h_r sigma_r ds.x; h_m tM ds.y; dT = -T dtau
-            const float hr[3] = {tR.x * ds.x, tR.y * ds.x, tR.z * ds.x}, hm = tM * ds.y;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                in[c] = A.add(in[c], both(T[c]), p);
-                const bool some = T[c] != 0.0f;
-                const float dtau[4] = {s.x, s.y, hr[c], hm};
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    din[k][c] = __ffma2_rn(both(some ? -(T[c] * dtau[k]) : -0.0f), p, din[k][c]);
-                din[2][c].x += some ? T[c] * dp.x : 0.0f;
-                din[3][c].y += some ? T[c] * dp.y : 0.0f;
-            }
+        const bool lit = j == 8;
+        G.s = __fadd2_rn(opt, l);
+        G.ds = __fadd2_rn(dopt, dl);
+        if (LANES > 1 || lit) {
+            const float3 tau = SkyIeee::depth(tR, tM, G.s);
+            G.T = make_float3(expf(-tau.x), expf(-tau.y), expf(-tau.z));
         }
-        t = xa(t, step);
+        if (LANES == 1) {
+            if (lit) S.add(A, tR, tM, G);
+            t = xa(t, step);
+        } else {
+            const unsigned all = __ballot_sync(mask, lit) >> (threadIdx.x & 31 & ~(LANES - 1));
+#pragma unroll 1
+            for (int q = 0; q < LANES; ++q) {
+                const GradStep Q = step_of<LANES>(mask, G, q);
+                if (all >> q & 1) S.add(A, tR, tM, Q);
+            }
+            opt = shfl_pair<LANES>(mask, opt, LANES - 1);
+            dopt = shfl_pair<LANES>(mask, dopt, LANES - 1);
+#pragma unroll
+            for (int q = 0; q < LANES; ++q) t = xa(t, step);
+        }
     }
-    const float3 iR = make_float3(in[0].x, in[1].x, in[2].x), iM = make_float3(in[0].y, in[1].y, in[2].y);
+    const float3 iR = make_float3(S.in[0].x, S.in[1].x, S.in[2].x), iM = make_float3(S.in[0].y, S.in[1].y, S.in[2].y);
     float3 diR[4], diM[4];
     for (int k = 0; k < 4; ++k) {
-        diR[k] = make_float3(din[k][0].x, din[k][1].x, din[k][2].x);
-        diM[k] = make_float3(din[k][0].y, din[k][1].y, din[k][2].y);
+        diR[k] = make_float3(S.din[k][0].x, S.din[k][1].x, S.din[k][2].x);
+        diM[k] = make_float3(S.din[k][0].y, S.din[k][1].y, S.din[k][2].y);
     }
     float mu = dot(d, P.sun_dir);
     float rp = (3.0f * (1.0f + Sqr(mu))) / (16.0f * PI_F);

@@ -169,9 +169,7 @@ struct kpt_context {
     DBuf<int> rec_count;
     DBuf<float4> adj_skyq;      // deferred double-precision sky Jacobians: (direction, weight)
     DBuf<int> adj_skyq_count;
-    DBuf<float4> adj_skyqf;     // deferred single-precision sky Jacobians
-    DBuf<int> adj_skyqf_count;
-    DBuf<float4> adj_vr, adj_vend, adj_vsky;   // the wavefront replay's vertex and end records, escape skies
+    DBuf<float4> adj_vr, adj_vend, adj_vsky, adj_vskyJ, adj_skyw;   // the wavefront replay's vertex and end records, escape skies
     DBuf<float4> adj_lpath;                    // the split adjoint's per-path radiance
     // the records kept by kpt_adjoint_forward_device for the backward call,
     // and the state they were replayed in
@@ -347,8 +345,8 @@ kpt_status kpt_destroy(kpt_context* c) {
     c->unsorted.release(); c->octants.release();
     c->shadow.release(); c->fetch.release();
     c->sun_J.release(); c->adj_in.release(); c->adj_image.release(); c->adj_grad.release(); c->rec_count.release();
-    c->adj_skyq.release(); c->adj_skyq_count.release(); c->adj_skyqf.release(); c->adj_skyqf_count.release();
-    c->adj_vr.release(); c->adj_vend.release(); c->adj_vsky.release(); c->adj_lpath.release(); c->adj_vis.release(); c->adj_esc.release();
+    c->adj_skyq.release(); c->adj_skyq_count.release();
+    c->adj_vr.release(); c->adj_vend.release(); c->adj_vsky.release(); c->adj_vskyJ.release(); c->adj_skyw.release(); c->adj_lpath.release(); c->adj_vis.release(); c->adj_esc.release();
     for (auto* v : {&c->ev_fork, &c->ev_join})
         for (cudaEvent_t e : *v) cudaEventDestroy(e);
     if (c->ev_sky) cudaEventDestroy(c->ev_sky);
@@ -1938,12 +1936,12 @@ static kpt_status adjoint_run(kpt_context* c, int sample0, int nsamples, const f
         KPT_CUDA(c->adj_vr.ensure((size_t)AV_FIELDS * (D + 1) * F.cap));
         KPT_CUDA(c->adj_vend.ensure(2 * (size_t)F.cap));
         KPT_CUDA(c->adj_vsky.ensure((size_t)F.cap));
-        KPT_CUDA(c->adj_esc.ensure((size_t)F.cap + 1));
+        KPT_CUDA(c->adj_vskyJ.ensure(3 * (size_t)F.cap));
+        KPT_CUDA(c->adj_skyw.ensure((size_t)F.cap));
+        KPT_CUDA(c->adj_esc.ensure((size_t)F.cap + 2));
         KPT_CUDA(c->adj_vis.ensure((size_t)(D + 1) * F.cap));
         KPT_CUDA(c->adj_skyq.ensure(2 * std::min<size_t>(qcap, (size_t)INT32_MAX / 2)));
         KPT_CUDA(c->adj_skyq_count.ensure(1));
-        KPT_CUDA(c->adj_skyqf.ensure(2 * std::min<size_t>(qcap, (size_t)INT32_MAX / 2)));
-        KPT_CUDA(c->adj_skyqf_count.ensure(1));
     }
     AdjParams A{};
     A.adjoint = reinterpret_cast<const float4*>(adjoint);
@@ -1958,14 +1956,14 @@ static kpt_status adjoint_run(kpt_context* c, int sample0, int nsamples, const f
         A.skyq = c->adj_skyq.p;
         A.skyq_count = c->adj_skyq_count.p;
         A.skyq_cap = (int)(c->adj_skyq.n / 2);
-        A.skyqf = c->adj_skyqf.p;
-        A.skyqf_count = c->adj_skyqf_count.p;
-        A.skyqf_cap = (int)(c->adj_skyqf.n / 2);
         A.vr = c->adj_vr.p;
         A.vend = c->adj_vend.p;
         A.vsky = c->adj_vsky.p;
         A.esc = c->adj_esc.p;
         A.esc_count = c->adj_esc.p + F.cap;
+        A.vskyJ = c->adj_vskyJ.p;
+        A.skyw = c->adj_skyw.p;
+        A.skyw_count = c->adj_esc.p + F.cap + 1;
         A.vis = c->adj_vis.p;
     }
     cudaStream_t s = c->stream;
@@ -1974,7 +1972,6 @@ static kpt_status adjoint_run(kpt_context* c, int sample0, int nsamples, const f
     if (image) KPT_CUDA(cudaMemsetAsync(image, 0, sizeof(float4) * (size_t)np, s));
     KPT_CUDA(cudaMemsetAsync(c->rec_count.p, 0, sizeof(int), s));
     if (A.skyq) KPT_CUDA(cudaMemsetAsync(A.skyq_count, 0, sizeof(int), s));
-    if (A.skyqf) KPT_CUDA(cudaMemsetAsync(A.skyqf_count, 0, sizeof(int), s));
     KPT_CUDA(cudaMemsetAsync(c->counts.p, 0, 4 * sizeof(int), s));
     const void* kern = rec ? (const void*)k_adjoint_rec : (const void*)k_adj_sweep;
     for (const void* k : {kern, (const void*)k_adjoint_miss})
@@ -1998,19 +1995,15 @@ static kpt_status adjoint_run(kpt_context* c, int sample0, int nsamples, const f
         for (long long w0 = 0; w0 < items; w0 += F.cap) {
             st = adjoint_wave(c, F, A, w0);
             if (st != KPT_OK) return st;
+            KPT_CUDA(cudaMemsetAsync(A.skyw_count, 0, sizeof(int), s));
             k_adj_sweep<<<grid, PATH_BLOCK, smem, s>>>(F, A, w0);
-            c->launches += 1;
+            k_adjoint_sky_w<<<persistent_grid(c, (const void*)k_adjoint_sky_w, PATH_BLOCK), PATH_BLOCK, 0, s>>>(A);
+            c->launches += 2;
         }
     }
     if (A.skyq) {
-        // the double (FP64 pipe) and single-precision (FP32) Jacobians side by side
-        KPT_CUDA(cudaEventRecord(c->ev_fork[0], s));
-        KPT_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork[0], 0));
-        k_adjoint_sky_f<<<c->sm_count * 4, PATH_BLOCK, 0, c->side>>>(F, A);
-        KPT_CUDA(cudaEventRecord(c->ev_join[0], c->side));
         k_adjoint_sky_d<<<c->sm_count * 4, PATH_BLOCK, 0, s>>>(F, A);
-        KPT_CUDA(cudaStreamWaitEvent(s, c->ev_join[0], 0));
-        c->launches += 2;
+        c->launches += 1;
     }
     KPT_CUDA(cudaGetLastError());
     return KPT_OK;
@@ -2061,13 +2054,13 @@ kpt_status kpt_adjoint_forward_device(kpt_context* c, int sample0, int nsamples,
     KPT_CUDA(c->adj_vr.ensure((size_t)AV_FIELDS * (D + 1) * F.cap));
     KPT_CUDA(c->adj_vend.ensure(2 * (size_t)F.cap));
     KPT_CUDA(c->adj_vsky.ensure((size_t)F.cap));
-    KPT_CUDA(c->adj_esc.ensure((size_t)F.cap + 1));
+    KPT_CUDA(c->adj_vskyJ.ensure(3 * (size_t)F.cap));
+    KPT_CUDA(c->adj_skyw.ensure((size_t)F.cap));
+    KPT_CUDA(c->adj_esc.ensure((size_t)F.cap + 2));
     KPT_CUDA(c->adj_vis.ensure((size_t)(D + 1) * F.cap));
     KPT_CUDA(c->adj_lpath.ensure((size_t)F.cap));
     KPT_CUDA(c->adj_skyq.ensure(2 * std::min<size_t>(qcap, (size_t)INT32_MAX / 2)));
     KPT_CUDA(c->adj_skyq_count.ensure(1));
-    KPT_CUDA(c->adj_skyqf.ensure(2 * std::min<size_t>(qcap, (size_t)INT32_MAX / 2)));
-    KPT_CUDA(c->adj_skyqf_count.ensure(1));
     AdjParams A{};
     A.image = reinterpret_cast<float4*>(image);
     A.lpath = c->adj_lpath.p;
@@ -2078,14 +2071,14 @@ kpt_status kpt_adjoint_forward_device(kpt_context* c, int sample0, int nsamples,
     A.skyq = c->adj_skyq.p;
     A.skyq_count = c->adj_skyq_count.p;
     A.skyq_cap = (int)(c->adj_skyq.n / 2);
-    A.skyqf = c->adj_skyqf.p;
-    A.skyqf_count = c->adj_skyqf_count.p;
-    A.skyqf_cap = (int)(c->adj_skyqf.n / 2);
     A.vr = c->adj_vr.p;
     A.vend = c->adj_vend.p;
     A.vsky = c->adj_vsky.p;
     A.esc = c->adj_esc.p;
     A.esc_count = c->adj_esc.p + F.cap;
+    A.vskyJ = c->adj_vskyJ.p;
+    A.skyw = c->adj_skyw.p;
+    A.skyw_count = c->adj_esc.p + F.cap + 1;
     A.vis = c->adj_vis.p;
     cudaStream_t s = c->stream;
     KPT_CUDA(cudaMemsetAsync(image, 0, sizeof(float4) * (size_t)np, s));
@@ -2146,20 +2139,16 @@ kpt_status kpt_adjoint_backward_device(kpt_context* c, const float* adjoint, dou
     cudaStream_t s = c->stream;
     KPT_CUDA(cudaMemsetAsync(grad, 0, sizeof(double) * ng, s));
     KPT_CUDA(cudaMemsetAsync(A.skyq_count, 0, sizeof(int), s));
-    KPT_CUDA(cudaMemsetAsync(A.skyqf_count, 0, sizeof(int), s));
+    KPT_CUDA(cudaMemsetAsync(A.skyw_count, 0, sizeof(int), s));
     // (the sun's Jacobian, A.sun_J, came with the forward call)
     KPT_CUDA(cudaEventRecord(c->ev_fork[0], s));
     KPT_CUDA(cudaStreamWaitEvent(c->sky, c->ev_fork[0], 0));
     k_adjoint_miss<<<c->sm_count, PATH_BLOCK, smem, c->sky>>>(F, A);
     KPT_CUDA(cudaEventRecord(c->ev_sky, c->sky));
     k_adj_sweep<<<grid, PATH_BLOCK, smem, s>>>(F, A, 0);
+    k_adjoint_sky_w<<<persistent_grid(c, (const void*)k_adjoint_sky_w, PATH_BLOCK), PATH_BLOCK, 0, s>>>(A);
     KPT_CUDA(cudaStreamWaitEvent(s, c->ev_sky, 0));
-    KPT_CUDA(cudaEventRecord(c->ev_fork[0], s));
-    KPT_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork[0], 0));
-    k_adjoint_sky_f<<<c->sm_count * 4, PATH_BLOCK, 0, c->side>>>(F, A);
-    KPT_CUDA(cudaEventRecord(c->ev_join[0], c->side));
     k_adjoint_sky_d<<<c->sm_count * 4, PATH_BLOCK, 0, s>>>(F, A);
-    KPT_CUDA(cudaStreamWaitEvent(s, c->ev_join[0], 0));
     c->launches += 4;
     KPT_CUDA(cudaGetLastError());
     return KPT_OK;

@@ -134,11 +134,6 @@ struct AdjParams {
     float4* skyq;
     int* skyq_count;
     int skyq_cap;
-    // the other escapes' single-precision Jacobians, the same way, for
-    // k_adjoint_sky_f
-    float4* skyqf;
-    int* skyqf_count;
-    int skyqf_cap;
     // the wavefront replay: per vertex AV_FIELDS float4 fields, field f of
     // level l, path slot i at vr[(l * cap + i) * AV_FIELDS + f]; per path slot
     // its end (direction, vertex count; throughput, escaped) at vend[2 i],
@@ -147,6 +142,9 @@ struct AdjParams {
     float4* vr;
     float4* vend;
     float4* vsky;              // [cap] the sky radiance of an escaped path's last ray
+    float4* vskyJ;             // [cap][3] its single-precision Jacobian
+    float4* skyw;              // [cap] weight and path slot of the escapes whose gradient takes that Jacobian
+    int* skyw_count;
     int* esc;                  // [cap] slots of the wave's escaped paths, esc_count of them
     int* esc_count;
     unsigned char* vis;
@@ -237,7 +235,7 @@ __global__ void k_sky_grad(SkyParams P, int n, const float3* dirs, float3* out);
 __global__ void k_adjoint_miss(FrameParams F, AdjParams A);
 __global__ void k_adjoint_rec(FrameParams F, AdjParams A);   // also writes the frozen-path records
 __global__ void k_adjoint_sky_d(FrameParams F, AdjParams A);
-__global__ void k_adjoint_sky_f(FrameParams F, AdjParams A);
+__global__ void k_adjoint_sky_w(AdjParams A);
 __global__ void k_adj_shade(FrameParams F, AdjParams A, int level, long long wave0);
 __global__ void k_adj_shadow(FrameParams F, AdjParams A, int level);
 __global__ void k_adj_sweep(FrameParams F, AdjParams A, long long wave0);

@@ -2443,8 +2443,8 @@ static kpt_status submit_shared(kpt_batch* b, int n, kpt_context* const* jobs, c
             if (extending) k_extend_batch<<<g_ext, TRACE_BLOCK, 0, b->stream>>>(b->m_view, Q, l + 1, b->d_counters.p);
             cudaStreamWaitEvent(b->stream, b->ev_shadow, 0);
             cudaEventRecord(b->ev_level, b->stream);
-            for (int j = 0; j < n; ++j) {   // the jobs whose last level this was
-                if (F[j].max_depth != l) continue;
+            for (int j = 0; j < n; ++j) {   // the jobs whose last level this was (a job with a tail has ended there)
+                if (F[j].max_depth != l || b->h_jobs[j].shaded <= l) continue;
                 cudaStreamWaitEvent(jobs[j]->side, b->ev_shadow, 0);
                 finish(j);
             }

@@ -401,13 +401,13 @@ static kpt_status apply_resolution(kpt_context* c, int w, int h) {
     if (up) KPT_CUDA(c->output.ensure(no));
     // bloom mip chain at the output resolution (mipchain.cuh:17-36): levels below mip 0, at most 6
     int levels = std::min((int)std::log2((double)w), (int)std::log2((double)h));
-    levels = std::min(levels, 6);
+    levels = std::min(levels, BLOOM_LEVELS - 1);
     for (auto& m : c->mips) m.release();
     c->mips.assign(levels + 1, DBuf<float4>());
     c->mip_dims.assign(levels + 1, make_int2(0, 0));
     for (int l = 0; l <= levels; ++l) {
         c->mip_dims[l] = make_int2(w >> l, h >> l);
-        KPT_CUDA(c->mips[l].ensure((size_t)(w >> l) * (h >> l)));
+        if (l > 0) KPT_CUDA(c->mips[l].ensure((size_t)(w >> l) * (h >> l)));   // level 0 is the output
     }
     c->W = rw;
     c->H = rh;
@@ -1326,25 +1326,24 @@ static void enqueue_post(kpt_context* c, const FrameParams& F, float delta_ms) {
         k_rcas<<<og, ob, 0, s>>>(c->easu.p, c->OW, c->OH, c->output.p);
         c->launches += 2;
     }
-    const float4* bloom0 = nullptr;
-    int levels = (int)c->mips.size() - 1;
+    BloomTop bloom{nullptr, 0, 0, c->settings.bloom_internal_blend};
+    const int levels = (int)c->mips.size() - 1;
     if (c->settings.bloom && levels > 0) {
-        dim3 b(16, 16);
+        const dim3 b(16, 16);
+        auto grid = [](int2 d) { return dim3((d.x + 15) / 16, (d.y + 15) / 16); };
+        // level 0 is the output (renderer.cu:446-451); its own blend is the tonemap's
         for (int l = 0; l < levels; ++l) {
             int2 sd = c->mip_dims[l], dd = c->mip_dims[l + 1];
-            const float4* src = l == 0 ? out : c->mips[l].p;
-            k_bloom_down<<<dim3((dd.x + 15) / 16, (dd.y + 15) / 16), b, 0, s>>>(src, sd.x, sd.y, c->mips[l + 1].p, dd.x, dd.y,
-                                                                               c->settings.karis && l == 0);
+            k_bloom_down<<<grid(dd), b, 0, s>>>(l == 0 ? out : c->mips[l].p, sd.x, sd.y, c->mips[l + 1].p, dd.x, dd.y,
+                                                c->settings.karis && l == 0);
         }
-        // mip 0 starts as a copy of the output (renderer.cu:446-451)
-        cudaMemcpyAsync(c->mips[0].p, out, sizeof(float4) * (size_t)c->OW * c->OH, cudaMemcpyDeviceToDevice, s);
-        for (int l = levels; l > 0; --l) {
+        for (int l = levels; l > 1; --l) {
             int2 sd = c->mip_dims[l], dd = c->mip_dims[l - 1];
-            k_bloom_up<<<dim3((dd.x + 15) / 16, (dd.y + 15) / 16), b, 0, s>>>(c->mips[l].p, sd.x, sd.y, c->mips[l - 1].p,
-                                                                             dd.x, dd.y, c->settings.bloom_internal_blend);
+            k_bloom_up<<<grid(dd), b, 0, s>>>(c->mips[l].p, sd.x, sd.y, c->mips[l - 1].p, dd.x, dd.y,
+                                              c->settings.bloom_internal_blend);
         }
-        c->launches += 2 * levels;
-        bloom0 = c->mips[0].p;
+        c->launches += 2 * levels - 1;
+        bloom = {c->mips[1].p, c->mip_dims[1].x, c->mip_dims[1].y, c->settings.bloom_internal_blend};
     }
     double N = c->exposure.aperture;
     double lavg = (10.0 / 0.65) * ((N * N) / ((double)c->exposure.iso * (double)c->exposure.shutter));
@@ -1352,7 +1351,7 @@ static void enqueue_post(kpt_context* c, const FrameParams& F, float delta_ms) {
     const bool fx = c->settings.postprocess_effects != 0;
     if (beside && c->settings.auto_exposure) cudaStreamWaitEvent(s, c->ev_branch[BRANCH_EXPOSURE], 0);
     k_tonemap<<<dim3((c->OW + 15) / 16, (c->OH + 15) / 16), dim3(16, 16), 0, s>>>(
-        c->OW, c->OH, out, bloom0, bloom0 != nullptr, c->settings.bloom_final_blend, c->expo_state.p, fixed_scalar,
+        c->OW, c->OH, out, bloom, c->settings.bloom_final_blend, c->expo_state.p, fixed_scalar,
         c->settings.auto_exposure, c->exposure.white_ev, c->exposure.black_ev, fx ? c->backbuf.p : c->image.p);
     c->launches += 1;
     if (fx) {   // launchFxComputeKernel (renderer.cu:162-167)

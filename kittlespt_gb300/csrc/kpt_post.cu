@@ -300,37 +300,124 @@ __device__ __forceinline__ float4 clamp_out(float4 c) {  // clampOutput on rgb, 
     return make_float4(fmaxf(0.0f, fminf(c.x, 1.0e8f)), fmaxf(0.0f, fminf(c.y, 1.0e8f)), fmaxf(0.0f, fminf(c.z, 1.0e8f)), 1.0f);
 }
 
-// 13 bilinear taps (bloom.cu:17-74); optional Karis average.
-__global__ void k_bloom_down(const float4* src, int sw, int sh_, float4* dst, int dw, int dh, int karis_avg) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= dw || y >= dh) return;
-    float px = __fmul_rn(__fdiv_rn((float)x, (float)dw), (float)sw);
-    float py = __fmul_rn(__fdiv_rn((float)y, (float)dh), (float)sh_);
-    auto T = [&](float ox, float oy) { return bilinear(src, sw, sh_, __fadd_rn(px, ox), __fadd_rn(py, oy)); };
-    float4 a = T(-2, 2), b = T(0, 2), c = T(2, 2), d = T(-2, 0), e = bilinear(src, sw, sh_, px, py), f = T(2, 0);
-    float4 g = T(-2, -2), h = T(0, -2), i = T(2, -2);
-    bool ka = karis_avg != 0;
-    float4 hb1 = box4(a, b, d, e, ka), hb2 = box4(b, c, e, f, ka), hb3 = box4(d, e, g, h, ka), hb4 = box4(e, f, h, i, ka);
-    float4 j = T(-1, 1), k = T(1, 1), l = T(-1, -1), m = T(1, -1);
-    float4 hb5 = box4(j, k, l, m, ka);
-    float4 r = f4lerp(hb5, f4lerp(f4lerp(hb1, hb2, 0.5f), f4lerp(hb3, hb4, 0.5f), 0.5f), 0.5f);
-    dst[(size_t)y * dw + x] = clamp_out(r);
+// Levels of at least this many pixels take a pixel's taps from one block of
+// texels where they form one (1920x1080: level 1 from 0 32 us, now 28; level 1
+// from 2 15.2 and 12.6); below, a warp at an edge runs both ways and the
+// latency counts (level 3 from 2 5.5 us, with blocks 7.5).
+constexpr int BLOOM_BLOCKS = 100000;
+
+// A tap position's texel index and weight per offset -R..R along one axis.
+// Where the indices are consecutive (`regular`: not where adding an offset
+// rounds up to a texel, or at a negative position) the taps' texels form one
+// block, read once instead of four per tap.
+template <int R>
+struct TapAxis {
+    int i;               // of offset 0
+    float w[2 * R + 1];
+    bool regular;
+    __device__ __forceinline__ TapAxis(float p) : i((int)p), regular(true) {
+#pragma unroll
+        for (int o = -R; o <= R; ++o) {
+            const float f = __fadd_rn(p, (float)o);
+            const int k = (int)f;
+            w[o + R] = __fsub_rn(f, (float)k);
+            regular = regular && k == i + o;
+        }
+    }
+    // the block's texels, R before to R + 1 after, inside an axis of n
+    __device__ __forceinline__ bool inside(int n) const { return regular && i >= R && i + R + 1 < n; }
+};
+// 13 bilinear taps around a finer level's position (bloom.cu:17-74); optional
+// Karis average.
+__device__ __forceinline__ float4 down_sample(const float4* src, int sw, int sh, float px, float py, bool ka, bool block) {
+    float4 a, b, c, d, e, f, g, h, i, j, k, l, m;
+    const TapAxis<2> X(px), Y(py);
+    if (block && X.inside(sw) && Y.inside(sh)) {
+        const float4* p = src + (size_t)(Y.i - 2) * sw + (X.i - 2);
+        // a texel row's horizontal steps at offsets -2, 0, 2 (even) and -1, 1 (odd)
+        float4 even[2][3], odd[2][2];
+        auto row = [&](int r) {
+            float4 t[6];
+#pragma unroll
+            for (int q = 0; q < 6; ++q) t[q] = __ldg(p + (size_t)r * sw + q);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) even[r & 1][q] = f4lerp(t[2 * q], t[2 * q + 1], X.w[2 * q]);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) odd[r & 1][q] = f4lerp(t[2 * q + 1], t[2 * q + 2], X.w[2 * q + 1]);
+        };
+        auto at_even = [&](int r, int q) { return f4lerp(even[r & 1][q], even[(r + 1) & 1][q], Y.w[r]); };
+        auto at_odd = [&](int r, int q) { return f4lerp(odd[r & 1][q], odd[(r + 1) & 1][q], Y.w[r]); };
+        row(0), row(1);
+        g = at_even(0, 0), h = at_even(0, 1), i = at_even(0, 2);
+        row(2);
+        l = at_odd(1, 0), m = at_odd(1, 1);
+        row(3);
+        d = at_even(2, 0), e = at_even(2, 1), f = at_even(2, 2);
+        row(4);
+        j = at_odd(3, 0), k = at_odd(3, 1);
+        row(5);
+        a = at_even(4, 0), b = at_even(4, 1), c = at_even(4, 2);
+    } else {
+        auto T = [&](float ox, float oy) { return bilinear(src, sw, sh, __fadd_rn(px, ox), __fadd_rn(py, oy)); };
+        a = T(-2, 2), b = T(0, 2), c = T(2, 2), d = T(-2, 0), e = bilinear(src, sw, sh, px, py), f = T(2, 0);
+        g = T(-2, -2), h = T(0, -2), i = T(2, -2);
+        j = T(-1, 1), k = T(1, 1), l = T(-1, -1), m = T(1, -1);
+    }
+    const float4 hb1 = box4(a, b, d, e, ka), hb2 = box4(b, c, e, f, ka), hb3 = box4(d, e, g, h, ka), hb4 = box4(e, f, h, i, ka);
+    const float4 hb5 = box4(j, k, l, m, ka);
+    return clamp_out(f4lerp(hb5, f4lerp(f4lerp(hb1, hb2, 0.5f), f4lerp(hb3, hb4, 0.5f), 0.5f), 0.5f));
 }
 
-// 3x3 tent of bilinear taps blended into the finer level (bloom.cu:112-146).
-__global__ void k_bloom_up(const float4* src, int sw, int sh_, float4* dst, int dw, int dh, float blend) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= dw || y >= dh) return;
-    float px = __fmul_rn(__fdiv_rn((float)x, (float)dw), (float)sw);
-    float py = __fmul_rn(__fdiv_rn((float)y, (float)dh), (float)sh_);
+// 3x3 tent of bilinear taps at a coarser level's position (bloom.cu:112-146).
+__device__ __forceinline__ float4 tent(const float4* src, int sw, int sh, float px, float py, bool block) {
     const float K[3][3] = {{0.0625f, 0.125f, 0.0625f}, {0.125f, 0.25f, 0.125f}, {0.0625f, 0.125f, 0.0625f}};
     float4 m = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const TapAxis<1> X(px), Y(py);
+    if (block && X.inside(sw) && Y.inside(sh)) {
+        const float4* p = src + (size_t)(Y.i - 1) * sw + (X.i - 1);
+        float4 above[3], row[3];
 #pragma unroll
-    for (int j = -1; j <= 1; ++j)
+        for (int r = 0; r < 4; ++r) {
+            float4 t[4];
 #pragma unroll
-        for (int i = -1; i <= 1; ++i)
-            m = f4add(m, f4mul(bilinear(src, sw, sh_, __fadd_rn(px, (float)i), __fadd_rn(py, (float)j)), K[j + 1][i + 1]));
+            for (int q = 0; q < 4; ++q) t[q] = __ldg(p + (size_t)r * sw + q);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                row[q] = f4lerp(t[q], t[q + 1], X.w[q]);
+                if (r > 0) m = f4add(m, f4mul(f4lerp(above[q], row[q], Y.w[r - 1]), K[r - 1][q]));
+                above[q] = row[q];
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = -1; j <= 1; ++j)
+#pragma unroll
+            for (int i = -1; i <= 1; ++i)
+                m = f4add(m, f4mul(bilinear(src, sw, sh, __fadd_rn(px, (float)i), __fadd_rn(py, (float)j)), K[j + 1][i + 1]));
+    }
+    return m;
+}
+
+// pixel x of a level of n texels on one of m
+__device__ __forceinline__ float mip_position(int x, int n, int m) { return __fmul_rn(__fdiv_rn((float)x, (float)n), (float)m); }
+
+// Issue bound (the taps' arithmetic; with Karis its divisions): 1920x1080 to
+// 960x540 28 us.
+__global__ void __launch_bounds__(256) k_bloom_down(const float4* src, int sw, int sh_, float4* dst, int dw, int dh,
+                                                    int karis_avg) {
+    int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+    if (x >= dw || y >= dh) return;
+    dst[(size_t)y * dw + x] =
+        down_sample(src, sw, sh_, mip_position(x, dw, sw), mip_position(y, dh, sh_), karis_avg != 0,
+                           dw * dh >= BLOOM_BLOCKS);
+}
+
+// The tent blended into the finer level.
+__global__ void __launch_bounds__(256) k_bloom_up(const float4* src, int sw, int sh_, float4* dst, int dw, int dh, float blend) {
+    int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+    if (x >= dw || y >= dh) return;
     size_t o = (size_t)y * dw + x;
+    const float4 m = tent(src, sw, sh_, mip_position(x, dw, sw), mip_position(y, dh, sh_), dw * dh >= BLOOM_BLOCKS);
     dst[o] = clamp_out(f4lerp(dst[o], m, blend));
 }
 
@@ -343,7 +430,7 @@ __device__ __forceinline__ float srgb_enc(float v) {  // color.cuh:421-426
 
 // Y (1 - cx - cy) / cy, the reference's double-precision expression rounded to
 // float.  In double it kept the FP64 pipe, 1/64 of the float rate, at 71%
-// (73 us at 1920x1080, in float 64).  Here as float sums and products with
+// (73 us at 1920x1080 without bloom, in float 64).  Here as float sums and products with
 // their exact rounding errors and a quotient corrected once, within 2^-44 of
 // the exact value; where that does not decide the rounding (about one input in
 // 2^20), or a product's error could leave the float range (a luminance outside
@@ -370,9 +457,12 @@ __device__ __forceinline__ float luminance_z(float Y, float cx, float cy) {
 // computePostProcess (kernels.cu:475-504) with Film / AgX (film.cuh:79-194).
 // The exposure range's logarithms, the same for every pixel, are taken once
 // per block.
-__global__ void k_tonemap(int W, int H, const float4* render, const float4* bloom, int use_bloom, float final_blend,
-                          const ExposureState* st, float fixed_scalar, int auto_exposure, float white_ev, float black_ev,
-                          float4* image) {
+// With bloom, level 0 of its chain too: the tent of level 1 blended into the
+// render, which then has no copy and no pass of its own (1920x1080: copy, blend and tonemap
+// about 125 us, now 91).
+__global__ void __launch_bounds__(256) k_tonemap(int W, int H, const float4* render, BloomTop bloom, float final_blend,
+                                                 const ExposureState* st, float fixed_scalar, int auto_exposure,
+                                                 float white_ev, float black_ev, float4* image) {
     __shared__ float range[2];
     if (threadIdx.y == 0 && threadIdx.x < 2)
         range[threadIdx.x] = log2f(__fmul_rn(exp2f(threadIdx.x ? white_ev : black_ev), 0.18f));
@@ -382,7 +472,11 @@ __global__ void k_tonemap(int W, int H, const float4* render, const float4* bloo
     int sx = (int)__fmul_rn(__fdiv_rn(__fadd_rn((float)x, 0.5f), (float)W), (float)W);
     int sy = (int)__fmul_rn(__fdiv_rn(__fadd_rn((float)y, 0.5f), (float)H), (float)H);
     float4 c = at(render, W, H, sx, sy);
-    if (use_bloom) c = f4lerp(c, at(bloom, W, H, sx, sy), final_blend);
+    if (bloom.mip) {
+        const int bx = min(max(sx, 0), W - 1), by = min(max(sy, 0), H - 1);
+        const float4 m = tent(bloom.mip, bloom.w, bloom.h, mip_position(bx, W, bloom.w), mip_position(by, H, bloom.h), W * H >= BLOOM_BLOCKS);
+        c = f4lerp(c, clamp_out(f4lerp(c, m, bloom.blend)), final_blend);
+    }
     float expo = auto_exposure ? st->exposure_scalar : fixed_scalar;
     // RGB -> XYZ -> Yxy, exposure on Y, back (color.cuh:33-83)
     float X = dot3(0.4124564f, 0.3575761f, 0.1804375f, c.x, c.y, c.z);

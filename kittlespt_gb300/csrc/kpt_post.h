@@ -22,9 +22,15 @@ __global__ void k_histogram(int W, int H, const float4* render, const float* thr
 __global__ void k_exposure(const unsigned long long* hist, ExposureState* st, ExposureIn in);
 __global__ void k_bloom_down(const float4* src, int sw, int sh, float4* dst, int dw, int dh, int karis_avg);
 __global__ void k_bloom_up(const float4* src, int sw, int sh, float4* dst, int dw, int dh, float blend);
-__global__ void k_tonemap(int W, int H, const float4* render, const float4* bloom, int use_bloom, float final_blend,
-                          const ExposureState* st, float fixed_scalar, int auto_exposure, float white_ev, float black_ev,
-                          float4* image);
+constexpr int BLOOM_LEVELS = 7;   // level 0 and at most 6 below (mipchain.cuh:17-36)
+// level 1 of the chain (null: no bloom) and its blend into level 0
+struct BloomTop {
+    const float4* mip;
+    int w, h;
+    float blend;
+};
+__global__ void k_tonemap(int W, int H, const float4* render, BloomTop bloom, float final_blend, const ExposureState* st,
+                          float fixed_scalar, int auto_exposure, float white_ev, float black_ev, float4* image);
 // computeEffects (kernels.cu:506-527): fisheye and chromatic aberration of
 // the tonemapped image
 __global__ void k_effects(int W, int H, const float4* src, float4* dst);

@@ -103,6 +103,7 @@ struct kpt_context {
     DBuf<float4> d_tris;
     DBuf<int> d_tri_leaf;   // per mesh, triangle id -> leaf-order slot (tri_base + id)
     DBuf<TriShade> d_shade;
+    RefitWork refit;
     DBuf<MeshRec> d_meshes;
     DBuf<InstRec> d_inst;
     DBuf<LightRec> d_lights;
@@ -330,7 +331,7 @@ kpt_status kpt_destroy(kpt_context* c) {
     for (auto& f : c->tframes)
         for (cudaEvent_t e : f.ev)
             if (e) cudaEventDestroy(e);
-    c->d_nodes.release(); c->d_tlas.release(); c->d_tris.release(); c->d_tri_leaf.release(); c->d_shade.release();
+    c->d_nodes.release(); c->d_tlas.release(); c->d_tris.release(); c->d_tri_leaf.release(); c->d_shade.release(); c->refit.release();
     c->d_meshes.release(); c->d_inst.release(); c->d_lights.release(); c->d_materials.release();
     c->d_textures.release(); c->d_pixels.release();
     c->acc.release(); c->albedo.release(); c->render.release(); c->image.release(); c->first_hit.release();
@@ -536,7 +537,7 @@ kpt_status kpt_refit_mesh(kpt_context* c, int mesh, const float* positions, cons
     m.pos.assign(positions, positions + n9);
     if (normals) m.nrm.assign(normals, normals + n9);
     const int tb = c->mesh_tri_base[mesh];
-    const int e = refit_blas_device(m, c->d_nodes.p, c->mesh_node_base[mesh], c->d_tris.p, tb, c->d_shade.p, c->stream);
+    const int e = refit_blas_device(m, c->d_nodes.p, c->mesh_node_base[mesh], c->d_tris.p, tb, c->d_shade.p, c->refit, c->stream);
     if (e != 0) return fail(KPT_ERR_CUDA, std::string("kpt_refit_mesh: ") + cudaGetErrorString((cudaError_t)e));
     c->scene_version = ++g_scene_versions;
     // the lights on the mesh's triangles

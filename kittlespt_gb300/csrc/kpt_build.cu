@@ -1159,27 +1159,22 @@ int build_blas_device(HostMesh& m, cudaStream_t st) {
 
 namespace {
 
-__global__ void k_refit_tris(const float* pos, const int* order, int n, int tri_base, float4* tris) {
+// One thread per triangle in leaf order: its record (whose id the record
+// already holds) and the geometric normal of tri_normal_area (kpt_scene.cpp),
+// the same IEEE operations: facing the mean vertex normal (Triangle
+// constructor, triangle.cuh:51-64).
+__global__ void k_refit_tris(const float* pos, const float* nrm, int n, float4* tris, TriShade* shade) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const int t = order[k];
-    const float* p = pos + 9 * (size_t)t;
-    float4* o = tris + 3 * ((size_t)tri_base + k);
-    o[0] = make_float4(p[0], p[1], p[2], __int_as_float(t));
-    o[1] = make_float4(__fsub_rn(p[3], p[0]), __fsub_rn(p[4], p[1]), __fsub_rn(p[5], p[2]), o[1].w);
-    o[2] = make_float4(__fsub_rn(p[6], p[0]), __fsub_rn(p[7], p[1]), __fsub_rn(p[8], p[2]), 0.0f);
-}
-
-// tri_normal_area (kpt_scene.cpp) on the device, the same IEEE operations:
-// the geometric normal facing the mean vertex normal (Triangle constructor,
-// triangle.cuh:51-64)
-__global__ void k_refit_shade(const float* pos, const float* nrm, int n, TriShade* shade) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
+    float4* o = tris + 3 * (size_t)k;
+    const int t = __float_as_int(o[0].w);
     const float* p = pos + 9 * (size_t)t;
     const float* q = nrm + 9 * (size_t)t;
     const float e0x = __fsub_rn(p[3], p[0]), e0y = __fsub_rn(p[4], p[1]), e0z = __fsub_rn(p[5], p[2]);
     const float e1x = __fsub_rn(p[6], p[0]), e1y = __fsub_rn(p[7], p[1]), e1z = __fsub_rn(p[8], p[2]);
+    o[0] = make_float4(p[0], p[1], p[2], o[0].w);
+    o[1] = make_float4(e0x, e0y, e0z, o[1].w);
+    o[2] = make_float4(e1x, e1y, e1z, 0.0f);
     const float gx = __fsub_rn(__fmul_rn(e0y, e1z), __fmul_rn(e0z, e1y));
     const float gy = __fsub_rn(__fmul_rn(e0z, e1x), __fmul_rn(e0x, e1z));
     const float gz = __fsub_rn(__fmul_rn(e0x, e1y), __fmul_rn(e0y, e1x));
@@ -1194,21 +1189,38 @@ __global__ void k_refit_shade(const float* pos, const float* nrm, int n, TriShad
     shade[t].gnz = __fmul_rn(oz, inv);
 }
 
-__device__ __forceinline__ void leaf_box(const float* pos, const int* order, int tri_base, int first, int count,
-                                         float* lo, float* hi) {
-    for (int q = 0; q < 3; ++q) {
-        lo[q] = FLT_MAX;
-        hi[q] = -FLT_MAX;
+// Parents (local), interior children to wait for, and the leaf children's
+// boxes: 8 lanes per child, a triangle each (a thread per node, one triangle
+// after the other, 19 us for 20,480 triangles: two dependent loads each).
+__global__ void k_refit_leaves(BvhNode* nodes, int node_base, int nn, const float* pos, const float4* tris, int* parent,
+                               int* need, int* arrive) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x, v = g >> 4, slot = g >> 3 & 1, lane = g & 7;
+    if (v >= nn) return;   // 16 lanes a node: whole groups
+    BvhNode& n = nodes[node_base + v];
+    const int4 d = n.d;
+    const int ref = slot ? d.z : d.x, cnt = slot ? d.w : d.y;
+    if (lane == 0 && cnt == 0) parent[ref - node_base] = v;
+    if (lane == 0 && slot == 0) {
+        need[v] = (d.y == 0) + (d.w == 0);
+        arrive[v] = 0;
+        if (v == 0) parent[0] = -1;
     }
-    for (int k = first; k < first + count; ++k) {
-        const float* v = pos + 9 * (size_t)order[k - tri_base];
+    if (cnt == 0) return;
+    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    for (int k = ref + lane; k < ref + cnt; k += 8) {
+        const float* p = pos + 9 * (size_t)__float_as_int(tris[3 * (size_t)k].w);
         for (int j = 0; j < 9; ++j) {
-            lo[j % 3] = fminf(lo[j % 3], v[j]);
-            hi[j % 3] = fmaxf(hi[j % 3], v[j]);
+            lo[j % 3] = fminf(lo[j % 3], p[j]);
+            hi[j % 3] = fmaxf(hi[j % 3], p[j]);
         }
     }
-}
-__device__ __forceinline__ void set_child(BvhNode& n, int slot, const float* lo, const float* hi) {
+    const unsigned group = 0xffu << (threadIdx.x & 24);
+    for (int q = 0; q < 3; ++q)
+        for (int o = 4; o > 0; o >>= 1) {
+            lo[q] = fminf(lo[q], __shfl_xor_sync(group, lo[q], o));
+            hi[q] = fmaxf(hi[q], __shfl_xor_sync(group, hi[q], o));
+        }
+    if (lane != 0) return;
     if (slot == 0) {
         n.a = make_float4(lo[0], lo[1], lo[2], hi[0]);
         n.b.x = hi[1];
@@ -1218,30 +1230,6 @@ __device__ __forceinline__ void set_child(BvhNode& n, int slot, const float* lo,
         n.b.w = lo[1];
         n.c = make_float4(lo[2], hi[0], hi[1], hi[2]);
     }
-}
-
-// parents (local), interior children to wait for, and the leaf children's boxes
-__global__ void k_refit_leaves(BvhNode* nodes, int node_base, int nn, int tri_base, const float* pos,
-                               const int* order, int* parent, int* need, int* arrive) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nn) return;
-    BvhNode n = nodes[node_base + v];
-    int nd = 0;
-    for (int slot = 0; slot < 2; ++slot) {
-        const int ref = slot ? n.d.z : n.d.x, cnt = slot ? n.d.w : n.d.y;
-        if (cnt == 0) {
-            parent[ref - node_base] = v;
-            ++nd;
-        } else {
-            float lo[3], hi[3];
-            leaf_box(pos, order, tri_base, ref, cnt, lo, hi);
-            set_child(n, slot, lo, hi);
-        }
-    }
-    nodes[node_base + v] = n;
-    need[v] = nd;
-    arrive[v] = 0;
-    if (v == 0) parent[0] = -1;
 }
 
 // a node whose children's boxes are final passes their union to its parent;
@@ -1277,28 +1265,51 @@ __global__ void k_refit_up(BvhNode* nodes, int node_base, int nn, const int* par
 
 }  // namespace
 
+void RefitWork::release() {
+    cudaFree(pos);
+    cudaFree(links);
+    *this = RefitWork{};
+}
+
+// Room for ntris triangles' positions and normals and nn nodes' links, kept
+// for the next call.
+static cudaError_t refit_room(RefitWork& w, size_t ntris, size_t nn) {
+    if (ntris > w.ntris) {
+        cudaFree(w.pos);
+        w.pos = nullptr;
+        w.ntris = 0;
+        const cudaError_t e = cudaMalloc(&w.pos, 18 * ntris * sizeof(float));
+        if (e != cudaSuccess) return e;
+        w.ntris = ntris;
+    }
+    if (nn > w.nn) {
+        cudaFree(w.links);
+        w.links = nullptr;
+        w.nn = 0;
+        const cudaError_t e = cudaMalloc(&w.links, 3 * nn * sizeof(int));
+        if (e != cudaSuccess) return e;
+        w.nn = nn;
+    }
+    return cudaSuccess;
+}
+
+// Small blocks: the nodes and triangles of one mesh are few for the GPU, and
+// their gathers bound by latency (20,480 triangles: 85 us of kernels before the launches below, 37 now).
 int refit_blas_device(HostMesh& m, BvhNode* d_nodes, int node_base, float4* d_tris, int tri_base, TriShade* d_shade,
-                      cudaStream_t st) {
+                      RefitWork& w, cudaStream_t st) {
+    constexpr int BLOCK = 64;
     const int N = m.ntris(), nn = (int)m.nodes.size();
-    DevArray<float> pos, nrm;
-    DevArray<int> order, parent, need, arrive;
-    cudaError_t e = cudaSuccess;
-    for (cudaError_t r : {pos.alloc(9 * (size_t)N), nrm.alloc(9 * (size_t)N), order.alloc(N), parent.alloc(nn),
-                          need.alloc(nn), arrive.alloc(nn)})
-        if (r != cudaSuccess && e == cudaSuccess) e = r;
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(pos.p, m.pos.data(), 9 * (size_t)N * sizeof(float), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(nrm.p, m.nrm.data(), 9 * (size_t)N * sizeof(float), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(order.p, m.order.data(), (size_t)N * sizeof(int), cudaMemcpyHostToDevice, st);
+    cudaError_t e = refit_room(w, (size_t)N, (size_t)nn);
     if (e != cudaSuccess) return (int)e;
-    k_refit_tris<<<(N + 255) / 256, 256, 0, st>>>(pos.p, order.p, N, tri_base, d_tris);
-    k_refit_shade<<<(N + 255) / 256, 256, 0, st>>>(pos.p, nrm.p, N, d_shade + tri_base);
+    float *pos = w.pos, *nrm = w.pos + 9 * (size_t)N;
+    int *parent = w.links, *need = w.links + nn, *arrive = w.links + 2 * (size_t)nn;
+    e = cudaMemcpyAsync(pos, m.pos.data(), 9 * (size_t)N * sizeof(float), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(nrm, m.nrm.data(), 9 * (size_t)N * sizeof(float), cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return (int)e;
+    k_refit_tris<<<(N + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(pos, nrm, N, d_tris + 3 * (size_t)tri_base, d_shade + tri_base);
     if (nn > 0) {
-        k_refit_leaves<<<(nn + 255) / 256, 256, 0, st>>>(d_nodes, node_base, nn, tri_base, pos.p, order.p, parent.p,
-                                                         need.p, arrive.p);
-        k_refit_up<<<(nn + 255) / 256, 256, 0, st>>>(d_nodes, node_base, nn, parent.p, need.p, arrive.p);
+        k_refit_leaves<<<(nn - 1) / (BLOCK / 16) + 1, BLOCK, 0, st>>>(d_nodes, node_base, nn, pos, d_tris, parent, need, arrive);
+        k_refit_up<<<(nn + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(d_nodes, node_base, nn, parent, need, arrive);
         // the host copy of the nodes: boxes from the device, references local as built
         std::vector<BvhNode> h(nn);
         e = cudaMemcpyAsync(h.data(), d_nodes + node_base, nn * sizeof(BvhNode), cudaMemcpyDeviceToHost, st);

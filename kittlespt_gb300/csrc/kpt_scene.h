@@ -49,12 +49,20 @@ void pack_blas(HostMesh& m, const std::vector<BlasNode>& nodes, std::vector<int>
 // triangle order.  Returns a CUDA error code (0 on success).
 int build_blas_device(HostMesh& m, cudaStream_t stream);
 
+// Device memory of refits, a context's own, kept from one to the next.
+struct RefitWork {
+    float* pos = nullptr;   // positions, then normals, 9 floats a triangle each
+    int* links = nullptr;   // per node: parent, interior children, those that have arrived
+    size_t ntris = 0, nn = 0;
+    void release();
+};
+
 // Refit on the GPU after m.pos (and m.nrm) changed, same tree: recomputes
 // the child boxes of the mesh's nodes at node_base of the scene's device
 // node array bottom up, rewrites its triangle records and the geometric
 // normals of its shading records at tri_base, and updates m.nodes' boxes
 // and m.lo / m.hi.  Returns a CUDA error code (0 on success).
-int refit_blas_device(HostMesh& m, BvhNode* d_nodes, int node_base, float4* d_tris, int tri_base, TriShade* d_shade,
+int refit_blas_device(HostMesh& m, BvhNode* d_nodes, int node_base, float4* d_tris, int tri_base, TriShade* d_shade, RefitWork& work,
                       cudaStream_t stream);
 
 // World bounds of an instance: the 8 transformed corners of the mesh bounds

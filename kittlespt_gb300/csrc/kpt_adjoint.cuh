@@ -589,14 +589,13 @@ struct GradStep {
     float2 s, ds, p, dp;
 };
 template <int LANES>
-__device__ __forceinline__ GradStep step_of(unsigned mask, const GradStep& G, int lane) {
+__device__ __forceinline__ GradStep step_of(const GradStep& G, int lane) {
     GradStep R;
-    R.T = make_float3(__shfl_sync(mask, G.T.x, lane, LANES), __shfl_sync(mask, G.T.y, lane, LANES),
-                      __shfl_sync(mask, G.T.z, lane, LANES));
-    R.s = shfl_pair<LANES>(mask, G.s, lane);
-    R.ds = shfl_pair<LANES>(mask, G.ds, lane);
-    R.p = shfl_pair<LANES>(mask, G.p, lane);
-    R.dp = shfl_pair<LANES>(mask, G.dp, lane);
+    R.T = make_float3(of_lane<LANES>(G.T.x, lane), of_lane<LANES>(G.T.y, lane), of_lane<LANES>(G.T.z, lane));
+    R.s = of_lane<LANES>(G.s, lane);
+    R.ds = of_lane<LANES>(G.ds, lane);
+    R.p = of_lane<LANES>(G.p, lane);
+    R.dp = of_lane<LANES>(G.dp, lane);
     return R;
 }
 
@@ -628,9 +627,11 @@ template <int LANES = 1>
 static __device__ __noinline__ float3 nishita_grad(const SkyParams& P, float3 o, float3 d, float3* J) {
     for (int i = 0; i < SKY_PARAMS; ++i) J[i] = make_float3(0.0f, 0.0f, 0.0f);
     float tmin = 0.0f, tmax = __int_as_float(0x7f800000);
+    bool seen;
     {
-        float te, tx;
-        if (!sphere_hit(o, d, P.atm_r, &te, &tx) || tx < 0.0f) return make_float3(0.0f, 0.0f, 0.0f);
+        float te = 0.0f, tx = 0.0f;
+        seen = sphere_hit(o, d, P.atm_r, &te, &tx) && !(tx < 0.0f);
+        if (LANES == 1 && !seen) return make_float3(0.0f, 0.0f, 0.0f);
         if (te > tmin && te > 0.0f) tmin = te;
         if (tx < tmax) tmax = tx;
     }
@@ -641,7 +642,6 @@ static __device__ __noinline__ float3 nishita_grad(const SkyParams& P, float3 o,
     const float half = xm(step, 0.5f);
     const float2 ih2 = make_float2(1.0f / (P.h_r * P.h_r), 1.0f / (P.h_m * P.h_m));
     const int lane = threadIdx.x & (LANES - 1);
-    const unsigned mask = ((1u << (LANES & 31)) - 1u) << (threadIdx.x & 31 & ~(LANES - 1));
     float t = tmin;
 #pragma unroll
     for (int q = 0; q < LANES - 1; ++q) t = q < lane ? xa(t, step) : t;
@@ -661,7 +661,7 @@ static __device__ __noinline__ float3 nishita_grad(const SkyParams& P, float3 o,
         } else {   // the sums up to this lane's step, carried on from the last lane's
 #pragma unroll
             for (int q = 0; q < LANES; ++q) {
-                const float2 p = shfl_pair<LANES>(mask, G.p, q), dp = shfl_pair<LANES>(mask, G.dp, q);
+                const float2 p = of_lane<LANES>(G.p, q), dp = of_lane<LANES>(G.dp, q);
                 if (q <= lane) {
                     opt = A.sum(opt, p);
                     dopt = A.sum(dopt, dp);
@@ -699,14 +699,14 @@ static __device__ __noinline__ float3 nishita_grad(const SkyParams& P, float3 o,
             if (lit) S.add(A, tR, tM, G);
             t = xa(t, step);
         } else {
-            const unsigned all = __ballot_sync(mask, lit) >> (threadIdx.x & 31 & ~(LANES - 1));
+            const unsigned all = __ballot_sync(0xffffffffu, lit) >> (threadIdx.x & 31 & ~(LANES - 1));
 #pragma unroll 1
             for (int q = 0; q < LANES; ++q) {
-                const GradStep Q = step_of<LANES>(mask, G, q);
+                const GradStep Q = step_of<LANES>(G, q);
                 if (all >> q & 1) S.add(A, tR, tM, Q);
             }
-            opt = shfl_pair<LANES>(mask, opt, LANES - 1);
-            dopt = shfl_pair<LANES>(mask, dopt, LANES - 1);
+            opt = of_lane<LANES>(opt, LANES - 1);
+            dopt = of_lane<LANES>(dopt, LANES - 1);
 #pragma unroll
             for (int q = 0; q < LANES; ++q) t = xa(t, step);
         }
@@ -717,6 +717,7 @@ static __device__ __noinline__ float3 nishita_grad(const SkyParams& P, float3 o,
         diR[k] = make_float3(S.din[k][0].x, S.din[k][1].x, S.din[k][2].x);
         diM[k] = make_float3(S.din[k][0].y, S.din[k][1].y, S.din[k][2].y);
     }
+    if (LANES > 1 && !seen) return make_float3(0.0f, 0.0f, 0.0f);
     float mu = dot(d, P.sun_dir);
     float rp = (3.0f * (1.0f + Sqr(mu))) / (16.0f * PI_F);
     const float g = 0.76f;

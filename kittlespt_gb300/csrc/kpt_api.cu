@@ -104,6 +104,7 @@ struct kpt_context {
     DBuf<int> d_tri_leaf;   // per mesh, triangle id -> leaf-order slot (tri_base + id)
     DBuf<TriShade> d_shade;
     RefitWork refit;
+    long long sky_threads = 0;   // of k_sky that the GPU holds at once
     DBuf<MeshRec> d_meshes;
     DBuf<InstRec> d_inst;
     DBuf<LightRec> d_lights;
@@ -1750,8 +1751,14 @@ kpt_status kpt_sky_device(kpt_context* c, int n, const float* dirs, float* rgb) 
     if (!c || n < 0 || (n > 0 && (!dirs || !rgb))) return fail(KPT_ERR_INVALID, "kpt_sky_device: bad arguments");
     KPT_CUDA(cudaSetDevice(c->device));
     if (n == 0) return KPT_OK;
-    // several lanes per direction where the GPU has the threads for them
-    const long long threads = (long long)persistent_grid(c, (const void*)k_sky, SKY_BLOCK) * SKY_BLOCK;
+    // several lanes per direction where the GPU has the threads for them (their number asked once: a
+    // call for few directions takes 7 us, the question 0.4)
+    if (c->sky_threads == 0) {
+        int per_sm = 0;
+        KPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sky, SKY_BLOCK, 0));
+        c->sky_threads = (long long)std::max(1, per_sm) * c->sm_count * SKY_BLOCK;
+    }
+    const long long threads = c->sky_threads;
     const int lanes = 8LL * n <= threads ? 8 : 2LL * n <= threads ? 2 : 1;
     const int per_block = SKY_BLOCK / lanes;
     k_sky<<<(n - 1) / per_block + 1, SKY_BLOCK, 0, c->stream>>>(frame_sky(c), n, lanes, (const float3*)dirs, (float3*)rgb);

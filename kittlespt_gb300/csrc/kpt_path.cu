@@ -1242,7 +1242,7 @@ __global__ void k_sun_constants_gpu(float phi, float theta, float diameter, floa
 
 // Nishita radiance towards the sun: a per-frame constant.
 __global__ void k_sky_constants(FrameParams F, float3* sun_radiance) {
-    if (threadIdx.x >= 8 || blockIdx.x != 0) return;
+    if (blockIdx.x != 0) return;   // one warp
     const SkyParams& P = F.sky;
     const float3 L = nishita<8>(P, make_float3(0.0f, P.earth_r + 1.0f, 0.0f), P.sun_dir);
     if (threadIdx.x == 0) *sun_radiance = L;

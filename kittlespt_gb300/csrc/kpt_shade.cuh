@@ -469,14 +469,20 @@ __device__ __forceinline__ SkyStep sky_step(const Arith& A, const SkyParams& P, 
     return S;
 }
 
+// `lane` of the group of LANES; every lane of the warp takes part (with a mask
+// of the group alone, groups that a branch parted run one after another)
 template <int LANES>
-__device__ __forceinline__ float2 shfl_pair(unsigned mask, float2 v, int lane) {
-    return make_float2(__shfl_sync(mask, v.x, lane, LANES), __shfl_sync(mask, v.y, lane, LANES));
+__device__ __forceinline__ float of_lane(float v, int lane) {
+    return __shfl_sync(0xffffffffu, v, lane, LANES);
+}
+template <int LANES>
+__device__ __forceinline__ float2 of_lane(float2 v, int lane) {
+    return make_float2(of_lane<LANES>(v.x, lane), of_lane<LANES>(v.y, lane));
 }
 
 // Radiance of the sky seen from `o` along `d`.  A direction's 16 view steps of
 // 8 light samples are one long chain for a thread; LANES neighbouring lanes
-// (with the same o and d) take LANES view steps at a time and add them in the
+// (with the same o and d, the whole warp in step) take LANES view steps at a time and add them in the
 // march's order, so the result does not depend on LANES.
 // Bound by the FP32 and MUFU pipes where directions are many (k_adj_sky: 70%
 // of issue slots, the pipes' throttle its largest stall), by the chain's
@@ -487,9 +493,11 @@ __device__ __forceinline__ float2 shfl_pair(unsigned mask, float2 v, int lane) {
 template <class Arith, int LANES>
 static __device__ __noinline__ float3 nishita_march(const SkyParams& P, float3 o, float3 d) {
     float tmin = 0.0f, tmax = __int_as_float(0x7f800000);
+    bool seen;
     {
-        float te, tx;
-        if (!Arith::hit(o, d, P.atm_r, &te, &tx) || tx < 0.0f) return make_float3(0.0f, 0.0f, 0.0f);
+        float te = 0.0f, tx = 0.0f;
+        seen = Arith::hit(o, d, P.atm_r, &te, &tx) && !(tx < 0.0f);
+        if (LANES == 1 && !seen) return make_float3(0.0f, 0.0f, 0.0f);
         if (te > tmin && te > 0.0f) tmin = te;
         if (tx < tmax) tmax = tx;
     }
@@ -498,7 +506,6 @@ static __device__ __noinline__ float3 nishita_march(const SkyParams& P, float3 o
     const float3 tR = make_float3(xa(P.sigma_r.x, 0.0f), xa(P.sigma_r.y, 0.0f), xa(P.sigma_r.z, 0.0f));
     const float tM = xa(P.sigma_m, P.sigma_am);
     const int lane = threadIdx.x & (LANES - 1);
-    const unsigned mask = LANES == 32 ? ~0u : ((1u << (LANES & 31)) - 1u) << (threadIdx.x & 31 & ~(LANES - 1));
     float t = tmin;
 #pragma unroll
     for (int q = 0; q < LANES - 1; ++q) t = q < lane ? xa(t, step) : t;
@@ -512,7 +519,7 @@ static __device__ __noinline__ float3 nishita_march(const SkyParams& P, float3 o
         } else {   // the sum up to this lane's step, carried on from the last lane's
 #pragma unroll
             for (int q = 0; q < LANES; ++q) {
-                const float2 p = shfl_pair<LANES>(mask, S.p, q);
+                const float2 p = of_lane<LANES>(S.p, q);
                 if (q <= lane) opt = A.sum(opt, p);
             }
         }
@@ -526,19 +533,18 @@ static __device__ __noinline__ float3 nishita_march(const SkyParams& P, float3 o
             }
             t = xa(t, step);
         } else {
-            const unsigned lit = __ballot_sync(mask, S.lit) >> (threadIdx.x & 31 & ~(LANES - 1));
+            const unsigned lit = __ballot_sync(0xffffffffu, S.lit) >> (threadIdx.x & 31 & ~(LANES - 1));
 #pragma unroll
             for (int q = 0; q < LANES; ++q) {
-                const float2 p = shfl_pair<LANES>(mask, S.p, q);
-                const float x = __shfl_sync(mask, Tr.x, q, LANES), y = __shfl_sync(mask, Tr.y, q, LANES),
-                            z = __shfl_sync(mask, Tr.z, q, LANES);
+                const float2 p = of_lane<LANES>(S.p, q);
+                const float x = of_lane<LANES>(Tr.x, q), y = of_lane<LANES>(Tr.y, q), z = of_lane<LANES>(Tr.z, q);
                 if (lit >> q & 1) {
                     iX = A.add(iX, both(x), p);
                     iY = A.add(iY, both(y), p);
                     iZ = A.add(iZ, both(z), p);
                 }
             }
-            opt = shfl_pair<LANES>(mask, opt, LANES - 1);
+            opt = of_lane<LANES>(opt, LANES - 1);
 #pragma unroll
             for (int q = 0; q < LANES; ++q) t = xa(t, step);
         }
@@ -550,7 +556,8 @@ static __device__ __noinline__ float3 nishita_march(const SkyParams& P, float3 o
     float den = (8.0f * PI_F) * ((2.0f + Sqr(g)) * powf(1.0f + Sqr(g) - 2.0f * g * mu, 1.5f));
     float mp = 3.0f * ((1.0f - Sqr(g)) * (1.0f + Sqr(mu))) / den;
     float3 L = P.sigma_r * iR * rp + make_float3(P.sigma_m, P.sigma_m, P.sigma_m) * iM * mp;
-    return L * 6.0e5f * P.sun_emission;
+    L = L * 6.0e5f * P.sun_emission;
+    return LANES == 1 || seen ? L : make_float3(0.0f, 0.0f, 0.0f);
 }
 
 // The sky in the arithmetic the frame selects (P.gpu_arith).
@@ -566,12 +573,19 @@ __device__ __forceinline__ int sky_lanes(int n, int threads) {
     return 8LL * n <= threads ? 8 : 2LL * n <= threads ? 2 : 1;
 }
 
-// use(i, lane 0 of its group) for every i in [i0, n), spread over the grid with
-// LANES lanes each.
+// use(i, whether it is the lane that stores) for every i in [i0, n), spread over
+// the grid with LANES lanes each.  With several, whole warps: the groups past
+// the end repeat the last.
 template <int LANES, class Use>
 __device__ __forceinline__ void sky_spread(int i0, int n, Use use) {
-    const int first = (blockIdx.x * blockDim.x + threadIdx.x) / LANES, all = gridDim.x * blockDim.x / LANES;
-    for (int i = i0 + first; i < n; i += all) use(i, (threadIdx.x & (LANES - 1)) == 0);
+    const int thread = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x / LANES;
+    if (LANES == 1) {
+        for (int i = i0 + thread; i < n; i += all) use(i, true);
+    } else {
+        const int group = (threadIdx.x & 31) / LANES;
+        for (int i = i0 + (thread & ~31) / LANES; i < n; i += all)   // the warp's first
+            use(min(i + group, n - 1), i + group < n && (threadIdx.x & (LANES - 1)) == 0);
+    }
 }
 
 }  // namespace kpt

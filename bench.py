@@ -55,12 +55,12 @@ WORKLOAD = "icosphere_grid_1080p_16spp_depth8"
 # warp instruction / 32), issue-active fraction, cache hit rates, DRAM
 # throughput against its peak, the top stall.
 NCU_RAY_KERNELS = {
-    "extend": {"simt_efficiency": 11.68 / 32, "issue_active": 0.693, "l1_hit": 0.686, "l2_hit": 0.825,
-               "dram_throughput_of_peak": 0.0154, "alu_pipe_active": 0.534,
-               "top_stall": "long scoreboard, 3.67 cycles per issue"},
-    "shadow": {"simt_efficiency": 11.44 / 32, "issue_active": 0.710, "l1_hit": 0.674, "l2_hit": 0.817,
-               "dram_throughput_of_peak": 0.0125, "alu_pipe_active": 0.528,
-               "top_stall": "long scoreboard"},
+    "extend": {"simt_efficiency": 21.06 / 32, "issue_active": 0.724, "l1_hit": 0.493, "l2_hit": 0.892,
+               "dram_throughput_of_peak": 0.0252, "alu_pipe_active": 0.545,
+               "top_stall": "long scoreboard, 3.55 cycles per issue"},
+    "shadow": {"simt_efficiency": 20.73 / 32, "issue_active": 0.713, "l1_hit": 0.480, "l2_hit": 0.885,
+               "dram_throughput_of_peak": 0.0238, "alu_pipe_active": 0.536,
+               "top_stall": "long scoreboard, 3.99 cycles per issue"},
 }
 
 
@@ -344,8 +344,8 @@ def run_gpu(args):
     kern = {"extend": ("k_extend", "path"), "shadow": ("k_shadow", "shadow")}
     # DRAM bytes per frame of each ray kernel from one ncu capture of the
     # 960x540x8 case (profiles/wave_kernels_960x540x8.md), scaled by samples
-    # (x8) to this workload
-    traffic = {"extend": (249.1e6 + 20.1e6) * 8.0, "shadow": (128.8e6 + 0.9e6) * 8.0}
+    # (x8) to this workload (there levels 1-6 and 0-5: later ones are the tail's)
+    traffic = {"extend": (220.1e6 + 17.5e6) * 8.0, "shadow": (119.4e6 + 0.2e6) * 8.0}
     dom = max(kern, key=lambda k: stage_ms[k])
     kname, pre = kern[dom]
     rays_frame = delta("camera_rays") + delta("path_rays") + delta("shadow_rays")
@@ -410,10 +410,10 @@ def run_gpu(args):
                                               "960x540x8 capture scaled x8 by samples "
                                               "(profiles/wave_kernels_960x540x8.md)",
                             "peak_kind": peak_kind,
-                            "why": "latency and issue bound: DRAM at ~1.5% of its peak, the algorithmic "
-                                   "bytes served 69% by L1 and 83% of the rest by L2; issue slots at 69% "
-                                   "with 11.7 of 32 lanes active per instruction; long-scoreboard stalls "
-                                   "on dependent node and triangle fetches",
+                            "why": "latency and issue bound: DRAM at ~2.5% of its peak, the algorithmic "
+                                   "bytes served 49% by L1 and 89% of the rest by L2; issue slots at 72% "
+                                   "with 21.1 of 32 lanes active per instruction; L1 at 78% of its "
+                                   "throughput; long-scoreboard stalls on dependent node and triangle fetches",
                             "ncu": NCU_RAY_KERNELS[dom],
                             "algorithmic_bytes_per_frame": alg_bytes, "kernel_ms_per_frame": launch_ms,
                             "launches_per_frame": DEPTH + (1 if dom == "shadow" else 0),

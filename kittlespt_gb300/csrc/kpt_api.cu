@@ -1752,7 +1752,7 @@ kpt_status kpt_sky_device(kpt_context* c, int n, const float* dirs, float* rgb) 
     KPT_CUDA(cudaSetDevice(c->device));
     if (n == 0) return KPT_OK;
     // several lanes per direction where the GPU has the threads for them (their number asked once: a
-    // call for few directions takes 7 us, the question 0.4)
+    // call for few directions takes 4 us, the question 0.4)
     if (c->sky_threads == 0) {
         int per_sm = 0;
         KPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sky, SKY_BLOCK, 0));

@@ -332,13 +332,13 @@ __device__ __forceinline__ bool trace_any(const SceneView& s, const XRay& r, flo
 //     the rays read from shared memory; the group's closest hit goes back to
 //     the lane that owns the ray;
 //   * instances: lanes entering or leaving one change the ray's space.
-// What bounds it: instruction issue (73% of cycles at 21 of 32 lanes active
-// per instruction) and the L1 data pipe (66%: 64-byte nodes and 48-byte
+// What bounds it: instruction issue (72% of cycles at 21 of 32 lanes active
+// per instruction) and the L1 data pipe (78%: 64-byte nodes and 48-byte
 // triangles at unrelated addresses).  One step of any kind per loop iteration
 // with leaves tested by their own lane, as before, ran 11.7 lanes per
 // instruction: the extension rays of the 1920x1080x16 frame (depth 8) took
-// 11.15 ms and its shadow rays 5.86 ms, now 6.33 and 2.95; 1M bounce chains
-// in 2M triangles 2.29 ms, now 1.39.  Measured on the way (the same frame's
+// 11.15 ms and its shadow rays 5.86 ms, now 6.41 and 2.82; 1M bounce chains
+// in 2M triangles 2.29 ms, now 1.25.  Measured on the way (the same frame's
 // extension rays): nodes and leaves in loops of their own 8.99, each left
 // early 7.94, node records in two 32-byte loads 7.61, the stack's first 16
 // entries in shared memory 7.44 (conflict-free; a divergent local pop spreads

@@ -566,6 +566,28 @@ __global__ void __launch_bounds__(PATH_BLOCK) k_adjoint_rec(FrameParams F, AdjPa
 
 __device__ __forceinline__ float3 xyz3(float4 v) { return make_float3(v.x, v.y, v.z); }
 
+// a sector of a vertex record (32-byte aligned)
+struct Sector {
+    float3 a, b;
+    float c, d;
+};
+__device__ __forceinline__ void store8(float* p, float3 a, float3 b, float c, float d) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z), "f"(b.x),
+                 "f"(b.y), "f"(b.z), "f"(c), "f"(d)
+                 : "memory");
+}
+__device__ __forceinline__ Sector load8(const float* p) {
+    Sector s;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(s.a.x), "=f"(s.a.y), "=f"(s.a.z), "=f"(s.b.x), "=f"(s.b.y), "=f"(s.b.z), "=f"(s.c), "=f"(s.d)
+                 : "l"(p)
+                 : "memory");
+    return s;
+}
+
+// Bound by latency (20 warps per SM) and, from level 1 on, by instruction
+// fetch.  Level 0 of 512x512x32 samples 431 us; with records of nine 16-byte
+// fields 570, half of whose sectors were written twice.
 // (held to 96 registers: at 80 the same gradient takes 6.61 ms, not 6.52; at 128, 6.56)
 __global__ void __launch_bounds__(PATH_BLOCK, 5) k_adj_shade(FrameParams F, AdjParams A, int level, long long wave0) {
     constexpr int MV = ADJ_MAX_VERTICES;
@@ -588,7 +610,7 @@ __global__ void __launch_bounds__(PATH_BLOCK, 5) k_adj_shade(FrameParams F, AdjP
     int* here = F.level_counts + LEVEL_WORDS * level;
     int* next = F.level_counts + LEVEL_WORDS * (level + 1);
     if (first && blockIdx.x == 0 && threadIdx.x == 0) here[0] = n;   // read back by kpt_get_level_counts
-    float4* const vr0 = A.vr + (size_t)level * cap * AV_FIELDS;
+    float* const vr0 = A.vr + (size_t)level * cap * AV_FLOATS;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float3 o, d, beta, prev;
         float p_b;
@@ -753,19 +775,16 @@ __global__ void __launch_bounds__(PATH_BLOCK, 5) k_adj_shade(FrameParams F, AdjP
                 int j;
                 if (nee == 1) j = group_append(here + 1);
                 else j = cap - 1 - group_append(here + 2);
-                ShadowRec r;
-                r.o_tmax = make_float4(so.x, so.y, so.z, tmax);
-                r.d_item = make_float4(sd.x, sd.y, sd.z, __int_as_float(loc));
-                r.contrib = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                F.shadow[j] = r;
+                F.shadow[j].o_tmax = make_float4(so.x, so.y, so.z, tmax);
+                F.shadow[j].d_item = make_float4(sd.x, sd.y, sd.z, __int_as_float(loc));
             }
         }
-        vr0[(size_t)loc * AV_FIELDS + AV_BETA] = make_float4(beta.x, beta.y, beta.z, __int_as_float(si.material));
-        vr0[(size_t)loc * AV_FIELDS + AV_EMIT] = make_float4(c.x, c.y, c.z, __int_as_float(nee));
-        vr0[(size_t)loc * AV_FIELDS + AV_FCOS] = make_float4(fcos.x, fcos.y, fcos.z, 0.0f);
-        vr0[(size_t)loc * AV_FIELDS + AV_K] = make_float4(kk.x, kk.y, kk.z, 0.0f);
-        vr0[(size_t)loc * AV_FIELDS + AV_DA] = make_float4(dat.x, dat.y, dat.z, 0.0f);
-        vr0[(size_t)loc * AV_FIELDS + AV_DAL] = make_float4(dalt.x, dalt.y, dalt.z, 0.0f);
+        float* const v = vr0 + (size_t)loc * AV_FLOATS;
+        store8(v, beta, c, __int_as_float(nee << AV_NEE_SHIFT | si.material), 0.0f);
+        if (nee) {
+            store8(v + AV_LIGHT, fcos, kk, 0.0f, 0.0f);
+            store8(v + AV_DLIGHT, dat, dalt, 0.0f, 0.0f);
+        }
         const int nv = level + 1;
         float3 w = zero, dwa = zero, dwr = zero;
         bool go = false;
@@ -802,9 +821,8 @@ __global__ void __launch_bounds__(PATH_BLOCK, 5) k_adj_shade(FrameParams F, AdjP
                 d = bs.wi;
             }
         }
-        vr0[(size_t)loc * AV_FIELDS + AV_W] = make_float4(w.x, w.y, w.z, 0.0f);
-        vr0[(size_t)loc * AV_FIELDS + AV_DWA] = make_float4(dwa.x, dwa.y, dwa.z, 0.0f);
-        vr0[(size_t)loc * AV_FIELDS + AV_DWR] = make_float4(dwr.x, dwr.y, dwr.z, 0.0f);
+        store8(v + AV_NEXT, w, dwa, dwr.x, dwr.y);
+        v[AV_DWR_Z] = dwr.z;
         if (!go) {
             end_path(false, nv, zero, zero);
             continue;
@@ -948,8 +966,8 @@ __device__ __forceinline__ float3 sample_weight(const AdjParams& A, int p, float
 // forward's sum), clamp, image, and the reverse sweep into the gradients.
 // Forward half: bound by the latency of the records' loads (held to 64
 // registers: left to 193 it keeps 8 warps per SM); backward half: by the FP64
-// pipe (72% busy, 1/64 of the FP32 rate).  512x512x32 samples, depth 6: 278 us
-// and 541 us; with an atomic add per lane, parameter and image channel, 363
+// pipe (72% busy, 1/64 of the FP32 rate).  512x512x32 samples, depth 6: 257 us
+// and 537 us; with an atomic add per lane, parameter and image channel, 363
 // and 784.
 __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjParams A, long long wave0) {
     extern __shared__ double sg[];
@@ -973,13 +991,10 @@ __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjP
         const bool in = i < n;
         int p = -1, nv = 0;
         float3 g = make_float3(0.0f, 0.0f, 0.0f), R = g, Lc = g;
-        // c of vertex k: its emission, plus its light sample where visible
-        auto vertex_c = [&](const float4* v, float4 emit, bool vis) {
-            const float3 c = xyz3(emit);
-            if (!vis) return c;
-            const float3 fcos = xyz3(v[AV_FCOS]);
-            const float3 kk = xyz3(v[AV_K]);
-            return __float_as_int(emit.w) == 1 ? c + fcos * sun_rad * kk.x : c + fcos * kk;
+        // c of a vertex: its emission, plus its light sample where visible
+        auto vertex_c = [&](float3 emit, const Sector& light, int nee) {
+            if (nee == 0) return emit;
+            return nee == 1 ? emit + light.a * sun_rad * light.b.x : emit + light.a * light.b;
         };
         if (in) {
             const long long item = wave0 + i;
@@ -998,11 +1013,12 @@ __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjP
 #pragma unroll 1
                 for (int k = 0; k < nv; ++k) {
                     const size_t o = (size_t)k * cap + i;
-                    const float4* v = A.vr + o * AV_FIELDS;
-                    const float3 b = xyz3(v[AV_BETA]);
-                    const float4 emit = v[AV_EMIT];
-                    const bool vis = A.vis[o] != 0 && __float_as_int(emit.w) != 0;
-                    L = L + b * vertex_c(v, emit, vis);
+                    const float* v = A.vr + o * AV_FLOATS;
+                    const Sector h = load8(v);
+                    const int nee = A.vis[o] ? __float_as_int(h.c) >> AV_NEE_SHIFT : 0;
+                    Sector light;
+                    if (nee) light = load8(v + AV_LIGHT);
+                    L = L + h.a * vertex_c(h.b, light, nee);
                 }
                 if (escaped) L = L + b_end * s_end;
                 if (A.lpath) A.lpath[i] = make_float4(L.x, L.y, L.z, 0.0f);
@@ -1028,27 +1044,29 @@ __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjP
             float add[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             if (k < nv) {
                 const size_t o = (size_t)k * cap + i;
-                const float4* v = A.vr + o * AV_FIELDS;
-                const float4 b4 = v[AV_BETA], emit = v[AV_EMIT];
-                const bool vis = A.vis[o] != 0 && __float_as_int(emit.w) != 0;
-                const float3 wk = xyz3(v[AV_W]), dwa = xyz3(v[AV_DWA]), dwr = xyz3(v[AV_DWR]);
-                const float3 ck = vertex_c(v, emit, vis);
+                const float* v = A.vr + o * AV_FLOATS;
+                const Sector h = load8(v), nx = load8(v + AV_NEXT);
+                const int kind = __float_as_int(h.c), nee = A.vis[o] ? kind >> AV_NEE_SHIFT : 0;
+                const float3 wk = nx.a, dwa = nx.b, dwr = make_float3(nx.c, nx.d, h.d);
+                Sector light;
+                if (nee) light = load8(v + AV_LIGHT);
+                const float3 ck = vertex_c(h.b, light, nee);
                 float3 dca = make_float3(0.0f, 0.0f, 0.0f), dcr = dca, cs = dca;
-                if (vis) {
-                    const float3 kk = xyz3(v[AV_K]);
-                    const float3 da = xyz3(v[AV_DA]), dl = xyz3(v[AV_DAL]);
-                    if (__float_as_int(emit.w) == 1) {
-                        dca = da * sun_rad * kk.x;
-                        dcr = dl * sun_rad * kk.x;
-                        cs = xyz3(v[AV_FCOS]) * kk.x;
+                if (nee) {
+                    const float3 kk = light.b;
+                    const Sector dl = load8(v + AV_DLIGHT);
+                    if (nee == 1) {
+                        dca = dl.a * sun_rad * kk.x;
+                        dcr = dl.b * sun_rad * kk.x;
+                        cs = light.a * kk.x;
                     } else {
-                        dca = da * kk;
-                        dcr = dl * kk;
+                        dca = dl.a * kk;
+                        dcr = dl.b * kk;
                     }
                 }
-                const float3 gb = wmul(g, xyz3(b4));
+                const float3 gb = wmul(g, h.a);
                 const float3 ta = wmul(gb, dca + wmul(dwa, R));
-                mat = __float_as_int(b4.w);
+                mat = kind & ((1 << AV_NEE_SHIFT) - 1);
                 add[0] = ta.x;
                 add[1] = ta.y;
                 add[2] = ta.z;

@@ -171,7 +171,8 @@ struct kpt_context {
     DBuf<int> rec_count;
     DBuf<float4> adj_skyq;      // deferred double-precision sky Jacobians: (direction, weight)
     DBuf<int> adj_skyq_count;
-    DBuf<float4> adj_vr, adj_vend, adj_vsky, adj_vskyJ, adj_skyw;   // the wavefront replay's vertex and end records, escape skies
+    DBuf<float> adj_vr;
+    DBuf<float4> adj_vend, adj_vsky, adj_vskyJ, adj_skyw;   // the wavefront replay's vertex and end records, escape skies
     DBuf<float4> adj_lpath;                    // the split adjoint's per-path radiance
     // the records kept by kpt_adjoint_forward_device for the backward call,
     // and the state they were replayed in
@@ -1858,6 +1859,10 @@ kpt_status kpt_set_tuning(kpt_context* c, const kpt_tuning* t) {
 // ---------------------------------------------------------------------------
 // path-replay adjoint
 
+// What a path slot takes of ADJ_WAVE_BYTES: a share of 145 bytes a vertex (its
+// record of 128, its visibility, the path's sky values) and the path's end.
+static size_t adj_path_bytes(int D) { return 145 * (size_t)(D + 1) + 2 * sizeof(float4); }
+
 static int adjoint_params(const kpt_context* c) { return 4 * (int)c->materials.size() + ADJ_SKY_PARAMS; }
 
 // What precedes the replay's waves: the sky's constants, the sun's
@@ -1938,11 +1943,11 @@ static kpt_status adjoint_run(kpt_context* c, int sample0, int nsamples, const f
     F.sky = sky_params(c->env);   // the replay and its Jacobians: IEEE sky arithmetic
     // the wavefront replay's records: a wave of at most ADJ_WAVE_BYTES of them
     const int D = F.max_depth;
-    const size_t per_path = sizeof(float4) * ((size_t)AV_FIELDS * (D + 1) + 2) + (size_t)(D + 1);
+    const size_t per_path = adj_path_bytes(D);
     if (!rec) {
         const size_t fit = std::max<size_t>(1 << 16, ADJ_WAVE_BYTES / per_path);
         F.cap = (int)std::min<size_t>((size_t)F.cap, fit);
-        KPT_CUDA(c->adj_vr.ensure((size_t)AV_FIELDS * (D + 1) * F.cap));
+        KPT_CUDA(c->adj_vr.ensure((size_t)AV_FLOATS * (D + 1) * F.cap));
         KPT_CUDA(c->adj_vend.ensure(2 * (size_t)F.cap));
         KPT_CUDA(c->adj_vsky.ensure((size_t)F.cap));
         KPT_CUDA(c->adj_vskyJ.ensure(3 * (size_t)F.cap));
@@ -2052,7 +2057,7 @@ kpt_status kpt_adjoint_forward_device(kpt_context* c, int sample0, int nsamples,
     FrameParams F = frame_params(c, sample0, nsamples);
     F.sky = sky_params(c->env);   // IEEE sky arithmetic, as the replay's Jacobians
     const int D = F.max_depth;
-    const size_t per_path = sizeof(float4) * ((size_t)AV_FIELDS * (D + 1) + 2) + (size_t)(D + 1);
+    const size_t per_path = adj_path_bytes(D);
     if (items > F.cap || (size_t)items * per_path > ADJ_WAVE_BYTES)
         return fail(KPT_ERR_INVALID, "kpt_adjoint_forward_device: the samples' records exceed one replay wave "
                                      "(use kpt_adjoint_device)");
@@ -2060,7 +2065,7 @@ kpt_status kpt_adjoint_forward_device(kpt_context* c, int sample0, int nsamples,
     const size_t qcap = (size_t)np * ((size_t)nsamples + 1);
     KPT_CUDA(c->sun_J.ensure(ADJ_SKY_PARAMS));
     KPT_CUDA(c->rec_count.ensure(1));
-    KPT_CUDA(c->adj_vr.ensure((size_t)AV_FIELDS * (D + 1) * F.cap));
+    KPT_CUDA(c->adj_vr.ensure((size_t)AV_FLOATS * (D + 1) * F.cap));
     KPT_CUDA(c->adj_vend.ensure(2 * (size_t)F.cap));
     KPT_CUDA(c->adj_vsky.ensure((size_t)F.cap));
     KPT_CUDA(c->adj_vskyJ.ensure(3 * (size_t)F.cap));

@@ -134,12 +134,13 @@ struct AdjParams {
     float4* skyq;
     int* skyq_count;
     int skyq_cap;
-    // the wavefront replay: per vertex AV_FIELDS float4 fields, field f of
-    // level l, path slot i at vr[(l * cap + i) * AV_FIELDS + f]; per path slot
+    // the wavefront replay: per vertex a record of AV_FLOATS floats, one line
+    // of memory (AdjVField), of level l, path slot i at
+    // vr + (l * cap + i) * AV_FLOATS; per path slot
     // its end (direction, vertex count; throughput, escaped) at vend[2 i],
     // vend[2 i + 1]; vis[l * cap + i] = 1 when the light sample of vertex l
     // is unoccluded
-    float4* vr;
+    float* vr;
     float4* vend;
     float4* vsky;              // [cap] the sky radiance of an escaped path's last ray
     float4* vskyJ;             // [cap][3] its single-precision Jacobian
@@ -155,7 +156,13 @@ struct AdjParams {
 };
 
 // fields of the wavefront replay's vertex record
-enum AdjVField { AV_BETA, AV_EMIT, AV_FCOS, AV_K, AV_DA, AV_DAL, AV_W, AV_DWA, AV_DWR, AV_FIELDS };
+// A vertex's record, in 32-byte sectors: throughput, emission, kind of light
+// sample and material, ... | light sample: f cos, weight | its derivatives by
+// albedo and roughness | weight to the next vertex, its derivatives by albedo
+// and (x, y) roughness.  The second and third only where a light sample's ray
+// was sent.
+enum AdjVField { AV_BETA = 0, AV_EMIT = 3, AV_KIND = 6, AV_DWR_Z = 7, AV_LIGHT = 8, AV_DLIGHT = 16, AV_NEXT = 24, AV_FLOATS = 32 };
+constexpr int AV_NEE_SHIFT = 28;   // AV_KIND: kind << AV_NEE_SHIFT | material
 
 // Frisvad basis applied to l, IEEE arithmetic (maths/matrix_maths.cuh:375-396).
 __device__ __forceinline__ float3 onb_apply_exact(float3 n, float3 l) {

@@ -63,14 +63,7 @@ struct CameraQueue {
     }
     __device__ __forceinline__ bool closest(int i, const Hit& h, float3&, float3&) const {
         const int2 p = tiled_pixel(i, F.W, F.H);
-        PrimaryRec r;
-        r.t = h.t;
-        r.u = h.u;
-        r.v = h.v;
-        r.inst = h.inst;
-        r.tri = h.tri;
-        r.pad0 = r.pad1 = r.pad2 = 0;
-        F.primary[p.y * F.W + p.x] = r;
+        store_hit(F.primary + p.y * F.W + p.x, h.t, h.u, h.v, h.inst, h.tri);
         return false;
     }
     __device__ __forceinline__ void any(int, bool) const {}
@@ -363,8 +356,7 @@ struct WaveSink {
         else emit_shadow(F, si, target, c, item, here + 2, true);
     }
     __device__ __forceinline__ void next(const PathRec& pr) {
-        const int j = group_append(ahead);
-        out[j] = pr;
+        store_path(out + group_append(ahead), pr);
     }
 };
 
@@ -411,7 +403,7 @@ __device__ __forceinline__ void shade_path(const FrameParams& F, bool first, int
         seed = S0.seed;
         h = F.primary[p];
     } else {
-        const PathRec pr = F.paths[level & 1][i];
+        const PathRec pr = load_path(F.paths[level & 1] + i);
         o = make_float3(pr.o_pb.x, pr.o_pb.y, pr.o_pb.z);
         p_b = pr.o_pb.w;
         d = make_float3(pr.d_seed.x, pr.d_seed.y, pr.d_seed.z);
@@ -419,7 +411,7 @@ __device__ __forceinline__ void shade_path(const FrameParams& F, bool first, int
         beta = make_float3(pr.beta_item.x, pr.beta_item.y, pr.beta_item.z);
         item = __float_as_int(pr.beta_item.w);
         prev = make_float3(pr.prev.x, pr.prev.y, pr.prev.z);
-        h = F.hits[i];
+        h = load_hit(F.hits + i);
         const float4 l4 = F.radiance[item];
         L = make_float3(l4.x, l4.y, l4.z);
     }
@@ -610,20 +602,14 @@ struct ExtendQueue {
     PrimaryRec* out;
     __device__ __forceinline__ float tmin() const { return 0.0f; }
     __device__ __forceinline__ void ray(int i, float3& o, float3& d, float& tmax) const {
-        const float4 a = in[i].o_pb, b = in[i].d_seed;
+        float4 a, b;
+        load_sector(&in[i].o_pb, a, b);
         o = make_float3(a.x, a.y, a.z);
         d = make_float3(b.x, b.y, b.z);
         tmax = __int_as_float(0x7f800000);
     }
     __device__ __forceinline__ bool closest(int i, const Hit& h, float3&, float3&) const {
-        PrimaryRec r;
-        r.t = h.t;
-        r.u = h.u;
-        r.v = h.v;
-        r.inst = h.inst;
-        r.tri = h.tri;
-        r.pad0 = r.pad1 = r.pad2 = 0;
-        out[i] = r;
+        store_hit(out + i, h.t, h.u, h.v, h.inst, h.tri);
         return false;
     }
     __device__ __forceinline__ void any(int, bool) const {}
@@ -1096,14 +1082,7 @@ struct BatchExtendQueue {
     __device__ __forceinline__ bool closest(int i, const Hit& h, float3&, float3&) const {
         const int j = batch_job_of(Q.ext_prefix, Q.njobs, i);
         const BatchJob& J = Q.jobs[j];
-        PrimaryRec r;
-        r.t = h.t;
-        r.u = h.u;
-        r.v = h.v;
-        r.inst = h.inst >= 0 ? h.inst - J.inst_base : -1;
-        r.tri = h.tri;
-        r.pad0 = r.pad1 = r.pad2 = 0;
-        J.hits[i - __ldg(Q.ext_prefix + j)] = r;
+        store_hit(J.hits + (i - __ldg(Q.ext_prefix + j)), h.t, h.u, h.v, h.inst >= 0 ? h.inst - J.inst_base : -1, h.tri);
         return false;
     }
     __device__ __forceinline__ void any(int, bool) const {}

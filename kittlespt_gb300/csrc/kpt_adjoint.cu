@@ -45,6 +45,31 @@ __device__ __forceinline__ void grad_end(const double* sg, int n, double* out) {
         if (sg[i] != 0.0) atomicAdd(out + i, sg[i]);
 }
 
+// A sum of floats as three floats: each addition's rounding error is kept in
+// the next (two-sums), the last of them good to 2^-72 of the sum -- nearer than
+// a double, whose additions run at 1/64 of the float rate.  A sum that leaves
+// 2^100 (or infinity or NaN) goes to *spill, in double.
+struct FloatSum {
+    float hi = 0.0f, mid = 0.0f, lo = 0.0f;
+    static __device__ __forceinline__ float two_sum(float& a, float b) {   // a += b, returning the error
+        const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+        const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+        a = s;
+        return e;
+    }
+    __device__ __forceinline__ double value() const { return (double)hi + ((double)mid + (double)lo); }
+    __device__ __forceinline__ void add(float v, double* spill) {
+        if (fabsf(__fadd_rn(hi, v)) < 0x1p100f) {
+            float e = two_sum(hi, v);
+            e = two_sum(mid, e);
+            lo = __fadd_rn(lo, e);
+        } else {
+            atomicAdd(spill, value() + (double)v);
+            hi = mid = lo = 0.0f;
+        }
+    }
+};
+
 // g * x per channel, 0 where the weight g is 0 (a clamped channel: its
 // derivative terms may be infinite)
 __device__ __forceinline__ float3 wmul(float3 g, float3 x) {
@@ -495,14 +520,14 @@ __device__ __forceinline__ void sum_jacobians(int n, double* grad, Jacobian jaco
     if ((int)(blockIdx.x * blockDim.x) >= n) return;   // the sums of blocks without entries would cost FP64 time too
     if (threadIdx.x < SKY_PARAMS) sg[threadIdx.x] = 0.0;
     __syncthreads();
-    double gsky[SKY_PARAMS] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    FloatSum gsky[SKY_PARAMS];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float3 J[SKY_PARAMS];
         const float3 w = jacobian(i, J);
-        for (int k = 0; k < SKY_PARAMS; ++k) gsky[k] += wdot(w, J[k]);
+        for (int k = 0; k < SKY_PARAMS; ++k) gsky[k].add(wdot(w, J[k]), sg + k);
     }
     for (int k = 0; k < SKY_PARAMS; ++k) {
-        double v = gsky[k];
+        double v = gsky[k].value();
         for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
         if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(sg + k, v);
     }
@@ -542,7 +567,7 @@ __device__ __forceinline__ void load_jacobian(const float4* v, float3* J) {
 // The single-precision sky Jacobians of the wave's other escapes, which
 // k_adj_sky stored, with the weights of k_adj_sweep.  (Summed in the sweep
 // itself, where half a warp's paths escape, they cost it 120 us of
-// 512x512x32 samples, here 110: both are bound by the FP64 additions.)
+// 512x512x32 samples; here, added in double too, 114, as FloatSums 70.)
 __global__ void __launch_bounds__(PATH_BLOCK) k_adjoint_sky_w(AdjParams A) {
     sum_jacobians(*A.skyw_count, A.grad + 4 * A.nmat, [&](int i, float3* J) {
         const float4 w = A.skyw[i];
@@ -966,8 +991,8 @@ __device__ __forceinline__ float3 sample_weight(const AdjParams& A, int p, float
 // forward's sum), clamp, image, and the reverse sweep into the gradients.
 // Forward half: bound by the latency of the records' loads (held to 64
 // registers: left to 193 it keeps 8 warps per SM); backward half: by the FP64
-// pipe (72% busy, 1/64 of the FP32 rate).  512x512x32 samples, depth 6: 257 us
-// and 537 us; with an atomic add per lane, parameter and image channel, 363
+// pipe (1/64 of the FP32 rate; the materials' sums, the sun's being FloatSums:
+// 537 us with all in double).  512x512x32 samples, depth 6: 257 us and 475 us; with an atomic add per lane, parameter and image channel, 363
 // and 784.
 __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjParams A, long long wave0) {
     extern __shared__ double sg[];
@@ -977,10 +1002,11 @@ __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjP
     const long long left = (long long)nhit * F.nsamples - wave0;
     const int n = (int)(left < 0 ? 0 : (left < cap ? left : cap));
     if ((long long)blockIdx.x * blockDim.x >= n) return;   // (its sums would cost FP64 time)
-    grad_begin(sg, ng);
+    grad_begin(sg, ng + SWEEP_SPILL);
     // the sun light samples' weights, summed: their sky gradient is linear in
     // the sun's Jacobian, applied once at the end
-    double cs0 = 0.0, cs1 = 0.0, cs2 = 0.0;
+    FloatSum cs0, cs1, cs2;
+    double* const spill = sg + ng;   // SWEEP_SPILL more slots
     const SkyParams& P = F.sky;
     const float3 obs = make_float3(0.0f, P.earth_r + 1.0f, 0.0f);
     const float3 sun_rad = *F.sun_radiance;
@@ -1073,9 +1099,9 @@ __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjP
                 add[3] = wdot(gb, dcr + wmul(dwr, R));
                 if (nonzero(cs)) {
                     const float3 gs = wmul(gb, cs);
-                    cs0 += gs.x;
-                    cs1 += gs.y;
-                    cs2 += gs.z;
+                    cs0.add(gs.x, spill);
+                    cs1.add(gs.y, spill + 1);
+                    cs2.add(gs.z, spill + 2);
                 }
                 R = ck + wk * R;
             }
@@ -1083,9 +1109,16 @@ __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjP
         }
     }
     if (!A.adjoint) return;   // uniform over the block: the image only, no gradient
+    __syncthreads();   // (what went to spill)
+    double c0 = cs0.value(), c1 = cs1.value(), c2 = cs2.value();
+    if (threadIdx.x == 0) {
+        c0 += spill[0];
+        c1 += spill[1];
+        c2 += spill[2];
+    }
     for (int q = 0; q < SKY_PARAMS; ++q) {   // one shared add per warp per sky parameter
         const float3 J = A.sun_J[q];
-        double v = cs0 * J.x + cs1 * J.y + cs2 * J.z;
+        double v = c0 * J.x + c1 * J.y + c2 * J.z;
         for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
         if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(sg + 4 * A.nmat + q, v);
     }

@@ -1931,8 +1931,8 @@ static kpt_status adjoint_run(kpt_context* c, int sample0, int nsamples, const f
     if (c->settings.max_depth + 1 > ADJ_MAX_VERTICES)
         return fail(KPT_ERR_INVALID, "kpt_adjoint: max_depth above 16");
     const int ng = adjoint_params(c);
-    const size_t smem = sizeof(double) * (size_t)ng;
-    if (smem > 200 * 1024) return fail(KPT_ERR_INVALID, "kpt_adjoint: too many materials");
+    const size_t smem = sizeof(double) * (size_t)(ng + SWEEP_SPILL);
+    if (sizeof(double) * (size_t)ng > 200 * 1024) return fail(KPT_ERR_INVALID, "kpt_adjoint: too many materials");
     st = ensure_work(c, nsamples);
     if (st != KPT_OK) return st;
     KPT_CUDA(c->sun_J.ensure(ADJ_SKY_PARAMS));
@@ -2048,8 +2048,8 @@ kpt_status kpt_adjoint_forward_device(kpt_context* c, int sample0, int nsamples,
     if (c->settings.max_depth + 1 > ADJ_MAX_VERTICES)
         return fail(KPT_ERR_INVALID, "kpt_adjoint_forward_device: max_depth above 16");
     const int ng = adjoint_params(c);
-    const size_t smem = sizeof(double) * (size_t)ng;
-    if (smem > 200 * 1024) return fail(KPT_ERR_INVALID, "kpt_adjoint_forward_device: too many materials");
+    const size_t smem = sizeof(double) * (size_t)(ng + SWEEP_SPILL);
+    if (sizeof(double) * (size_t)ng > 200 * 1024) return fail(KPT_ERR_INVALID, "kpt_adjoint_forward_device: too many materials");
     st = ensure_work(c, nsamples);
     if (st != KPT_OK) return st;
     const int np = c->W * c->H;
@@ -2146,7 +2146,7 @@ kpt_status kpt_adjoint_backward_device(kpt_context* c, const float* adjoint, dou
     A.grad = grad;
     A.lpath_ready = 1;
     const int ng = adjoint_params(c);
-    const size_t smem = sizeof(double) * (size_t)ng;
+    const size_t smem = sizeof(double) * (size_t)(ng + SWEEP_SPILL);
     int per_sm = 0;
     KPT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adj_sweep, PATH_BLOCK, smem));
     const int grid = std::max(1, per_sm) * c->sm_count;

@@ -201,6 +201,7 @@ struct AdjParams {
 // and (x, y) roughness.  The second and third only where a light sample's ray
 // was sent.
 enum AdjVField { AV_BETA = 0, AV_EMIT = 3, AV_KIND = 6, AV_DWR_Z = 7, AV_LIGHT = 8, AV_DLIGHT = 16, AV_NEXT = 24, AV_FLOATS = 32 };
+constexpr int SWEEP_SPILL = 3;     // doubles of shared memory after the gradient's in k_adj_sweep
 constexpr int AV_NEE_SHIFT = 28;   // AV_KIND: kind << AV_NEE_SHIFT | material
 
 // Frisvad basis applied to l, IEEE arithmetic (maths/matrix_maths.cuh:375-396).

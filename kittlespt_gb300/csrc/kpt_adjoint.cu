@@ -991,9 +991,9 @@ __device__ __forceinline__ float3 sample_weight(const AdjParams& A, int p, float
 // forward's sum), clamp, image, and the reverse sweep into the gradients.
 // Forward half: bound by the latency of the records' loads (held to 64
 // registers: left to 193 it keeps 8 warps per SM); backward half: by the FP64
-// pipe (1/64 of the FP32 rate; the materials' sums, the sun's being FloatSums:
-// 537 us with all in double).  512x512x32 samples, depth 6: 257 us and 475 us; with an atomic add per lane, parameter and image channel, 363
-// and 784.
+// pipe (1/64 of the FP32 rate; the materials' sums, the sun's being FloatSums).
+// 512x512x32 samples, depth 6: 257 us and 475 us; with every sum in double 537,
+// with an atomic add per lane, parameter and image channel 363 and 784.
 __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjParams A, long long wave0) {
     extern __shared__ double sg[];
     const int ng = 4 * A.nmat + ADJ_SKY_PARAMS;

@@ -1,0 +1,32 @@
+// kpt_index.h -- the kernels' index arithmetic that reaches the end of a
+// 32-bit range, also as plain C++ (tests/index_range.cpp walks it on the CPU).
+#pragma once
+
+#ifdef __CUDACC__
+#define KPT_HOST_DEVICE __host__ __device__ __forceinline__
+#else
+#define KPT_HOST_DEVICE inline
+#endif
+
+namespace kpt {
+
+// use(i, whether it is the lane that stores) for every i in [i0, n) that
+// `thread` of a grid of `threads` (whole warps) takes, LANES neighbouring lanes
+// to an i.  With several, whole warps: the groups past the end repeat the last.
+// Unsigned: i < 2^31 and, where a grid of one thread per i covers n, a stride
+// of up to 2^31, whose sum an int does not hold from n = 2^30 + 1 on.
+template <int LANES, class Use>
+KPT_HOST_DEVICE void spread(unsigned thread, unsigned threads, int i0, int n, Use use) {
+    const unsigned all = threads / LANES, end = (unsigned)n;
+    if (LANES == 1) {
+        for (unsigned i = (unsigned)i0 + thread; i < end; i += all) use((int)i, true);
+    } else {
+        const unsigned lane = thread & 31u, group = lane / LANES;
+        for (unsigned i = (unsigned)i0 + (thread & ~31u) / LANES; i < end; i += all) {   // the warp's first
+            const unsigned k = i + group;
+            use((int)(k < end ? k : end - 1u), k < end && (lane & (LANES - 1)) == 0);
+        }
+    }
+}
+
+}  // namespace kpt

@@ -8,6 +8,7 @@
 // result rounded to float is formed in float (ggx_b).
 #pragma once
 #include "kpt_device.cuh"
+#include "kpt_index.h"
 
 // KPT_BSDF_CALL: the BSDF's f / pdf / sample are compiled as one out-of-line
 // copy each (the shading kernel calls f and pdf twice per vertex; inlined it
@@ -573,19 +574,10 @@ __device__ __forceinline__ int sky_lanes(int n, int threads) {
     return 8LL * n <= threads ? 8 : 2LL * n <= threads ? 2 : 1;
 }
 
-// use(i, whether it is the lane that stores) for every i in [i0, n), spread over
-// the grid with LANES lanes each.  With several, whole warps: the groups past
-// the end repeat the last.
+// spread() over the kernel's grid.
 template <int LANES, class Use>
 __device__ __forceinline__ void sky_spread(int i0, int n, Use use) {
-    const int thread = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x / LANES;
-    if (LANES == 1) {
-        for (int i = i0 + thread; i < n; i += all) use(i, true);
-    } else {
-        const int group = (threadIdx.x & 31) / LANES;
-        for (int i = i0 + (thread & ~31) / LANES; i < n; i += all)   // the warp's first
-            use(min(i + group, n - 1), i + group < n && (threadIdx.x & (LANES - 1)) == 0);
-    }
+    spread<LANES>(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, i0, n, use);
 }
 
 }  // namespace kpt

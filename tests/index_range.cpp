@@ -1,0 +1,42 @@
+// Walks the kernels' index arithmetic (kpt_index.h) at the ends of its ranges.
+// Prints "<name> <places checked> <wrong>".
+#include <cstdio>
+#include <initializer_list>
+
+#include "kpt_index.h"
+
+// k_sky's launch for n directions, blocks of 64 threads: every thread of the
+// blocks around the ends and the middle of the grid, and around n - 2^30 and
+// 2^31 - (grid), where a signed sum of index and stride changes sign.
+template <int LANES>
+static void sky(long long n, long long& places, long long& wrong) {
+    constexpr long long BLOCK = 64;
+    const long long per_block = BLOCK / LANES, blocks = (n - 1) / per_block + 1, threads = blocks * BLOCK;
+    for (long long near : {0LL, threads / 3, threads / 2, threads, n - (1LL << 30), (1LL << 31) - threads, (1LL << 30)}) {
+        for (long long t = near - 256; t < near + 256; ++t) {
+            if (t < 0 || t >= threads) continue;
+            int visits = 0, stored = -1;
+            bool inside = true;
+            kpt::spread<LANES>((unsigned)t, (unsigned)threads, 0, (int)n, [&](int i, bool first) {
+                inside = inside && i >= 0 && i < n;
+                if (first) stored = i;
+                ++visits;
+            });
+            const long long mine = t / LANES;   // the grid covers n once
+            const bool stores = t % LANES == 0 && mine < n;
+            const bool warp_in = (t & ~31LL) / LANES < n;
+            ++places;
+            if (!inside || visits != (warp_in && (LANES > 1 || mine < n) ? 1 : 0) || stored != (stores ? (int)mine : -1)) ++wrong;
+        }
+    }
+}
+
+int main() {
+    long long places = 0, wrong = 0;
+    for (long long n : {1LL, 31LL, 63LL, 64LL, 65LL, 131072LL, (1LL << 30) - 1, 1LL << 30, (1LL << 30) + 1, 1500000000LL,
+                        (1LL << 31) - 65, (1LL << 31) - 64, (1LL << 31) - 63, (1LL << 31) - 1})
+        sky<1>(n, places, wrong);
+    for (long long n : {1LL, 3LL, 4LL, 5LL, 31LL, 33LL, 30000LL}) sky<8>(n, places, wrong), sky<2>(n, places, wrong);
+    std::printf("sky %lld %lld\n", places, wrong);
+    return 0;
+}

@@ -29,4 +29,13 @@ KPT_HOST_DEVICE void spread(unsigned thread, unsigned threads, int i0, int n, Us
     }
 }
 
+// Lanes of each of `warps` that take rays of a queue of n > 0 rays.
+KPT_HOST_DEVICE int lanes_of_queue(int n, int warps) { return (n - 1) / warps + 1; }
+
+// The queue's entry `rank` after the fetch counter's value `base`, and whether
+// the queue of n has it.  Unsigned: the counter ends up to a grid's lanes past
+// n, beyond 2^31 - 1 for the longest queues.
+KPT_HOST_DEVICE int queue_entry(int base, int rank) { return (int)((unsigned)base + (unsigned)rank); }
+KPT_HOST_DEVICE bool queued(int entry, int n) { return (unsigned)entry < (unsigned)n; }
+
 }  // namespace kpt

@@ -761,8 +761,8 @@ __global__ void __launch_bounds__(TRACE_BLOCK, TAIL_MIN_BLOCKS) k_tail(const __g
                 PrimaryRec h;
                 float3 wo, wd;
                 if (i < 0) {
-                    i = base + __popc(want & ((1u << lane) - 1u));
-                    if (i < n) {
+                    i = queue_entry(base, __popc(want & ((1u << lane) - 1u)));
+                    if (queued(i, n)) {
                         h = F.hits[i];
                         level = level0;
                         shade = true;

@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 
 #include "kpt_device.cuh"
+#include "kpt_index.h"
 #include "kpt_internal.h"
 
 namespace kpt {
@@ -669,8 +670,7 @@ struct Traversal {
 // (1021 rays 88 -> 27 us, the 65k paths of a 256x256 frame 0.85 -> 0.42 ms
 // with this and the above).
 __device__ __forceinline__ int queue_lanes(int n) {
-    const int warps = gridDim.x * (TRACE_BLOCK / 32);
-    return (n + warps - 1) / warps;
+    return lanes_of_queue(n, gridDim.x * (TRACE_BLOCK / 32));
 }
 
 template <bool ANY, class Src, bool ROOTS = false>
@@ -701,8 +701,8 @@ __device__ __forceinline__ void trace_queue(const SceneView& s, int n, int* next
             base = __shfl_sync(FULL, base, 0);
             if (r.cur == T::DONE) {
                 if (!more) {
-                    ray = base + __popc(want & ((1u << lane) - 1u));
-                    if (ray < n) {
+                    ray = queue_entry(base, __popc(want & ((1u << lane) - 1u)));
+                    if (queued(ray, n)) {
                         src.ray(ray, wo, wd, r.tmax);
                         r.bound0 = next_up(r.tmax);
                         more = true;

@@ -31,6 +31,19 @@ static void sky(long long n, long long& places, long long& wrong) {
     }
 }
 
+// A queue of n rays on `warps`: the lanes that take rays (some, and enough for a
+// short queue), and the entries at the counter's values around and past n.
+static void queue(long long n, int warps, long long& places, long long& wrong) {
+    const long long lanes = kpt::lanes_of_queue((int)n, warps);
+    ++places;
+    if (lanes < 1 || lanes * warps < n || (lanes - 1) * warps >= n) ++wrong;
+    for (long long c = n > 40 ? n - 40 : 0; c < n + 32LL * warps; ++c) {
+        const int entry = kpt::queue_entry((int)(unsigned)(c - c % 32), (int)(c % 32));
+        ++places;
+        if (kpt::queued(entry, (int)n) != (c < n) || (c < n && entry != c)) ++wrong;
+    }
+}
+
 int main() {
     long long places = 0, wrong = 0;
     for (long long n : {1LL, 31LL, 63LL, 64LL, 65LL, 131072LL, (1LL << 30) - 1, 1LL << 30, (1LL << 30) + 1, 1500000000LL,
@@ -38,5 +51,11 @@ int main() {
         sky<1>(n, places, wrong);
     for (long long n : {1LL, 3LL, 4LL, 5LL, 31LL, 33LL, 30000LL}) sky<8>(n, places, wrong), sky<2>(n, places, wrong);
     std::printf("sky %lld %lld\n", places, wrong);
+    places = wrong = 0;
+    for (int warps : {1, 4, 1216, 9728})
+        for (long long n : {1LL, 31LL, 1021LL, 9728LL, 9729LL, 700001LL, (1LL << 31) - 320000, (1LL << 31) - 9728,
+                            (1LL << 31) - 9727, (1LL << 31) - 1})
+            queue(n, warps, places, wrong);
+    std::printf("queue %lld %lld\n", places, wrong);
     return 0;
 }

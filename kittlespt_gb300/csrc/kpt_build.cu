@@ -36,6 +36,7 @@
 #include <climits>
 #include <vector>
 
+#include "kpt_index.h"
 #include "kpt_scene.h"
 
 namespace kpt {
@@ -1194,8 +1195,9 @@ __global__ void k_refit_tris(const float* pos, const float* nrm, int n, float4* 
 // after the other, 19 us for 20,480 triangles: two dependent loads each).
 __global__ void k_refit_leaves(BvhNode* nodes, int node_base, int nn, const float* pos, const float4* tris, int* parent,
                                int* need, int* arrive) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x, v = g >> 4, slot = g >> 3 & 1, lane = g & 7;
-    if (v >= nn) return;   // 16 lanes a node: whole groups
+    const unsigned node = node_of_16(blockIdx.x, blockDim.x, threadIdx.x);
+    if (node >= (unsigned)nn) return;   // 16 lanes a node: whole groups
+    const int v = (int)node, slot = threadIdx.x >> 3 & 1, lane = threadIdx.x & 7;
     BvhNode& n = nodes[node_base + v];
     const int4 d = n.d;
     const int ref = slot ? d.z : d.x, cnt = slot ? d.w : d.y;

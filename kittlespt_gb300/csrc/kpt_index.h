@@ -38,4 +38,11 @@ KPT_HOST_DEVICE int lanes_of_queue(int n, int warps) { return (n - 1) / warps + 
 KPT_HOST_DEVICE int queue_entry(int base, int rank) { return (int)((unsigned)base + (unsigned)rank); }
 KPT_HOST_DEVICE bool queued(int entry, int n) { return (unsigned)entry < (unsigned)n; }
 
+// The node (of nn < 2^31) that a thread of a block of block_size threads works
+// on where 16 neighbouring threads take one; the thread's number in the grid
+// would pass 2^31 - 1 at 2^27 nodes.
+KPT_HOST_DEVICE unsigned node_of_16(unsigned block, unsigned block_size, unsigned thread) {
+    return block * (block_size / 16u) + thread / 16u;
+}
+
 }  // namespace kpt

@@ -44,6 +44,20 @@ static void queue(long long n, int warps, long long& places, long long& wrong) {
     }
 }
 
+// k_refit_leaves' launch for nn nodes: blocks of 64 threads, 16 to a node.
+static void refit(long long nn, long long& places, long long& wrong) {
+    constexpr int BLOCK = 64;
+    const long long blocks = (nn - 1) / (BLOCK / 16) + 1;
+    for (long long near : {0LL, (1LL << 25), (1LL << 26), blocks / 2, blocks})
+        for (long long b = near - 3; b < near + 3; ++b)
+            for (int t = 0; t < BLOCK && b >= 0 && b < blocks; ++t) {
+                const unsigned node = kpt::node_of_16((unsigned)b, BLOCK, (unsigned)t);
+                const long long want = (b * BLOCK + t) / 16;
+                ++places;
+                if ((long long)node != want || (node < (unsigned)nn) != (want < nn)) ++wrong;
+            }
+}
+
 int main() {
     long long places = 0, wrong = 0;
     for (long long n : {1LL, 31LL, 63LL, 64LL, 65LL, 131072LL, (1LL << 30) - 1, 1LL << 30, (1LL << 30) + 1, 1500000000LL,
@@ -57,5 +71,9 @@ int main() {
                             (1LL << 31) - 9727, (1LL << 31) - 1})
             queue(n, warps, places, wrong);
     std::printf("queue %lld %lld\n", places, wrong);
+    places = wrong = 0;
+    for (long long nn : {1LL, 3LL, 4LL, 5LL, 20479LL, (1LL << 27) - 1, 1LL << 27, (1LL << 27) + 1, 1LL << 28, (1LL << 31) - 1})
+        refit(nn, places, wrong);
+    std::printf("refit %lld %lld\n", places, wrong);
     return 0;
 }

@@ -17,7 +17,7 @@ def counts(tmp_path_factory):
     return {line.split()[0]: tuple(int(v) for v in line.split()[1:]) for line in out.splitlines()}
 
 
-@pytest.mark.parametrize("walk", ["sky", "queue"])
+@pytest.mark.parametrize("walk", ["sky", "queue", "refit"])
 def test_every_index_is_taken_once_and_in_range(counts, walk):
     places, wrong = counts[walk]
     assert places > 1000 and wrong == 0

@@ -21,6 +21,7 @@
 // and writes the frozen-path records (kpt_adjoint_records_device).
 #include "kpt_adjoint.cuh"
 #include "kpt_pathfn.cuh"
+#include "kpt_sum.h"
 
 namespace kpt {
 
@@ -45,30 +46,16 @@ __device__ __forceinline__ void grad_end(const double* sg, int n, double* out) {
         if (sg[i] != 0.0) atomicAdd(out + i, sg[i]);
 }
 
-// A sum of floats as three floats: each addition's rounding error is kept in
-// the next (two-sums), the last of them good to 2^-72 of the sum -- nearer than
-// a double, whose additions run at 1/64 of the float rate.  A sum that leaves
-// 2^100 (or infinity or NaN) goes to *spill, in double.
-struct FloatSum {
-    float hi = 0.0f, mid = 0.0f, lo = 0.0f;
-    static __device__ __forceinline__ float two_sum(float& a, float b) {   // a += b, returning the error
-        const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
-        const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
-        a = s;
-        return e;
-    }
-    __device__ __forceinline__ double value() const { return (double)hi + ((double)mid + (double)lo); }
-    __device__ __forceinline__ void add(float v, double* spill) {
-        if (fabsf(__fadd_rn(hi, v)) < 0x1p100f) {
-            float e = two_sum(hi, v);
-            e = two_sum(mid, e);
-            lo = __fadd_rn(lo, e);
-        } else {
-            atomicAdd(spill, value() + (double)v);
-            hi = mid = lo = 0.0f;
-        }
-    }
+// A thread's sums of floats (kpt_sum.h), spilling to a double that threads share.
+struct FloatArith {
+    static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+    static __device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b); }
+    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 };
+using FloatSum = FloatSumOf<FloatArith>;
+__device__ __forceinline__ void sum_add(FloatSum& s, float v, double* spill) {
+    s.add(v, [&](double x) { atomicAdd(spill, x); });
+}
 
 // g * x per channel, 0 where the weight g is 0 (a clamped channel: its
 // derivative terms may be infinite)
@@ -524,7 +511,7 @@ __device__ __forceinline__ void sum_jacobians(int n, double* grad, Jacobian jaco
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float3 J[SKY_PARAMS];
         const float3 w = jacobian(i, J);
-        for (int k = 0; k < SKY_PARAMS; ++k) gsky[k].add(wdot(w, J[k]), sg + k);
+        for (int k = 0; k < SKY_PARAMS; ++k) sum_add(gsky[k], wdot(w, J[k]), sg + k);
     }
     for (int k = 0; k < SKY_PARAMS; ++k) {
         double v = gsky[k].value();
@@ -1099,9 +1086,9 @@ __global__ void __launch_bounds__(PATH_BLOCK, 8) k_adj_sweep(FrameParams F, AdjP
                 add[3] = wdot(gb, dcr + wmul(dwr, R));
                 if (nonzero(cs)) {
                     const float3 gs = wmul(gb, cs);
-                    cs0.add(gs.x, spill);
-                    cs1.add(gs.y, spill + 1);
-                    cs2.add(gs.z, spill + 2);
+                    sum_add(cs0, gs.x, spill);
+                    sum_add(cs1, gs.y, spill + 1);
+                    sum_add(cs2, gs.z, spill + 2);
                 }
                 R = ck + wk * R;
             }

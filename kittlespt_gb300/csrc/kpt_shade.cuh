@@ -365,10 +365,7 @@ __device__ __forceinline__ bool sphere_hit_gpu(float3 o, float3 d, float radius,
 // Pairs of single-precision values (two light samples of a march, or its
 // Rayleigh and Mie parts), each operation one instruction for both.
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 exp_pair(float2 x) {   // expf of both, under fast maths
-    x = __fmul2_rn(x, both(1.44269504f));
-    return make_float2(exp2f(x.x), exp2f(x.y));
-}
+__device__ __forceinline__ float2 exp_pair(float2 x) { return make_float2(expf(x.x), expf(x.y)); }
 
 // A view step of the march: the air passed along the step and, from its
 // middle, towards the sun, as (Rayleigh, Mie) optical depths; lit: the light
@@ -378,10 +375,10 @@ struct SkyStep {
     bool lit;
 };
 
-// The model in the arithmetic of the reference's GPU build: the operations
-// that fast maths makes of the reference's expressions (intersectSphere,
-// atmosphere.cuh:30-57; sampleLi, :132-223) -- approximate square root,
-// division and exponential, contracted products.  Its altitudes carry that
+// The model (intersectSphere, atmosphere.cuh:30-57; sampleLi, :132-223) under
+// fast maths, as the reference's GPU build has it: approximate square root and
+// exponential, contracted products; an altitude over a scale height is its
+// product with the height's reciprocal, formed once.  Its altitudes carry that
 // build's rounding (one ulp of a ~6.4e6 m length is 0.5 m), so its sky agrees
 // with that build's rather than with IEEE arithmetic.
 struct SkyGpu {

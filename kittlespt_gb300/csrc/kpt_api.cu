@@ -2240,7 +2240,6 @@ struct kpt_batch {
     cudaEvent_t ev_counts = nullptr, ev_shadow = nullptr, ev_level = nullptr;
     DBuf<BvhNode> m_nodes, m_tlas;
     DBuf<float4> m_tris;
-    DBuf<MeshRec> m_meshes;
     DBuf<InstRec> m_inst;
     SceneView m_view{};
     std::vector<std::pair<const kpt_context*, unsigned long long>> m_key;
@@ -2270,37 +2269,36 @@ double job_cost(const kpt_context* c, int spp) {
     return (double)c->W * c->H * spp * (c->settings.max_depth + 1);
 }
 
-// The batch's merged scene: every job's BLAS nodes, triangles, meshes,
-// instances and TLAS nodes one after the other, their indices moved by the
-// job's offsets (enqueued on the batch stream; rebuilt only when the jobs or
-// one of their scenes changed).
+// The batch's merged scene: every job's BLAS nodes, triangles, instances and
+// TLAS nodes one after the other, their indices moved by the job's offsets
+// (enqueued on the batch stream; rebuilt only when the jobs or one of their
+// scenes changed).  It has no mesh records: its rays enter a BLAS by the
+// instance's root, and what else reads them has the job's own scene.
 kpt_status merge_scenes(kpt_batch* b, int n, kpt_context* const* jobs) {
     std::vector<std::pair<const kpt_context*, unsigned long long>> key(n);
     for (int j = 0; j < n; ++j) key[j] = {jobs[j], jobs[j]->scene_version};
     if (key == b->m_key) return KPT_OK;
-    long long nn = 0, nt = 0, nm = 0, ni = 0, nl = 0;
+    long long nn = 0, nt = 0, ni = 0, nl = 0;
     for (int j = 0; j < n; ++j) {
         nn += jobs[j]->n_nodes;
         nt += jobs[j]->n_tris;
-        nm += (long long)jobs[j]->meshes.size();
         ni += (long long)jobs[j]->instances.size();
         nl += jobs[j]->view.ntlas;
     }
-    if (nn > INT32_MAX / 2 || nt > INT32_MAX / 4 || nm > INT32_MAX || ni > INT32_MAX / 2 || nl > INT32_MAX / 2)
+    if (nn > INT32_MAX / 2 || nt > INT32_MAX / 4 || ni > INT32_MAX / 2 || nl > INT32_MAX / 2)
         return fail(KPT_ERR_INVALID, "kpt_submit_batch: the jobs' scenes together are too large to merge");
     b->m_key.clear();
     KPT_CUDA(b->m_nodes.ensure(nn));
     KPT_CUDA(b->m_tris.ensure(3 * nt + TRI_PAD));
-    KPT_CUDA(b->m_meshes.ensure(nm));
     KPT_CUDA(b->m_inst.ensure(ni));
     KPT_CUDA(b->m_tlas.ensure(nl));
     b->m_tlas_root.assign(n, 0);
     b->m_inst_base.assign(n, 0);
-    int node_base = 0, tri_base = 0, mesh_base = 0, inst_base = 0, tlas_base = 0;
+    int node_base = 0, tri_base = 0, inst_base = 0, tlas_base = 0;
     auto blocks = [](int k) { return (k + 255) / 256; };
     for (int j = 0; j < n; ++j) {
         const kpt_context* c = jobs[j];
-        const int nodes = c->n_nodes, tris = c->n_tris, meshes = (int)c->meshes.size();
+        const int nodes = c->n_nodes, tris = c->n_tris;
         const int inst = (int)c->instances.size(), tlas = c->view.ntlas;
         if (nodes > 0)
             k_merge_nodes<<<blocks(nodes), 256, 0, b->stream>>>(c->d_nodes.p, nodes, b->m_nodes.p + node_base,
@@ -2308,11 +2306,8 @@ kpt_status merge_scenes(kpt_batch* b, int n, kpt_context* const* jobs) {
         if (tris > 0)
             KPT_CUDA(cudaMemcpyAsync(b->m_tris.p + 3 * (size_t)tri_base, c->d_tris.p, 3 * sizeof(float4) * (size_t)tris,
                                      cudaMemcpyDeviceToDevice, b->stream));
-        if (meshes > 0)
-            k_merge_meshes<<<blocks(meshes), 256, 0, b->stream>>>(c->d_meshes.p, meshes, b->m_meshes.p + mesh_base,
-                                                                   node_base, tri_base);
         if (inst > 0)
-            k_merge_inst<<<blocks(inst), 256, 0, b->stream>>>(c->d_inst.p, inst, b->m_inst.p + inst_base, mesh_base, node_base, tri_base);
+            k_merge_inst<<<blocks(inst), 256, 0, b->stream>>>(c->d_inst.p, inst, b->m_inst.p + inst_base, node_base, tri_base);
         if (tlas > 0)
             k_merge_nodes<<<blocks(tlas), 256, 0, b->stream>>>(c->d_tlas.p, tlas, b->m_tlas.p + tlas_base, tlas_base,
                                                                 inst_base);
@@ -2321,14 +2316,12 @@ kpt_status merge_scenes(kpt_batch* b, int n, kpt_context* const* jobs) {
         b->m_inst_base[j] = inst_base;
         node_base += nodes;
         tri_base += tris;
-        mesh_base += meshes;
         inst_base += inst;
         tlas_base += tlas;
     }
     SceneView v{};
     v.nodes = b->m_nodes.p;
     v.tris = b->m_tris.p;
-    v.meshes = b->m_meshes.p;
     v.inst = b->m_inst.p;
     v.tlas = b->m_tlas.p;
     v.ntlas = tlas_base;
@@ -2532,7 +2525,7 @@ kpt_status kpt_batch_destroy(kpt_batch* b) {
         for (cudaEvent_t e : *v) cudaEventDestroy(e);
     for (cudaEvent_t e : {b->ev_counts, b->ev_shadow, b->ev_level})
         if (e) cudaEventDestroy(e);
-    b->m_nodes.release(); b->m_tlas.release(); b->m_tris.release(); b->m_meshes.release(); b->m_inst.release();
+    b->m_nodes.release(); b->m_tlas.release(); b->m_tris.release(); b->m_inst.release();
     b->d_jobs.release(); b->d_queues.release(); b->d_counters.release();
     if (b->side) cudaStreamDestroy(b->side);
     if (b->stream) cudaStreamDestroy(b->stream);

@@ -271,11 +271,10 @@ __global__ void k_sky_constants(FrameParams F, float3* sun_radiance);
 __global__ void k_batch_level(BatchQueues Q, int level);
 __global__ void k_extend_batch(SceneView s, BatchQueues Q, int level, unsigned long long* counters);
 __global__ void k_shadow_batch(SceneView s, BatchQueues Q, int level, unsigned long long* counters);
-// the merged scene of a batch: one job's BLAS / TLAS nodes, meshes and
+// the merged scene of a batch: one job's BLAS / TLAS nodes and
 // instances with their indices moved by the job's offsets
 __global__ void k_merge_nodes(const BvhNode* src, int n, BvhNode* dst, int node_add, int leaf_add);
-__global__ void k_merge_meshes(const MeshRec* src, int n, MeshRec* dst, int node_add, int tri_add);
-__global__ void k_merge_inst(const InstRec* src, int n, InstRec* dst, int mesh_add, int node_add, int tri_add);
+__global__ void k_merge_inst(const InstRec* src, int n, InstRec* dst, int node_add, int tri_add);
 // kpt_adjoint.cu (fast maths)
 __global__ void k_adjoint_constants(FrameParams F, AdjParams A);
 __global__ void k_sky_grad(SkyParams P, int n, const float3* dirs, float3* out);

@@ -1155,21 +1155,10 @@ __global__ void k_merge_nodes(const BvhNode* src, int n, BvhNode* dst, int node_
     dst[i] = b;
 }
 
-__global__ void k_merge_meshes(const MeshRec* src, int n, MeshRec* dst, int node_add, int tri_add) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    MeshRec m = src[i];
-    if (m.node_root >= 0) m.node_root += node_add;
-    m.leaf_first += tri_add;
-    m.tri_base += tri_add;
-    dst[i] = m;
-}
-
-__global__ void k_merge_inst(const InstRec* src, int n, InstRec* dst, int mesh_add, int node_add, int tri_add) {
+__global__ void k_merge_inst(const InstRec* src, int n, InstRec* dst, int node_add, int tri_add) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     InstRec r = src[i];
-    r.mesh += mesh_add;
     r.root = r.root >= 0 ? r.root + node_add : ~(~r.root + tri_add);
     dst[i] = r;
 }

@@ -11,8 +11,7 @@ graphics stack, so the display image is copied into a numpy array.
 from __future__ import annotations
 
 import ctypes as C
-import threading
-import weakref
+import sys
 from typing import Optional
 
 import numpy as np
@@ -42,17 +41,6 @@ def _mat(rec) -> K.Material:
     return m
 
 
-class _Lease:
-    """What an array over `memory` and every view of it refer to: gone when the
-    last of them is."""
-
-    __slots__ = ("__array_interface__", "_memory", "__weakref__")
-
-    def __init__(self, memory: np.ndarray, interface: dict):
-        self._memory = memory
-        self.__array_interface__ = interface
-
-
 class Renderer:
     """One GPU path tracer: scene, camera, settings, accumulation, post chain."""
 
@@ -61,7 +49,7 @@ class Renderer:
         self._ctx = C.c_void_p()
         self._device = device
         self._open = False
-        self._host = []   # of _host_image: memory, its array interface, a weak reference to its lease
+        self._host = []   # image buffers of _host_image
 
     # -- lifetime (renderer.cu:22-53) ----------------------------------------
     def initialize(self):
@@ -265,26 +253,23 @@ class Renderer:
     def synchronize(self):
         K.check(self._L.kpt_synchronize(self._ctx))
 
-    _host_lock = threading.Lock()
-
     def _host_image(self, shape):
         """An image for a read-back, in memory that the CPU has touched.  Of the
         last two images of a renderer, one whose array (and every view of it)
         is gone is used again: a device-to-host copy into untouched pages
         faults page by page from the GPU (1920x1080: 20 ms against 0.19 ms),
         and a new allocation is zeroed or mapped anew on each call (0.55 ms)."""
-        with self._host_lock:
-            for kept in self._host:
-                if kept[0].shape == shape and kept[2]() is None:
-                    break
-            else:
-                memory = np.empty(shape, np.float32)
-                memory.fill(0.0)
-                kept = [memory, memory.__array_interface__, None]
-                self._host = self._host[-1:] + [kept]
-            lease = _Lease(kept[0], kept[1])
-            kept[2] = weakref.ref(lease)
-            return np.asarray(lease)
+        # the references counted for an object that its list and the loop's name alone
+        # hold (3 or fewer, as the interpreter borrows some for the call)
+        for alone in [object()]:
+            unheld = sys.getrefcount(alone)
+        for b in self._host:
+            if b.shape == shape and sys.getrefcount(b) == unheld:
+                return b[...]
+        b = np.empty(shape, np.float32)
+        b.fill(0.0)
+        self._host = self._host[-1:] + [b]
+        return b[...]
 
     def _read(self, fn, shape=None):
         out = self._host_image((self.height, self.width, 4) if shape is None else shape)

@@ -308,7 +308,12 @@ kpt_status kpt_sky_device(kpt_context* ctx, int n, const float* dirs, float* rgb
  * nodes between its launches).  kpt_stage_ms sums, per stage, the time of
  * the last n frames rendered with timing on (n <= 32) into
  * ms[KPT_STAGE_COUNT]; kpt_path_kernel_ms sums the path wave (shade, shadow
- * and extension kernels).  Both synchronise the stream. */
+ * and extension kernels).  Both synchronise the stream.
+ * A frame rendered with timing on runs its stages one after the other and
+ * every level of its paths as a stage; one rendered without runs some of them
+ * beside each other and the later levels in one kernel.  The images are the
+ * same; the stage times are those of the timed frame and add up to it, not to
+ * the untimed one. */
 enum {
     KPT_STAGE_CAMERA = 0,     /* sky constants, camera rays, their sky */
     KPT_STAGE_SHADE = 1,      /* path vertices: emission, light sample, BSDF sample */

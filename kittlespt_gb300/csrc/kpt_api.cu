@@ -1155,13 +1155,21 @@ static void enqueue_path_end(kpt_context* c, const FrameParams& F, int total_sam
 }
 
 // The level (>= 2) from which k_tail takes a wave's paths one by one, above
-// max_depth: none.  It pays while fewer than about 60,000 paths enter it (four
-// per resident warp of the ray kernels: 1920x1080x2 over 64 instances 3.30 ms
-// per level, 3.19 from a level of 75,837 paths, 3.28 from one of 232,618;
-// 640x360x1 over 16 spheres 1.19 and 1.10 ms from one of 50,799).  The host
-// knows the wave's items only; of them at most about 22, 12 and 5% enter
-// levels 2, 3 and 4 and half as many each later one (convex objects under an
-// open sky lose paths sooner and could start earlier, for 1-3% of the frame).
+// max_depth: none.  Under an open sky it pays while fewer than about 60,000
+// paths enter it (twelve per resident warp of the ray kernels: 1920x1080x2 over
+// 64 instances 3.30 ms per level, 3.19 from a level of 75,837 paths, 3.28 from
+// one of 232,618; 640x360x1 over 16 spheres 1.19 and 1.10 ms from one of
+// 50,799).  The host knows the wave's items only; of them there at most about
+// 22, 12 and 5% enter levels 2, 3 and 4 and half as many each later one (convex
+// objects lose paths sooner and could start earlier, for 1-4% of the frame).
+// In a closed room 36, 23 and 14% do and two thirds go on at each later level;
+// there the levels are faster one by one but for the smallest frames, per level
+// and with this rule's tail, depth 8: 12 spheres in a box 256x256x1 0.70 and
+// 0.71 ms, 640x360x1 1.01 and 1.11, 853x481x1 1.25 and 1.39, 1920x1080x1 3.19
+// and 3.63; 16 displaced spheres in a box 0.88 and 0.80, 1.25 and 1.31, 1.53
+// and 1.62, 3.72 and 4.09.  A number of paths alone does not part the two: the
+// room loses 3% from a level of 21,715 paths, the open scene gains 3% from one
+// of 75,837.
 static int tail_level(const FrameParams& F) {
     const double items = std::min<double>((double)F.W * F.H * F.nsamples, (double)F.cap);
     const double most[] = {0.3e6, 0.55e6, 1.25e6};   // items of a wave whose tail starts at 2, 3, 4
@@ -1859,8 +1867,12 @@ kpt_status kpt_set_tuning(kpt_context* c, const kpt_tuning* t) {
 // ---------------------------------------------------------------------------
 // path-replay adjoint
 
-// What a path slot takes of ADJ_WAVE_BYTES: a share of 145 bytes a vertex (its
-// record of 128, its visibility, the path's sky values) and the path's end.
+// What a path slot counts for against ADJ_WAVE_BYTES: 145 bytes a vertex and
+// 32 a path.  Its arrays take 129 a vertex (the record of 128, the visibility)
+// and 132 a path (its end, sky, sky Jacobian, weight, escape and radiance): less
+// from depth 6 on, 11% more at depth 2, where a wave of 12 GiB as counted is
+// 14.3 GB.  The count is also the limit of the split form's records; it stays
+// as it is so that what that form takes does.
 static size_t adj_path_bytes(int D) { return 145 * (size_t)(D + 1) + 2 * sizeof(float4); }
 
 static int adjoint_params(const kpt_context* c) { return 4 * (int)c->materials.size() + ADJ_SKY_PARAMS; }

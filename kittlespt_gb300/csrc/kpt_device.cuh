@@ -3,7 +3,7 @@
 // Layout in HBM (all arrays are owned by the context, see kpt_api.cu):
 //   nodes      : BvhNode[ ]   64 B per interior node; each node carries the
 //                              boxes of both children, so one pop reads one
-//                              64-byte record (four 16-byte loads) instead of
+//                              64-byte record (two 32-byte loads) instead of
 //                              two 32-byte child records;
 //   tris       : float4[3*T]  per triangle in BVH leaf order:
 //                              (v0.xyz, local id), (v1-v0, 1 for the last
